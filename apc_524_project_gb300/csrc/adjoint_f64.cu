@@ -646,7 +646,7 @@ FOut field_out(double *const *slots, int bswap) {
 // One step of the loop without sort and charge density (the primal step the
 // tangent and adjoint runs differentiate).
 int primal_step(emoo_handle *h) {
-    EMOO_TRY(fused_step_f64(h, h->dtp, 0));
+    EMOO_TRY(fused_step_f64(h, h->dtp));
     EMOO_TRY(ad_execute_bc(h, EMOO_SEND_JRHO));
     EMOO_TRY(yee_f64(h, h->dtp));
     EMOO_TRY(ad_execute_bc(h, EMOO_SEND_EB));
@@ -742,7 +742,7 @@ static int tlm_step(emoo_handle *h, AdRun &R, double **dP, double *const *dslot,
     else launch_tlm<false>(h, corr, st, P, F, dF, D, R.np, dJ);
     EMOO_CUDA(cudaGetLastError());
     // primal particle step, then the linear field part on both
-    EMOO_TRY(fused_step_f64(h, h->dtp, 0));
+    EMOO_TRY(fused_step_f64(h, h->dtp));
     EMOO_TRY(ad_execute_bc(h, EMOO_SEND_JRHO));
     if (corr) {
         // the tangent fields through the same halves, periodic images and

@@ -22,7 +22,7 @@ int cuda_status(cudaError_t e) {
     return EMOO_ERR_CUDA;
 }
 
-static bool is_pow2(double v) {
+bool is_pow2(double v) {
     int e;
     double m = frexp(v, &e);
     return m == 0.5;
@@ -53,6 +53,8 @@ void make_geom(const emoo_input_info &in, Geom &g) {
         g.area_p2[i] = is_pow2(g.area[i]);
         g.iarea[i] = 1.0 / g.area[i];
     }
+    g.unit = 1;
+    for (int i = 0; i < 3; i++) g.unit = g.unit && g.d[i] == 1.0 && g.x0[i] == 0.0;
 }
 
 // Queues the (start, stop) event pair of the timed kernel and takes a fresh
@@ -1456,7 +1458,7 @@ int emoo_step(emoo_handle *h, int nsteps, int64_t counts6[6]) {
             h->next_hist += h->opts.history_every;
         }
         if (h->precision == EMOO_FP64) {
-            EMOO_TRY(fused_step_f64(h, h->dtp, 0));
+            EMOO_TRY(fused_step_f64(h, h->dtp));
             if (h->policy == EMOO_POLICY_CORRECTED) EMOO_TRY(fold_full_f64(h, fold_what));
             else
                 for (int d = 0; d < 3; d++)

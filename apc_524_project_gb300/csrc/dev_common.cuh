@@ -65,27 +65,6 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
-// Index of the last lane of the run of equal keys that lane `lane` belongs
-// to, given the ballot of run heads (keys sorted or not: runs are maximal
-// stretches of equal consecutive keys).
-__device__ __forceinline__ int run_end(unsigned heads, int lane) {
-    unsigned later = heads & ~((2u << lane) - 1u);  // heads strictly after lane (lane 31: none)
-    if (lane == 31) later = 0u;
-    return later ? (__ffs(later) - 2) : 31;
-}
-
-// Sum of v over lanes [lane, run_end] of the calling lane's run (suffix sum
-// inside the run); the run head ends up with the run total.
-template <typename T>
-__device__ __forceinline__ T run_suffix_sum(T v, int lane, int rend) {
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        T o = __shfl_down_sync(0xffffffffu, v, off);
-        if (lane + off <= rend) v += o;
-    }
-    return v;
-}
-
 __device__ __forceinline__ void atomic_max_nonneg(double *addr, double v) {
     // non-negative doubles order like their bit patterns
     atomicMax((unsigned long long *)addr, (unsigned long long)__double_as_longlong(v));

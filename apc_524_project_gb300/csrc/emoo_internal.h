@@ -41,6 +41,7 @@ struct Geom {
     int vol_p2;
     double area[3], iarea[3];  // area[i] = d[j] * d[k], j,k the other two axes in cyclic order
     int area_p2[3];
+    int unit;  // unit cells with the origin at 0 on every axis
     // gather / deposit vertex of cell i: x0 + d (i - vshift); 0 the reference's
     // ghost-offset vertex, 1 the cell's own lower corner (corrected policy)
     int vshift = 0;
@@ -63,6 +64,8 @@ struct SpeciesTab {
     int64_t off[EMOO_NSPEC + 1];  // species s occupies [off[s], off[s+1])
     double q[EMOO_NSPEC], m[EMOO_NSPEC];
     double qp[EMOO_NSPEC];   // ((0.5 * dt * q) / m) * UNIT_ACC   (src/pusher/boris.cpp:34-35)
+    double hqp[EMOO_NSPEC];  // qp / 2
+    double vbc[EMOO_NSPEC];  // uq / vol / dt, the charge-conserving current's coefficient (0 at dt = 0)
     double uq[EMOO_NSPEC];   // UNIT_RHOJ * q                      (src/particles/deposit.cpp:30)
     double cr[EMOO_NSPEC];   // (UNIT_RHOJ * (q / vol)) / vol      (src/particles/deposit.cpp:53)
     int deposit[EMOO_NSPEC]; // 0 for test-particle species
@@ -223,6 +226,7 @@ namespace emoo {
 
 // ---- geometry ----
 void make_geom(const emoo_input_info &in, Geom &g);
+bool is_pow2(double v);
 
 // ---- FP64 field kernels (fields_f64.cu) ----
 int yee_f64(emoo_handle *h, double dt);
@@ -269,7 +273,7 @@ int push_cached_f64(emoo_handle *h, double dtp);
 int particle_bc_f64(emoo_handle *h);
 int perturb_f64(emoo_handle *h, uint64_t seed, double rel);
 int deposit_f64(emoo_handle *h, int with_rho);
-int fused_step_f64(emoo_handle *h, double dtp, int with_rho);
+int fused_step_f64(emoo_handle *h, double dtp);  // J alone
 int deposit_rho_f64(emoo_handle *h);  // rho alone at the current positions, plus the background
 int particle_moments_f64(emoo_handle *h, double out4[4]);
 int sort_keys_f64(emoo_handle *h);
