@@ -955,6 +955,7 @@ int emoo_destroy(emoo_handle *h) {
     dfree(h->wprof);
     dfree(h->wproff);
     if (h->jacobi_state) cudaFree(h->jacobi_state);
+    if (h->jacobi_tiles) cudaFree(h->jacobi_tiles);
     multigrid_free(h);
     if (h->mhost) cudaFree(h->mhost);
     for (int i = 0; i < 2; i++)

@@ -166,6 +166,7 @@ struct emoo_handle {
     double *red = nullptr;  // reduction partials
     size_t red_cap = 0;
     void *jacobi_state = nullptr;
+    void *jacobi_tiles = nullptr;  // face exchange of the tiled Jacobi (fields_f64.cu)
     int poisson_solver = 0;      // EMOO_POISSON_JACOBI / EMOO_POISSON_MULTIGRID
     double poisson_rtol = 1e-10; // multigrid stop, relative to the start residual
     void *mg = nullptr;          // multigrid levels (multigrid.cu), kept between solves

@@ -8,6 +8,7 @@
 // All kernels are HBM-bound stencils over the (n+3)^3 reference layout with
 // k (the contiguous axis) mapped to threadIdx.x for coalescing.
 #include <cuda_runtime.h>
+#include <stdio.h>
 
 #include <algorithm>
 #include <vector>
@@ -174,7 +175,7 @@ struct JacobiState {
     int skip;       // boundary fills no-ops (one sweep after done, with the test in the sweep)
     double maxdiff; // current iteration's max |u2 - u1|
     unsigned int blocks_done;
-    unsigned int pad2;
+    int error;      // a bounded wait ran out
 };
 
 // One Jacobi sweep, src/poisson/poisson.cpp:216-241.
@@ -240,6 +241,239 @@ __global__ void k_jacobi_check(Geom g, const double *u1, const double *u2, doubl
         st->iter = it + 1;
         st->maxdiff = 0.0;
         st->blocks_done = 0u;
+    }
+}
+
+// ---- Jacobi on tiles held in shared memory ---------------------------------
+//
+// The whole iteration of a small grid (every side periodic) in one cooperative
+// launch: the grid is cut into one tile a block, at most one block an SM, and
+// a tile's two buffers (ping-pong, one ghost layer) and right side stay in
+// shared memory. After each sweep a block hands its face values to its six
+// neighbours and takes theirs; no block waits for any other. A value travels
+// as one 16-byte word of two (32 bits, sequence number) pairs, each 8-byte
+// pair written and read whole, so the reader polls the value itself and no
+// fence or flag is needed; two slots a face suffice, because a block writes
+// sequence q + 2 only after it has read its neighbours' q + 1, which they made
+// from its q. A sweep of 32^3 takes 1.8 us, of which the FP64 pipe needs 0.6
+// (10 instructions a point, 8 warps an SM) and the exchange's latency the
+// rest; as two kernels a sweep it took 7.7 us. Used where a tile fits a
+// block's shared memory, up to about 100^3.
+//
+// The stop test must stop the iteration at the same sweep as the reference.
+// Blocks run JT_BATCH sweeps between grid barriers, each noting for every
+// sweep whether one of its points moved by tol or more; the barrier ORs the
+// notes, and if some sweep has none, every block goes back to the state at the
+// start of the batch (kept in the first potential's array) and repeats it up
+// to that sweep. Every wait is bounded; one that runs out sets st->error.
+constexpr int JT_BATCH = 64;
+constexpr int JT_THREADS = 1024;
+constexpr int JT_SPIN = 1 << 22;
+
+struct JacobiTiles {
+    int b[3];        // tiles per dimension
+    int t[3];        // points of the largest tile per dimension
+    int face;        // points of the largest face
+    uint4 *faces;    // [block][side][slot][face]
+    unsigned long long *moved;  // [batch] OR over the blocks
+    unsigned int *arrived;      // grid barrier
+};
+
+// blocks that passed barrier number `round` (1, 2, ..); false when it ran out
+__device__ __forceinline__ bool jt_barrier(unsigned int *arrived, unsigned int round) {
+    __syncthreads();
+    int ok = 1;
+    if (threadIdx.x == 0) {
+        const unsigned int target = round * gridDim.x;
+        __threadfence();
+        atomicAdd(arrived, 1u);
+        int spin = 0;
+        while (*((volatile unsigned int *)arrived) < target && ++spin < JT_SPIN) __nanosleep(64);
+        ok = spin < JT_SPIN;
+        __threadfence();
+    }
+    return __syncthreads_and(threadIdx.x == 0 ? ok : 1);
+}
+
+__global__ void __launch_bounds__(JT_THREADS) k_jacobi_tiles(Geom g, double *u1, double *u2, const double *R, double ax,
+                                                             double ay, double az, double af, double mult, double tol,
+                                                             JacobiTiles jt, JacobiState *st) {
+    extern __shared__ double jt_sm[];
+    int bc[3], lo[3], sz[3], nb[6];
+    {
+        int r = blockIdx.x;
+        bc[2] = r % jt.b[2];
+        r /= jt.b[2];
+        bc[1] = r % jt.b[1];
+        bc[0] = r / jt.b[1];
+        for (int d = 0; d < 3; d++) {
+            const int q = g.n[d] / jt.b[d], m = g.n[d] % jt.b[d];  // the first m tiles have one point more
+            lo[d] = bc[d] * q + min(bc[d], m) + 1;
+            sz[d] = q + (bc[d] < m ? 1 : 0);
+            for (int side = 0; side < 2; side++) {
+                int c[3] = {bc[0], bc[1], bc[2]};
+                c[d] = side ? (bc[d] + 1 == jt.b[d] ? 0 : bc[d] + 1) : (bc[d] == 0 ? jt.b[d] - 1 : bc[d] - 1);
+                nb[2 * d + side] = (c[0] * jt.b[1] + c[1]) * jt.b[2] + c[2];
+            }
+        }
+    }
+    const int py = sz[2] + 2, px = (sz[1] + 2) * py;  // strides of the tile with its ghost layer
+    const int vol = sz[0] * sz[1] * sz[2], whole = (sz[0] + 2) * px;
+    double *cur = jt_sm, *next = cur + whole, *rhs = next + whole;
+    const int area[3] = {sz[1] * sz[2], sz[0] * sz[2], sz[0] * sz[1]};
+    const int halo = 2 * (area[0] + area[1] + area[2]);
+    auto point = [&](int p, int &i, int &j, int &k) {  // of the tile, from 0
+        k = p % sz[2];
+        const int r = p / sz[2];
+        j = r % sz[1];
+        i = r / sz[1];
+    };
+    // halo value q of side `side` of dimension d: its ghost point in the tile
+    auto halo_at = [&](int p, int &d, int &side, int &q) -> int {
+        d = 0;
+        q = p;
+        while (q >= 2 * area[d]) q -= 2 * area[d++];
+        side = q >= area[d];
+        q -= side * area[d];
+        const int o1 = d == 0 ? 1 : 0, o2 = d == 2 ? 1 : 2;
+        int c[3];
+        c[d] = side ? sz[d] + 1 : 0;
+        c[o1] = q / sz[o2] + 1;
+        c[o2] = q % sz[o2] + 1;
+        return c[0] * px + c[1] * py + c[2];
+    };
+    // this thread's first point and first halo value, kept: most tiles have no
+    // more than one a thread, and the divisions would cost each sweep 0.1 us
+    int mi = 0, mj = 0, mk = 0, hd = 0, hside = 0, hq = 0, hat = 0;
+    if (threadIdx.x < vol) point(threadIdx.x, mi, mj, mk);
+    if (threadIdx.x < halo) hat = halo_at(threadIdx.x, hd, hside, hq);
+    auto load = [&](double *dst, const double *u) {  // tile and ghost layer of a global potential
+        for (int p = threadIdx.x; p < whole; p += blockDim.x) {
+            int c[3] = {p / px, (p % px) / py, p % py};
+            for (int d = 0; d < 3; d++) {
+                c[d] += lo[d] - 1;
+                c[d] = c[d] < 1 ? g.n[d] : (c[d] > g.n[d] ? 1 : c[d]);
+            }
+            dst[p] = __ldcg(u + gidx(g, c[0], c[1], c[2]));
+        }
+    };
+    auto store = [&](const double *src, double *u) {
+        for (int p = threadIdx.x; p < vol; p += blockDim.x) {
+            int i, j, k;
+            point(p, i, j, k);
+            u[gidx(g, lo[0] + i, lo[1] + j, lo[2] + k)] = src[(i + 1) * px + (j + 1) * py + k + 1];
+        }
+    };
+    auto slot = [&](int block, int side, unsigned int seq) {
+        return jt.faces + ((size_t)(block * 6 + side) * 2 + (seq & 1u)) * jt.face;
+    };
+    for (int p = threadIdx.x; p < vol; p += blockDim.x) {
+        int i, j, k;
+        point(p, i, j, k);
+        rhs[p] = af * R[gidx(g, lo[0] + i, lo[1] + j, lo[2] + k)] * mult;
+    }
+    load(cur, u1);
+    __syncthreads();
+    const long long ltol = __double_as_longlong(tol), linf = 0x7ff0000000000000LL;
+    unsigned int seq = 0, round = 0;
+    bool fresh = true, ok = true;  // fresh: cur's ghost layer is filled
+    // one sweep; whether a point of the block moved by tol or more
+    auto sweep = [&]() -> bool {
+        if (!fresh) {
+            bool got = true;
+            for (int p = threadIdx.x; p < halo; p += blockDim.x) {
+                int d = hd, side = hside, q = hq, at = hat;
+                if (p != threadIdx.x) at = halo_at(p, d, side, q);
+                // my ghost plane on this side is the neighbour's face on the other
+                const uint4 *src = slot(nb[2 * d + side], 2 * d + 1 - side, seq) + q;
+                unsigned int x, f0, y, f1;
+                int spin = 0;
+                do {
+                    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(x), "=r"(f0), "=r"(y), "=r"(f1)
+                                 : "l"(src)
+                                 : "memory");
+                } while ((f0 != seq || f1 != seq) && ++spin < JT_SPIN);
+                got = got && spin < JT_SPIN;
+                cur[at] = __hiloint2double((int)y, (int)x);
+            }
+            ok = __syncthreads_and(got);
+            if (!ok) return true;
+        }
+        seq++;
+        bool far = false;
+        for (int p = threadIdx.x; p < vol; p += blockDim.x) {
+            int c[3] = {mi, mj, mk};
+            if (p != threadIdx.x) point(p, c[0], c[1], c[2]);
+            const int o = (c[0] + 1) * px + (c[1] + 1) * py + c[2] + 1;
+            const double v = ax * (cur[o - px] + cur[o + px]) + ay * (cur[o - py] + cur[o + py]) +
+                             az * (cur[o - 1] + cur[o + 1]) - rhs[p];
+            next[o] = v;
+            const unsigned int x = (unsigned int)__double2loint(v), y = (unsigned int)__double2hiint(v);
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                const int o1 = d == 0 ? 1 : 0, o2 = d == 2 ? 1 : 2;
+#pragma unroll
+                for (int side = 0; side < 2; side++) {
+                    if (c[d] != (side ? sz[d] - 1 : 0)) continue;
+                    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(
+                                     slot(blockIdx.x, 2 * d + side, seq) + c[o1] * sz[o2] + c[o2]),
+                                 "r"(x), "r"(seq), "r"(y)
+                                 : "memory");
+                }
+            }
+            // |v - u| >= tol on the words (false for NaN, as the comparison is)
+            const long long a = __double_as_longlong(fabs(v - cur[o]));
+            far = far || (a >= ltol && a <= linf);
+        }
+        far = __syncthreads_or(far);
+        double *t = cur;
+        cur = next;
+        next = t;
+        fresh = false;
+        return far;
+    };
+    int done = 0;  // sweeps completed before this batch; sweep s is iteration number s
+    bool converged = false;
+    for (int batch = 0; ok; batch++) {
+        const int n = min(JT_BATCH, ITER_MAX + 1 - done);
+        if (batch) store(cur, u1);
+        unsigned long long moved = 0;
+        for (int s = 0; s < n && ok; s++)
+            if (sweep()) moved |= 1ull << s;
+        if (!ok) break;
+        if (threadIdx.x == 0 && moved) atomicOr(jt.moved + batch, moved);
+        ok = jt_barrier(jt.arrived, ++round);
+        if (!ok) break;
+        const unsigned long long still = ~__ldcg(jt.moved + batch);
+        const int first = still ? __ffsll((long long)still) - 1 : JT_BATCH;  // first sweep in which nothing moved
+        if (first < n) {
+            converged = true;
+            if (first < n - 1) {  // back to the batch's start, and up to that sweep
+                load(cur, u1);
+                fresh = true;
+                ok = jt_barrier(jt.arrived, ++round);
+                for (int s = 0; s <= first && ok; s++) sweep();
+            }
+            done += first + 1;
+            break;
+        }
+        done += n;
+        if (done > ITER_MAX) break;
+    }
+    // the last sweep's result and the one before it, in the arrays the
+    // alternating sweeps leave them in
+    if (ok) {
+        store(cur, (done - 1) % 2 == 0 ? u2 : u1);
+        store(next, (done - 1) % 2 == 0 ? u1 : u2);
+    }
+    if (threadIdx.x == 0) {
+        if (!ok) st->error = 1;
+        if (blockIdx.x == 0) {
+            st->done = 1;
+            st->iter = done;
+            st->converged = converged;
+        }
     }
 }
 
@@ -749,6 +983,53 @@ static int single_field_bc(emoo_handle *h, int id, const int *skip) {
 // applies it, for the multigrid's start and result.
 int poisson_field_bc(emoo_handle *h, int id) { return single_field_bc(h, id, nullptr); }
 
+// The tiles of k_jacobi_tiles for this grid and their scratch (kept with the
+// handle); b[0] = 0 where the kernel does not apply: a side that is not
+// periodic, or a tile that does not fit a block's shared memory. The cut is
+// the one whose largest tile takes the fewest cycles: 160 of the FP64 pipe for
+// each 32 points, and about 4 for a face value sent and received.
+static int jacobi_tiling(emoo_handle *h, JacobiTiles *jt, size_t *smem) {
+    const Geom &g = h->g;
+    *jt = JacobiTiles{};
+    for (int s = 0; s < 6; s++)
+        if (h->bc.fbc[s] != FBC_PERIODIC) return EMOO_OK;
+    int sms = 0, smem_max = 0, coop = 0;
+    EMOO_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev));
+    EMOO_CUDA(cudaDeviceGetAttribute(&smem_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->dev));
+    EMOO_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->dev));
+    if (!coop) return EMOO_OK;
+    int64_t best = INT64_MAX;
+    for (int bx = 1; bx <= std::min(sms, g.n[0]); bx++)
+        for (int by = 1; by <= std::min(sms / bx, g.n[1]); by++) {
+            const int bz = std::min(sms / (bx * by), g.n[2]);
+            const int64_t t[3] = {(g.n[0] + bx - 1) / bx, (g.n[1] + by - 1) / by, (g.n[2] + bz - 1) / bz};
+            const int64_t vol = t[0] * t[1] * t[2], halo = 2 * (t[0] * t[1] + t[0] * t[2] + t[1] * t[2]);
+            const int64_t bytes = (2 * (t[0] + 2) * (t[1] + 2) * (t[2] + 2) + vol) * (int64_t)sizeof(double);
+            const int64_t cost = (vol + 31) / 32 * 160 + halo * 4;
+            if (bytes > smem_max || cost >= best) continue;
+            best = cost;
+            *smem = (size_t)bytes;
+            const int b[3] = {bx, by, bz};
+            for (int d = 0; d < 3; d++) {
+                jt->b[d] = b[d];
+                jt->t[d] = (int)t[d];
+            }
+            jt->face = (int)std::max(t[0] * t[1], std::max(t[0] * t[2], t[1] * t[2]));
+        }
+    if (!jt->b[0]) return EMOO_OK;
+    EMOO_CUDA(cudaFuncSetAttribute(k_jacobi_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+    const int blocks = jt->b[0] * jt->b[1] * jt->b[2], batches = ITER_MAX / JT_BATCH + 2;
+    const size_t faces = (size_t)blocks * 12 * jt->face * sizeof(uint4);
+    const size_t bytes = faces + batches * sizeof(unsigned long long) + sizeof(unsigned long long);
+    if (!h->jacobi_tiles) EMOO_CUDA(cudaMalloc(&h->jacobi_tiles, bytes));  // one grid, one size a handle
+    char *p = (char *)h->jacobi_tiles;
+    jt->faces = (uint4 *)p;
+    jt->moved = (unsigned long long *)(p + faces);
+    jt->arrived = (unsigned int *)(jt->moved + batches);
+    EMOO_CUDA(cudaMemsetAsync(p, 0, bytes, h->stream));
+    return EMOO_OK;
+}
+
 // Poisson_Solver::run_poisson_solver_, src/poisson/poisson.cpp:172-287, with
 // the iteration control on the device: iterations are queued in batches and
 // become no-ops once the stop test of the reference has fired.
@@ -766,6 +1047,28 @@ int jacobi_f64(emoo_handle *h, int id1, int id2, int rid, double tol, double mul
     EMOO_TRY(single_field_bc(h, id1, nullptr));
     double *u1 = h->slot[id1], *u2 = h->slot[id2];
     const double *R = h->slot[rid];
+    JacobiState hs;
+    JacobiTiles jt;
+    size_t smem = 0;
+    EMOO_TRY(jacobi_tiling(h, &jt, &smem));
+    if (jt.b[0]) {
+        int threads = std::min(JT_THREADS, (jt.t[0] * jt.t[1] * jt.t[2] + 31) / 32 * 32);
+        void *args[] = {(void *)&g,  &u1, &u2, (void *)&R, &ax, &ay, &az, &af, &mult, &tol, &jt, &st};
+        h->launches++;
+        EMOO_CUDA(cudaLaunchCooperativeKernel((const void *)k_jacobi_tiles, dim3(jt.b[0] * jt.b[1] * jt.b[2]),
+                                              dim3(threads), args, smem, h->stream));
+        EMOO_TRY(single_field_bc(h, id1, nullptr));
+        EMOO_TRY(single_field_bc(h, id2, nullptr));
+        EMOO_CUDA(cudaMemcpyAsync(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost, h->stream));
+        EMOO_CUDA(cudaStreamSynchronize(h->stream));
+        if (hs.error) {
+            fprintf(stderr, "emoo: a wait of the Jacobi kernel ran out\n");
+            return EMOO_ERR_CUDA;
+        }
+        if (iters) *iters = hs.iter - 1;
+        if (converged) *converged = hs.converged;
+        return EMOO_OK;
+    }
     dim3 blk(32, 8);
     dim3 grd = phys_grid(g, blk);
     int rb = reduce_blocks(g);
@@ -775,8 +1078,8 @@ int jacobi_f64(emoo_handle *h, int id1, int id2, int rid, double tol, double mul
     // a launch latency each. Once the stop test has fired they are no-ops.
     const int batch = 32;
     int batch_launches = 0;
-    // With every side periodic the stop test can run inside the sweep: one
-    // kernel fewer per sweep, which pays where launches dominate. On large
+    // With every side periodic (and a grid past the tiles' shared memory) the
+    // stop test can run inside the sweep: one kernel fewer per sweep. On large
     // grids the sweep's per-block FP64 max trees (FP64 pipe) cost more than
     // the separate check's grid-stride reduction, so it stays separate there.
     bool all_periodic = (int64_t)g.n[0] * g.n[1] * g.n[2] <= (int64_t)1 << 21;
@@ -813,7 +1116,6 @@ int jacobi_f64(emoo_handle *h, int id1, int id2, int rid, double tol, double mul
     cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (ie != cudaSuccess) return cuda_status(ie);
-    JacobiState hs;
     int launched = 0;
     int rc = EMOO_OK;
     for (;;) {
