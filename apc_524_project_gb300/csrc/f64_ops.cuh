@@ -3,10 +3,11 @@
 //
 // This GPU issues FP64 arithmetic, comparisons and FP64 conversions at two
 // lanes per clock per SM: one warp instruction of them takes as long as some
-// 64 of any other kind. The helpers below give bit-identical results from
-// integer instructions on the halves of the word (truncation, conversion of
-// small integers, halving, tests), or with fewer FP64 instructions (several
-// quotients over one divisor).
+// 64 of any other kind. The helpers below give the same results from integer
+// instructions on the halves of the word (truncation, conversions, halving,
+// tests), or with fewer FP64 instructions (several quotients over one
+// divisor). They are complete over all words: a rare case left to the FP64
+// instruction would be predicated in by the compiler and issued always.
 #ifndef EMOO_F64_OPS_CUH
 #define EMOO_F64_OPS_CUH
 
@@ -23,31 +24,70 @@ __device__ __forceinline__ bool f64_not_nan(double x) {
 
 __device__ __forceinline__ bool f64_sign(double x) { return __double2hiint(x) < 0; }
 
-// __double2int_rz(t): by shifts for |t| < 2^20, by the conversion above.
+// __double2int_rz(t): truncated, saturated, NaN to the smallest.
 __device__ __forceinline__ int f64_trunc(double t) {
     const int hi = __double2hiint(t);
+    const unsigned lo = (unsigned)__double2loint(t);
     const int e = ((hi >> 20) & 0x7ff) - 1023;
-    if (e >= 20) return __double2int_rz(t);
-    const int m = e < 0 ? 0 : ((hi & 0xfffff) | 0x100000) >> (20 - e);
+    const unsigned top = ((unsigned)hi << 11) | (lo >> 21) | 0x80000000u;  // the 32 leading bits
+    if (e > 30) return hi < 0 || !f64_not_nan(t) ? (int)0x80000000 : 0x7fffffff;
+    const int m = e < 0 ? 0 : (int)(top >> (31 - e));
     return hi < 0 ? -m : m;
 }
 
-// (double)i: assembled for |i| < 2^20 (every cell index of a grid that fits
-// the device), by the conversion above.
+// (double)i
 __device__ __forceinline__ double f64_of_int(int i) {
-    const int a = i < 0 ? -i : i;
-    if ((unsigned)a >= (1u << 20)) return (double)i;
-    const int e = 31 - __clz(a);  // -1 for 0
-    const int hi = a ? ((1023 + e) << 20) | ((a << (20 - e)) & 0xfffff) : 0;
-    return __hiloint2double(hi | (i & 0x80000000), 0);
+    const unsigned a = i < 0 ? 0u - (unsigned)i : (unsigned)i;
+    const int z = __clz((int)a);
+    const unsigned m = a << (z & 31);  // the leading one at bit 31
+    const unsigned hi = ((1023u + 31u - (unsigned)z) << 20) | ((m >> 11) & 0xfffffu);
+    return a ? __hiloint2double((int)(hi | ((unsigned)i & 0x80000000u)), (int)(m << 21)) : 0.0;
 }
 
-// 0.5 * x for x that is normally a positive number of ordinary size: one off
-// the exponent; zeros, denormals, infinities, NaN and negatives multiply.
+// 0.5 * x where neither is denormal: one off the exponent (zero, infinity and
+// NaN stay).
 __device__ __forceinline__ double f64_half(double x) {
-    const int hi = __double2hiint(x);
-    if ((unsigned)(hi - 0x00200000) >= 0x7fd00000u) return 0.5 * x;
-    return __hiloint2double(hi - 0x00100000, __double2loint(x));
+    const unsigned hi = (unsigned)__double2hiint(x), e = hi & 0x7ff00000u;
+    return __hiloint2double((int)(e - 1u < 0x7fefffffu ? hi - 0x00100000u : hi), __double2loint(x));
+}
+
+// (float)x: to nearest, ties to even
+__device__ __forceinline__ float f64_to_f32(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned sign = hi & 0x80000000u;
+    const int e = (int)((hi >> 20) & 0x7ffu) - 896;  // the float's exponent field
+    unsigned b;
+    if (e >= 255) {  // too large, infinite or NaN
+        b = f64_not_nan(x) ? 0x7f800000u : 0x7fffffffu;
+    } else if (e >= 1) {  // a carry out of the mantissa rounds up the exponent
+        b = ((unsigned)e << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+        b += (lo & 0x1fffffffu) > 0x10000000u - (b & 1u) ? 1u : 0u;
+    } else {  // denormal or zero: the mantissa shifted down, 30 bits at e = 0
+        const int s = 30 - e;
+        const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+        if (s > 54) {
+            b = 0u;
+        } else {
+            const unsigned long long half = 1ull << (s - 1), rest = m & (2ull * half - 1ull);
+            b = (unsigned)(m >> s);
+            b += rest > half - (b & 1u) ? 1u : 0u;
+        }
+    }
+    return __uint_as_float(b | sign);
+}
+
+// (double)x
+__device__ __forceinline__ double f64_of_f32(float x) {
+    const unsigned b = __float_as_uint(x), sign = b & 0x80000000u;
+    unsigned e = (b >> 23) & 0xffu, m = b & 0x7fffffu;
+    if (e == 0u) {  // zero, or a denormal moved up to a leading one
+        if (m == 0u) return __hiloint2double((int)b, 0);
+        const int z = __clz((int)m) - 8;
+        m = (m << z) & 0x7fffffu;
+        e = 1u - (unsigned)z;  // below 0: wraps, and back with the bias
+    }
+    const unsigned hi = e == 255u ? 0x7ff00000u : (e + 896u) << 20;
+    return __hiloint2double((int)(sign | hi | (m >> 3)), (int)(m << 29));
 }
 
 // A total order on the words that agrees with < on numbers, zeros apart

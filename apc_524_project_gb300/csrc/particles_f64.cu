@@ -91,17 +91,23 @@ __device__ __forceinline__ void gather_cell(const Geom &g, const GatherPtrs &P, 
     }
 }
 
-// x + dt v; with dt a power of two (dt_p2) the product is exact and one fused
+// What a kernel's instance may take for granted: unit cells at the origin,
+// and with them a time step that is a power of two.
+enum { ANY = 0, UNIT_CELLS = 1, UNIT_DT2 = 2 };
+
+// x + dt v; with dt a power of two the product is exact and one fused
 // instruction gives the same sum.
-__device__ __forceinline__ double advance(double x, double dt, int dt_p2, double v) {
-    return dt_p2 ? __fma_rn(dt, v, x) : x + dt * v;
+template <int MODE>
+__device__ __forceinline__ double advance(double x, double dt, double v) {
+    return MODE == UNIT_DT2 ? __fma_rn(dt, v, x) : x + dt * v;
 }
 
 // Boris::Step, src/pusher/boris.cpp:33-85 (q_p precomputed per species, hq
 // half of it), on e and b2 = 2 B: hq b2 = q_p B, and 2 / (1 + q_p q_p B^2)
 // from the same scaled words.
+template <int MODE>
 __device__ __forceinline__ void boris_push(double q_p, double hq, const double e[3], const double b2[3], double dt,
-                                           int dt_p2, double p[3], double v[3]) {
+                                           double p[3], double v[3]) {
     const double ex = e[0], ey = e[1], ez = e[2];
     double tx = hq * b2[0], ty = hq * b2[1], tz = hq * b2[2];
     double bsqr4 = b2[0] * b2[0] + b2[1] * b2[1] + b2[2] * b2[2];
@@ -119,14 +125,15 @@ __device__ __forceinline__ void boris_push(double q_p, double hq, const double e
     v[1] = v_py + qey;
     v[2] = v_pz + qez;
 #pragma unroll
-    for (int a = 0; a < 3; a++) p[a] = advance(p[a], dt, dt_p2, v[a]);
+    for (int a = 0; a < 3; a++) p[a] = advance<MODE>(p[a], dt, v[a]);
 }
 
 // Relativistic_Boris::Step (Vay), src/pusher/relativisticBoris.cpp:53-140, on
 // e and b2 = 2 B: hq b2 = q_p B; e + v x B as one fused instruction with the
 // exact half of v x b2; sigma^2 + 4 (..) likewise.
+template <int MODE>
 __device__ __forceinline__ void vay_push(double q_p, double hq, const double e[3], const double b2[3], double dt,
-                                         int dt_p2, double p[3], double v[3], double &gamma) {
+                                         double p[3], double v[3], double &gamma) {
     const double bx = b2[0], by = b2[1], bz = b2[2];
     double vXbx = v[1] * bz - v[2] * by, vXby = v[2] * bx - v[0] * bz, vXbz = v[0] * by - v[1] * bx;
     double uhx = gamma * v[0] + q_p * __fma_rn(0.5, vXbx, e[0]);
@@ -149,7 +156,7 @@ __device__ __forceinline__ void vay_push(double q_p, double hq, const double e[3
     v[1] = f64_quot(s * (upy + udott * ty + upXt_y), dg);
     v[2] = f64_quot(s * (upz + udott * tz + upXt_z), dg);
 #pragma unroll
-    for (int a = 0; a < 3; a++) p[a] = advance(p[a], dt, dt_p2, v[a]);
+    for (int a = 0; a < 3; a++) p[a] = advance<MODE>(p[a], dt, v[a]);
     gamma = gi;
 }
 
@@ -367,8 +374,8 @@ __global__ void k_interpolate(Geom g, GatherPtrs P, PState S, int64_t np, int64_
 }
 
 // emoo_push: Particle_Handler::Push with the cached fields.
-__global__ void k_push_cached(SpeciesTab st, PState S, int64_t np, int64_t cap, const double *fc, double dt, int dt_p2,
-                              int rel) {
+__global__ void k_push_cached(SpeciesTab st, PState S, int64_t np, int64_t cap, const double *fc, double dt, int rel) {
+    constexpr int MODE = ANY;
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= np) return;
     double pos[3] = {S.x[p], S.y[p], S.z[p]};
@@ -383,10 +390,10 @@ __global__ void k_push_cached(SpeciesTab st, PState S, int64_t np, int64_t cap, 
     double v[3] = {S.vx[p], S.vy[p], S.vz[p]};
     if (rel) {
         double ga = S.g[p];
-        vay_push(st.qp[s], st.hqp[s], e, b2, dt, dt_p2, pos, v, ga);
+        vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga);
         S.g[p] = ga;
     } else {
-        boris_push(st.qp[s], st.hqp[s], e, b2, dt, dt_p2, pos, v);
+        boris_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v);
     }
     S.x[p] = pos[0]; S.y[p] = pos[1]; S.z[p] = pos[2];
     S.vx[p] = v[0]; S.vy[p] = v[1]; S.vz[p] = v[2];
@@ -542,10 +549,11 @@ __device__ void absorbed_exit(const Geom &g, const BCTab &bc, const DepositPtrs 
 // particles in 49x37x29 unit cells: 1063 us a launch, FP64 pipe 84 % active,
 // against 1877 us with every particle's pieces committed one by one (12
 // atomics a piece) and the FP64 tests, conversions and divisions in place.
-template <bool REL, bool UNIT>
+template <bool REL, int MODE>
 __global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
-                                                         int64_t np, DepositPtrs D, double dt, int dt_p2,
+                                                         int64_t np, DepositPtrs D, double dt,
                                                          DevCounters *ctr) {
+    constexpr bool UNIT = MODE != ANY;
     __shared__ CommitTile tiles[PART_WARPS];
     __shared__ double s_move[6][PART_BLOCK];  // start and end of the listed moves
     __shared__ double s_coef[PART_BLOCK];
@@ -575,10 +583,10 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, 
                 for (int a = 0; a < 3; a++) p0[a] = pos[a];
                 if (REL) {
                     double ga = S.g[p];
-                    vay_push(st.qp[s], st.hqp[s], e, b2, dt, dt_p2, pos, v, ga);
+                    vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga);
                     S.g[p] = ga;
                 } else {
-                    boris_push(st.qp[s], st.hqp[s], e, b2, dt, dt_p2, pos, v);
+                    boris_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v);
                 }
 #pragma unroll
                 for (int a = 0; a < 3; a++) p1[a] = pos[a];
@@ -654,14 +662,14 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, 
 // The fused time-loop kernel: gather at the current position (what
 // InterpolateEB cached at the end of the previous step), push, the six
 // boundaries, then the current deposit at the new position. Bound by the FP64
-// pipe: 232 FP64 instructions a particle (405 with tests, conversions and
+// pipe: 228 FP64 instructions a particle (405 with tests, conversions and
 // divisions on that pipe and the deposit summed in shuffle trees), 85 % active.
-// Relativistic, 3,538,944 particles in 48^3 unit cells, sorted: 1543 us a
+// Relativistic, 3,538,944 particles in 48^3 unit cells, sorted: 1507 us a
 // launch against 2550 us.
-template <bool REL, bool UNIT>
+template <bool REL, int MODE>
 __global__ void __launch_bounds__(PART_BLOCK) k_fused(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
-                                                      int64_t np, DepositPtrs D, double dt, int dt_p2,
-                                                      DevCounters *ctr) {
+                                                      int64_t np, DepositPtrs D, double dt, DevCounters *ctr) {
+    constexpr bool UNIT = MODE != ANY;
     __shared__ CommitTile tiles[PART_WARPS];
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     bool active = false;
@@ -683,10 +691,10 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused(Geom g, SpeciesTab st, BCT
                 double v[3] = {S.vx[p], S.vy[p], S.vz[p]};
                 if (REL) {
                     double ga = S.g[p];
-                    vay_push(st.qp[s], st.hqp[s], e, b2, dt, dt_p2, pos, v, ga);
+                    vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga);
                     S.g[p] = ga;
                 } else {
-                    boris_push(st.qp[s], st.hqp[s], e, b2, dt, dt_p2, pos, v);
+                    boris_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v);
                 }
                 if (maybe_crossed(bc, pos)) mask = apply_bc(bc, pos, v);
                 if (mask & 64) {
@@ -852,7 +860,7 @@ int push_cached_f64(emoo_handle *h, double dtp) {
     species_tab(h, dtp, st);
     h->launches++;
     k_push_cached<<<blocks_for(h->np), 256, 0, h->stream>>>(st, pstate(h), h->np, h->cap, h->fcache, dtp,
-                                                            is_pow2(dtp), h->info.relativity != 0);
+                                                            h->info.relativity != 0);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -892,15 +900,15 @@ int deposit_rho_f64(emoo_handle *h) {
     return rho_background_f64(h, 1);
 }
 
-template <bool REL, bool UNIT>
+template <bool REL, int MODE>
 static void launch_fused(emoo_handle *h, const SpeciesTab &st, double dtp) {
     const int nb = blocks_for(h->np, PART_BLOCK);
     if (h->policy == EMOO_POLICY_CORRECTED)
-        k_fused_vb<REL, UNIT><<<nb, PART_BLOCK, 0, h->stream>>>(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
-                                                                deposit_ptrs(h), dtp, is_pow2(dtp), h->ctr);
+        k_fused_vb<REL, MODE><<<nb, PART_BLOCK, 0, h->stream>>>(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
+                                                                deposit_ptrs(h), dtp, h->ctr);
     else
-        k_fused<REL, UNIT><<<nb, PART_BLOCK, 0, h->stream>>>(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
-                                                             deposit_ptrs(h), dtp, is_pow2(dtp), h->ctr);
+        k_fused<REL, MODE><<<nb, PART_BLOCK, 0, h->stream>>>(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
+                                                             deposit_ptrs(h), dtp, h->ctr);
 }
 
 int fused_step_f64(emoo_handle *h, double dtp) {
@@ -912,12 +920,15 @@ int fused_step_f64(emoo_handle *h, double dtp) {
     const bool timed = h->prof_on && h->policy != EMOO_POLICY_CORRECTED;
     h->launches++;
     if (timed) EMOO_CUDA(cudaEventRecord(h->prof_ev[0], h->stream));
+    const int mode = !h->g.unit ? ANY : is_pow2(dtp) ? UNIT_DT2 : UNIT_CELLS;
     if (h->info.relativity) {
-        if (h->g.unit) launch_fused<true, true>(h, st, dtp);
-        else launch_fused<true, false>(h, st, dtp);
+        if (mode == UNIT_DT2) launch_fused<true, UNIT_DT2>(h, st, dtp);
+        else if (mode == UNIT_CELLS) launch_fused<true, UNIT_CELLS>(h, st, dtp);
+        else launch_fused<true, ANY>(h, st, dtp);
     } else {
-        if (h->g.unit) launch_fused<false, true>(h, st, dtp);
-        else launch_fused<false, false>(h, st, dtp);
+        if (mode == UNIT_DT2) launch_fused<false, UNIT_DT2>(h, st, dtp);
+        else if (mode == UNIT_CELLS) launch_fused<false, UNIT_CELLS>(h, st, dtp);
+        else launch_fused<false, ANY>(h, st, dtp);
     }
     EMOO_CUDA(cudaGetLastError());
     if (timed) {

@@ -33,6 +33,7 @@
 #include "dev_common.cuh"
 #include "ad_mixed.cuh"
 #include "emoo_internal.h"
+#include "f64_ops.cuh"
 
 namespace emoo {
 
@@ -435,52 +436,62 @@ constexpr int COL_STRIDE = 36;
 // (cell, in-cell offsets, u); false when the position is outside the box or
 // not a number. vmode (relativistic, before the first push): u holds v and
 // g0 the loaded gamma. Shared by the loader and the host-resident step, so
-// both convert bit-identically.
+// both convert bit-identically. Truncation and FP32 rounding are integer
+// instructions (f64_ops.cuh): on the FP64 pipe they were four fifths of it.
+template <bool UNIT>
 __device__ __forceinline__ bool f64_to_m(const Geom &g, const double pos[3], const double v[3], double ga, int rel,
                                          int vmode, int32_t &cell, float o[3], float u[3], float &g0) {
     int ci[3];
     bool ok = true;
     for (int d = 0; d < 3; d++) {
-        double t = (pos[d] - g.x0[d]) * g.id[d];  // cells from x0
-        double fl = floor(t);
-        ci[d] = (int)fl + 1;
-        float of = (float)(t - fl);
+        const double t = UNIT ? pos[d] : (pos[d] - g.x0[d]) * g.id[d];  // cells from x0
+        int k = f64_trunc(t);
+        const bool zero = (unsigned long long)__double_as_longlong(t) << 1 == 0ull;
+        if (!zero && k > (int)0x80000000 && f64_key(t) < f64_key(f64_of_int(k))) k--;  // floor
+        ci[d] = k + 1;
+        float of = f64_to_f32(t - f64_of_int(k));
         if (of >= 1.0f) {
             of = 0.0f;
             ci[d] += 1;
         }
         o[d] = of;
-        if (!(t == t) || ci[d] < 1 || ci[d] > g.n[d]) ok = false;
+        if (!f64_not_nan(t) || ci[d] < 1 || ci[d] > g.n[d]) ok = false;
     }
     if (!ok) return false;
     cell = (int32_t)((int64_t)ci[0] * g.sx + (int64_t)ci[1] * g.sy + ci[2]);
     if (rel && vmode) {
-        for (int d = 0; d < 3; d++) u[d] = (float)v[d];
-        g0 = (float)ga;
+        for (int d = 0; d < 3; d++) u[d] = f64_to_f32(v[d]);
+        g0 = f64_to_f32(ga);
     } else {
-        const double f = rel ? ga : 1.0;
-        for (int d = 0; d < 3; d++) u[d] = (float)(f * v[d]);
+        for (int d = 0; d < 3; d++) u[d] = f64_to_f32(rel ? ga * v[d] : v[d]);
     }
     return true;
 }
 
 // The mixed state of one live particle back to FP64: out = x, y, z, vx, vy,
 // vz, gamma (gamma 0 for the non-relativistic pusher, as new_particle()).
-__device__ __forceinline__ void m_to_f64(const Geom &g, int32_t c, const float o[3], const float uf[3], int rel,
-                                         double out[7]) {
-    int ix = (int)(c / g.sx);
-    int64_t r = c - ix * g.sx;
-    int iy = (int)(r / g.sy);
-    int iz = (int)(r - iy * g.sy);
-    out[0] = g.x0[0] + g.d[0] * ((double)(ix - 1) + (double)o[0]);
-    out[1] = g.x0[1] + g.d[1] * ((double)(iy - 1) + (double)o[1]);
-    out[2] = g.x0[2] + g.d[2] * ((double)(iz - 1) + (double)o[2]);
-    double ux = uf[0], uy = uf[1], uz = uf[2];
-    double ga = rel ? sqrt(1.0 + ux * ux + uy * uy + uz * uz) : 1.0;
-    out[3] = ux / ga;
-    out[4] = uy / ga;
-    out[5] = uz / ga;
-    out[6] = rel ? ga : 0.0;
+template <bool UNIT>
+__device__ __forceinline__ void m_to_f64(const Geom &g, const Div3 &dv, int32_t c, const float o[3],
+                                         const float uf[3], int rel, double out[7]) {
+    const uint32_t uc = (uint32_t)c;
+    const uint32_t ix = dv.sx.d == 1 ? uc : fdiv(uc, dv.sx), r = uc - ix * dv.sx.d;
+    const uint32_t iy = dv.sy.d == 1 ? r : fdiv(r, dv.sy);
+    const int i[3] = {(int)ix, (int)iy, (int)(r - iy * dv.sy.d)};
+    double u[3];
+    for (int a = 0; a < 3; a++) {
+        const double q = f64_of_int(i[a] - 1) + f64_of_f32(o[a]);
+        out[a] = UNIT ? q : g.x0[a] + g.d[a] * q;
+        u[a] = f64_of_f32(uf[a]);
+    }
+    if (rel) {  // v = u / gamma: three quotients over one divisor
+        const double ga = sqrt(1.0 + u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+        const F64Quot q = f64_divisor(ga);
+        for (int a = 0; a < 3; a++) out[3 + a] = f64_quot(u[a], q);
+        out[6] = ga;
+    } else {
+        for (int a = 0; a < 3; a++) out[3 + a] = u[a];
+        out[6] = 0.0;
+    }
 }
 
 // A dropped particle in the caller's arrays, as the readback writes it.
@@ -690,12 +701,12 @@ __device__ __forceinline__ void vb_pieces_list(const MGeom &g, const BCTab &bc, 
 // more warps hide the L2 latency that grows as particles drift between sorts
 // (12.59 against 13.06 ms a launch at 5); 4 (64 registers, no spills) for the
 // corrected policy's pieces (19.23 against 20.01 ms at 5 with 148 bytes of
-// spills, 24.6 ms at 6); 5 (48 registers) for the host-resident conversions.
+// spills, 24.6 ms at 6) and for the host-resident conversions (spills at 5).
 // The same warps in blocks of 128 threads, twice as many blocks, take 12.36
 // ms (blocks of 64: 12.60; of 96: 12.63; of 512: 12.92).
 template <bool CORR, bool HOST>
 constexpr int fused_min_blocks() {
-    return 256 / FUSED_BLOCK * (CORR ? 4 : (HOST ? 5 : 6));
+    return 256 / FUSED_BLOCK * (CORR || HOST ? 4 : 6);
 }
 
 template <bool REL, bool FIRST, bool PUSH, bool CORR = false, bool HOST = false>
@@ -733,7 +744,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
             const double v[3] = {Hp->vx[hs][hi], Hp->vy[hs][hi], Hp->vz[hs][hi]};
             const double ga = Hp->gam[hs] ? Hp->gam[hs][hi] : 0.0;
             float o3[3], u3[3], gz;
-            if (f64_to_m(Hp->g, pos, v, ga, Hp->rel, 0, c, o3, u3, gz)) {
+            if (f64_to_m<false>(Hp->g, pos, v, ga, Hp->rel, 0, c, o3, u3, gz)) {
                 ox = o3[0], oy = o3[1], oz = o3[2];
                 ux = u3[0], uy = u3[1], uz = u3[2];
             } else {  // outside the box (the loader's bounds check): dropped as the readback drops it
@@ -809,7 +820,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
                 if (PUSH && HOST) {
                     const float o3[3] = {ox, oy, oz}, u3[3] = {ux, uy, uz};
                     double out[7];
-                    m_to_f64(Hp->g, onew, o3, u3, Hp->rel, out);
+                    m_to_f64<false>(Hp->g, dv, onew, o3, u3, Hp->rel, out);
                     Hp->x[hs][hi] = out[0];
                     Hp->y[hs][hi] = out[1];
                     Hp->z[hs][hi] = out[2];
@@ -1072,6 +1083,10 @@ __global__ void k_cells_to_points(int64_t npts, int sx, int sy, const unsigned l
 
 // vmode (relativistic, before the first push): the momentum slots take the
 // loaded velocity and g0 the loaded gamma; otherwise u = gamma v directly.
+// UNIT: unit cells at the origin (no product and sum with 1 and 0). With the
+// truncations and roundings as integer instructions the FP64 pipe no longer
+// bounds it: 80 us for 4,194,304 particles, 207 us with them on that pipe.
+template <bool UNIT>
 __global__ void k_from_f64(Geom g, MState S, int64_t at, int64_t n, const double *x, const double *y,
                            const double *z, const double *vx, const double *vy, const double *vz, const double *gam,
                            int rel, int vmode, float *g0, DevCounters *ctr) {
@@ -1081,7 +1096,7 @@ __global__ void k_from_f64(Geom g, MState S, int64_t at, int64_t n, const double
         int32_t cell;
         float o[3], u[3], gz = 0.0f;
         const int64_t p = at + i;
-        if (!f64_to_m(g, pos, v, ga, rel, vmode, cell, o, u, gz)) {
+        if (!f64_to_m<UNIT>(g, pos, v, ga, rel, vmode, cell, o, u, gz)) {
             atomicOr(&ctr->err, (unsigned long long)ERR_BOUNDS);
             S.cell[p] = -1;
             continue;
@@ -1097,7 +1112,11 @@ __global__ void k_from_f64(Geom g, MState S, int64_t at, int64_t n, const double
     }
 }
 
-__global__ void k_to_f64(Geom g, MState S, int64_t at, int64_t n, double *x, double *y, double *z, double *vx,
+// Bound by the FP64 pipe: a square root, a reciprocal, nine instructions of
+// quotients. 214 us for 4,194,304 relativistic particles (383 us with the
+// conversions and divisions on that pipe).
+template <bool UNIT>
+__global__ void k_to_f64(Geom g, Div3 dv, MState S, int64_t at, int64_t n, double *x, double *y, double *z, double *vx,
                          double *vy, double *vz, double *gam, int rel, const float *g0) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t p = at + i;
@@ -1109,7 +1128,7 @@ __global__ void k_to_f64(Geom g, MState S, int64_t at, int64_t n, double *x, dou
         }
         const float o[3] = {S.ox[p], S.oy[p], S.oz[p]}, u[3] = {S.ux[p], S.uy[p], S.uz[p]};
         double out[7];
-        m_to_f64(g, c, o, u, rel, out);
+        m_to_f64<UNIT>(g, dv, c, o, u, rel, out);
         x[i] = out[0];
         y[i] = out[1];
         z[i] = out[2];
@@ -1937,6 +1956,30 @@ static bool device_accessible(const emoo_handle *h, const void *p) {
     return pt != 0;
 }
 
+static void from_f64(emoo_handle *h, int64_t at, int64_t n, const double *x, const double *y, const double *z,
+                     const double *vx, const double *vy, const double *vz, const double *gam, int vmode) {
+    const int rel = h->info.relativity != 0;
+    h->launches++;
+    if (h->g.unit)
+        k_from_f64<true><<<nblk(n), 256, 0, h->stream>>>(h->g, mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel, vmode,
+                                                         h->g0, h->ctr);
+    else
+        k_from_f64<false><<<nblk(n), 256, 0, h->stream>>>(h->g, mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel, vmode,
+                                                          h->g0, h->ctr);
+}
+
+static void to_f64(emoo_handle *h, int64_t at, int64_t n, double *x, double *y, double *z, double *vx, double *vy,
+                   double *vz, double *gam, const float *g0) {
+    const int rel = h->info.relativity != 0;
+    h->launches++;
+    if (h->g.unit)
+        k_to_f64<true><<<nblk(n), 256, 0, h->stream>>>(h->g, div3(h), mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel,
+                                                       g0);
+    else
+        k_to_f64<false><<<nblk(n), 256, 0, h->stream>>>(h->g, div3(h), mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel,
+                                                        g0);
+}
+
 // n > 0: host FP64 arrays (read in place where the device can, else copied
 // through the payload scratch in chunks); n < 0: |n| particles already
 // staged on the device at the given pointers.
@@ -1956,9 +1999,7 @@ int mixed_from_f64(emoo_handle *h, int64_t at, int64_t n, const double *x, const
     }
     int vmode = rel && h->first_push;
     if (dev) {
-        h->launches++;
-        k_from_f64<<<nblk(n), 256, 0, h->stream>>>(h->g, mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel, vmode,
-                                                   h->g0, h->ctr);
+        from_f64(h, at, n, x, y, z, vx, vy, vz, gam, vmode);
         EMOO_CUDA(cudaGetLastError());
         EMOO_CUDA(cudaStreamSynchronize(h->stream));
         return EMOO_OK;
@@ -1973,10 +2014,7 @@ int mixed_from_f64(emoo_handle *h, int64_t at, int64_t n, const double *x, const
         for (int q = 0; q < 7; q++) {
             if (src[q]) EMOO_CUDA(cudaMemcpyAsync(s + q * m, src[q] + b, bytes, cudaMemcpyHostToDevice, h->stream));
         }
-        h->launches++;
-        k_from_f64<<<nblk(m), 256, 0, h->stream>>>(h->g, mstate(h), at + b, m, s, s + m, s + 2 * m, s + 3 * m,
-                                                   s + 4 * m, s + 5 * m, gam ? s + 6 * m : nullptr, rel, vmode,
-                                                   h->g0, h->ctr);
+        from_f64(h, at + b, m, s, s + m, s + 2 * m, s + 3 * m, s + 4 * m, s + 5 * m, gam ? s + 6 * m : nullptr, vmode);
         EMOO_CUDA(cudaGetLastError());
         EMOO_CUDA(cudaStreamSynchronize(h->stream));
     }
@@ -1985,15 +2023,13 @@ int mixed_from_f64(emoo_handle *h, int64_t at, int64_t n, const double *x, const
 
 int mixed_to_f64(emoo_handle *h, int64_t at, int64_t n, double *x, double *y, double *z, double *vx, double *vy,
                  double *vz, double *gam) {
-    int rel = h->info.relativity != 0;
     const float *g0 = (h->first_push && h->g0) ? h->g0 : nullptr;
     bool direct = true;
     for (const void *q : {(const void *)x, (const void *)y, (const void *)z, (const void *)vx, (const void *)vy,
                           (const void *)vz, (const void *)gam})
         direct = direct && device_accessible(h, q);
     if (direct) {  // written in place (see device_accessible)
-        h->launches++;
-        k_to_f64<<<nblk(n), 256, 0, h->stream>>>(h->g, mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel, g0);
+        to_f64(h, at, n, x, y, z, vx, vy, vz, gam, g0);
         EMOO_CUDA(cudaGetLastError());
         EMOO_CUDA(cudaStreamSynchronize(h->stream));
         return EMOO_OK;
@@ -2002,9 +2038,7 @@ int mixed_to_f64(emoo_handle *h, int64_t at, int64_t n, double *x, double *y, do
     double *s = (double *)h->pay;
     for (int64_t b = 0; b < n; b += chunk) {
         int64_t m = std::min(chunk, n - b);
-        h->launches++;
-        k_to_f64<<<nblk(m), 256, 0, h->stream>>>(h->g, mstate(h), at + b, m, s, s + m, s + 2 * m, s + 3 * m,
-                                                 s + 4 * m, s + 5 * m, s + 6 * m, rel, g0);
+        to_f64(h, at + b, m, s, s + m, s + 2 * m, s + 3 * m, s + 4 * m, s + 5 * m, s + 6 * m, g0);
         EMOO_CUDA(cudaGetLastError());
         double *dst[7] = {x, y, z, vx, vy, vz, gam};
         size_t bytes = sizeof(double) * (size_t)m;
