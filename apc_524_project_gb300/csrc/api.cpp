@@ -1143,7 +1143,12 @@ int emoo_get_particle_fields(emoo_handle *h, int species, int64_t cap, double *e
 }
 
 int emoo_get_field(emoo_handle *h, int id, double *out) {
-    HANDLE_CHECK(h);
+    if (!h) return EMOO_ERR_ARG;
+    EMOO_TRY(set_device(h));
+    // of the fields only rho may be formed from the particles: the others are
+    // read without refreshing a host-resident store (an upload over the host
+    // link, 0.3 ms for 2.2 M particles)
+    if (id == EMOO_RHO) EMOO_TRY(host_store_sync(h));
     if (id < 0 || id >= EMOO_NFIELDS || !out) return EMOO_ERR_ARG;
     if (id == EMOO_RHO) EMOO_TRY(materialize_rho(h));
     size_t b = sizeof(double) * (size_t)h->g.npts;
