@@ -226,7 +226,7 @@ MSnapView handle_view(emoo_handle *h) {
 }
 
 int primal_step_m(emoo_handle *h) {
-    EMOO_TRY(mixed_step(h, h->dtp, 0, FOLD_J));
+    EMOO_TRY(mixed_step(h, h->dtp, FOLD_J));
     h->t += h->dtp;
     h->step_index++;
     return EMOO_OK;

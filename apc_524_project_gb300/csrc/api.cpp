@@ -1473,7 +1473,7 @@ int emoo_step(emoo_handle *h, int nsteps, int64_t counts6[6]) {
             else EMOO_TRY(yee_f64(h, h->dtp));
             EMOO_TRY(execute_bc(h, EMOO_SEND_EB));
         } else {
-            EMOO_TRY(mixed_step(h, h->dtp, 0, fold_what));
+            EMOO_TRY(mixed_step(h, h->dtp, fold_what));
         }
         h->t += h->dtp;
         h->step_index++;

@@ -297,7 +297,7 @@ int mixed_from_f64(emoo_handle *h, int64_t first, int64_t n, const double *x, co
                    const double *vx, const double *vy, const double *vz, const double *gam);
 int mixed_to_f64(emoo_handle *h, int64_t first, int64_t n, double *x, double *y, double *z, double *vx,
                  double *vy, double *vz, double *gam);
-int mixed_step(emoo_handle *h, double dtp, int with_rho, int fold_what);
+int mixed_step(emoo_handle *h, double dtp, int fold_what);
 int mixed_materialize_rho(emoo_handle *h);
 int mixed_sort_keys(emoo_handle *h);
 int mixed_compact_keys(emoo_handle *h);

@@ -45,6 +45,7 @@ struct FieldsF32 {
     float4 *pack = nullptr;  // interpolation pack, 5 float4 per grid point (interior cells filled)
     unsigned long long *wj = nullptr;  // per-cell J deposit sums, 12 int64 per grid point
     unsigned long long *wr = nullptr;  // per-cell rho deposit sums, 8 int64 per grid point
+    bool wj_ghosts_zero = false;  // the J records of ghost cells are zero (only walled moves reach them)
 };
 
 namespace {
@@ -262,38 +263,55 @@ __device__ __forceinline__ float4 edge_coef_true(float f00, float f10, float f11
     return make_float4(f00, f10 - f00, f01 - f00, (f00 - f10) + (f11 - f01));
 }
 
+// A warp packs 32 consecutive cells of a row: each lane forms one cell's five
+// float4, and the warp writes them, staged in shared memory, as one contiguous
+// stretch. With `wj` it also zeroes the cells' J records, which the deposit
+// that follows accumulates into (a fill of its own costs a launch more).
 template <bool CORR>
-__global__ void k_pack_m(MGeom g, MGather P, float4 *__restrict__ pack) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
-    int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
-    int i = blockIdx.z + 1;
-    if (k > g.n[2] || j > g.n[1]) return;
+__global__ void __launch_bounds__(256) k_pack_m(MGeom g, MGather P, float4 *__restrict__ pack, uint4 *wj) {
+    __shared__ float4 stage[8][32 * PACK_F4];
+    const int lane = threadIdx.x, k0 = blockIdx.x * 32 + 1, k = k0 + lane;
+    const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
+    const int i = blockIdx.z + 1;
+    if (j > g.n[1]) return;  // the whole warp
     const int64_t sx = g.sx, sy = g.sy;
-    const int64_t o = (int64_t)i * sx + (int64_t)j * sy + k;
-    const float *Ex = P.E[0], *Ey = P.E[1], *Ez = P.E[2];
-    float4 *dst = pack + o * PACK_F4;
-    auto coef = [](float f00, float f10, float f11, float f01) {
-        return CORR ? edge_coef_true(f00, f10, f11, f01) : edge_coef(f00, f10, f11, f01);
-    };
-    // face term: d0 = S0 - S1/2 over the ghost-offset vertex, S0/2 over the true one
-    auto d0 = [](float s0, float s1) { return CORR ? 0.5f * s0 : s0 - 0.5f * s1; };
-    dst[0] = coef(Ex[o], Ex[o + sy], Ex[o + sy + 1], Ex[o + 1]);
-    dst[1] = coef(Ey[o], Ey[o + 1], Ey[o + sx + 1], Ey[o + sx]);
-    dst[2] = coef(Ez[o], Ez[o + sx], Ez[o + sx + sy], Ez[o + sy]);
-    float s0, s1;
-    float4 b;
-    s0 = P.T[0][o] + P.B[0][o];
-    s1 = P.T[0][o + sx] + P.B[0][o + sx];
-    b.x = d0(s0, s1);
-    b.y = 0.5f * (s1 - s0);
-    s0 = P.T[1][o] + P.B[1][o];
-    s1 = P.T[1][o + sy] + P.B[1][o + sy];
-    b.z = d0(s0, s1);
-    b.w = 0.5f * (s1 - s0);
-    dst[3] = b;
-    s0 = P.T[2][o] + P.B[2][o];
-    s1 = P.T[2][o + 1] + P.B[2][o + 1];
-    dst[4] = make_float4(d0(s0, s1), 0.5f * (s1 - s0), 0.0f, 0.0f);
+    const int64_t row = (int64_t)i * sx + (int64_t)j * sy + k0;
+    const int cells = min(32, g.n[2] - k0 + 1);
+    float4 *st = stage[threadIdx.y];
+    if (k <= g.n[2]) {
+        const int64_t o = row + lane;
+        const float *Ex = P.E[0], *Ey = P.E[1], *Ez = P.E[2];
+        float4 *dst = st + lane * PACK_F4;
+        auto coef = [](float f00, float f10, float f11, float f01) {
+            return CORR ? edge_coef_true(f00, f10, f11, f01) : edge_coef(f00, f10, f11, f01);
+        };
+        // face term: d0 = S0 - S1/2 over the ghost-offset vertex, S0/2 over the true one
+        auto d0 = [](float s0, float s1) { return CORR ? 0.5f * s0 : s0 - 0.5f * s1; };
+        dst[0] = coef(Ex[o], Ex[o + sy], Ex[o + sy + 1], Ex[o + 1]);
+        dst[1] = coef(Ey[o], Ey[o + 1], Ey[o + sx + 1], Ey[o + sx]);
+        dst[2] = coef(Ez[o], Ez[o + sx], Ez[o + sx + sy], Ez[o + sy]);
+        float s0, s1;
+        float4 b;
+        s0 = P.T[0][o] + P.B[0][o];
+        s1 = P.T[0][o + sx] + P.B[0][o + sx];
+        b.x = d0(s0, s1);
+        b.y = 0.5f * (s1 - s0);
+        s0 = P.T[1][o] + P.B[1][o];
+        s1 = P.T[1][o + sy] + P.B[1][o + sy];
+        b.z = d0(s0, s1);
+        b.w = 0.5f * (s1 - s0);
+        dst[3] = b;
+        s0 = P.T[2][o] + P.B[2][o];
+        s1 = P.T[2][o + 1] + P.B[2][o + 1];
+        dst[4] = make_float4(d0(s0, s1), 0.5f * (s1 - s0), 0.0f, 0.0f);
+    }
+    __syncwarp();
+    float4 *out = pack + row * PACK_F4;
+    for (int q = lane; q < cells * PACK_F4; q += 32) out[q] = st[q];
+    if (wj) {
+        uint4 *rec = wj + row * (DEP_JSLOTS / 2);
+        for (int q = lane; q < cells * (DEP_JSLOTS / 2); q += 32) rec[q] = make_uint4(0u, 0u, 0u, 0u);
+    }
 }
 
 // E and B at offsets (ox, oy, oz) of the cell whose pack starts at pk.
@@ -1007,6 +1025,151 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
     }
 }
 
+struct MF3 {
+    float *p[3];
+};
+struct MCF3 {
+    const float *p[3];
+};
+struct MFix4 {
+    long long *p[4];
+};
+struct MF9 {
+    float *p[9];
+};
+
+// ---- J at the points, folded, and the E update, in one pass -----------------
+
+// How a dimension folds J: periodic (both policies), or the corrected
+// policy's mirror fold at reflecting walls.
+struct MFold {
+    int per[3];      // 1: periodic fields
+    int mirror[6];   // 1: corrected policy, external fields, reflecting particles on that side
+};
+
+// One component of J at point (i, j, k), unfolded: the sum of the four record
+// slots that feed it (slot q of cell p - off(q), the inverse of the deposit
+// table; corr: the corrected policy's Jx index, slot 4 from cell p - 1).
+__device__ __forceinline__ unsigned long long j_raw(const unsigned long long *__restrict__ wj, int64_t p, int sx, int sy,
+                                                    int a, bool corr) {
+    auto slot = [&](int64_t c, int k) -> unsigned long long { return c >= 0 ? __ldg(wj + c * DEP_JSLOTS + k) : 0ull; };
+    if (a == 0) return slot(p, 0) + slot(p - sy, 3) + slot(corr ? p - 1 : p - sy, 4) + slot(p - sy - 1, 7);
+    if (a == 1) return slot(p, 1) + slot(p - 1, 6) + slot(p - sx - 1, 8) + slot(p - sx, 10);
+    return slot(p, 2) + slot(p - sy, 5) + slot(p - sx - sy, 9) + slot(p - sx, 11);
+}
+
+// The points whose unfolded values the corrected policy's fold sums into index
+// c of dimension d, for component a: itself and its images, with signs; none
+// where the mirror fold has cleared the value.
+__device__ __forceinline__ int fold_sources(const MGeom &g, const MFold &f, int d, int a, int c, int src[4], int sgn[4]) {
+    const int n = g.n[d];
+    int m = 0;
+    src[m] = c;
+    sgn[m++] = 1;
+    if (f.per[d]) {
+        if (c == n) src[m] = 0, sgn[m++] = 1;
+        if (c == 1) src[m] = n + 1, sgn[m++] = 1;
+        if (c == 2) src[m] = n + 2, sgn[m++] = 1;
+        return m;
+    }
+    const bool normal = a == d;
+    for (int r = 0; r < 2; r++) {
+        if (!f.mirror[2 * d + r]) continue;
+        const int from = normal ? (r ? n + 1 : 0) : (r ? n + 2 : 0), to = normal ? (r ? n : 1) : (r ? n : 2);
+        if (c == from) return 0;
+        if (c == to) src[m] = from, sgn[m++] = normal ? -1 : 1;
+    }
+    return m;
+}
+
+// Jx, Jy, Jz at every grid point from the per-cell records, folded over the
+// boundaries, and E there (E -= dt (curl B_tm1 + 4 pi J), or the electrostatic
+// E = -dt 4 pi J) at the physical points. Every value is formed from the
+// records alone, so the folds need no order among the points: under the
+// reference policy plane 1 of a periodic dimension adds plane n + 1's two
+// transverse components over the physical transverse range; under the
+// corrected one (CORR) the points near a boundary sum their images over all
+// dimensions. Integer sums: the same words as a gather, three folds and the
+// update one after the other, which took five launches and read J again.
+template <bool CORR>
+__global__ void __launch_bounds__(256) k_current_e_m(MGeom g, MFold f, const unsigned long long *__restrict__ wj, MFix4 J,
+                                                     MF3 E, MCF3 T, float dt, float q0, int es, int t1, int t2) {
+    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
+    if (k >= t2 || j >= t1) return;
+    const int sx = (int)g.sx, sy = (int)g.sy;
+    const int64_t o = (int64_t)i * g.sx + (int64_t)j * g.sy + k;
+    const bool phys = i >= 1 && i <= g.n[0] && j >= 1 && j <= g.n[1] && k >= 1 && k <= g.n[2];
+    unsigned long long c[3];
+    if (o >= (int64_t)sx + sy + 1) {
+        // J record of cell c: wj + 12 c (96 bytes, 32-byte aligned)
+        auto rec = [&](int64_t q) { return wj + q * DEP_JSLOTS; };
+        const ulonglong2 g0a = __ldg(reinterpret_cast<const ulonglong2 *>(rec(o)));  // slots 0, 1
+        const unsigned long long g0b = __ldg(rec(o) + 2);
+        const unsigned long long g2a = __ldg(rec(o - sy) + 3);
+        const ulonglong2 g2b = __ldg(reinterpret_cast<const ulonglong2 *>(rec(o - sy) + 4));  // 4, 5
+        const unsigned long long g1 = __ldg(rec(o - 1) + 6);
+        const unsigned long long g3 = __ldg(rec(o - sy - 1) + 7);
+        const unsigned long long g5 = __ldg(rec(o - sx - 1) + 8);
+        const unsigned long long g6 = __ldg(rec(o - sx - sy) + 9);
+        const ulonglong2 g4 = __ldg(reinterpret_cast<const ulonglong2 *>(rec(o - sx) + 10));  // 10, 11
+        const unsigned long long q3 = CORR ? __ldg(rec(o - 1) + 4) : g2b.x;
+        c[0] = g0a.x + g2a + q3 + g3;    // q 0, 1, 3, 2
+        c[1] = g0a.y + g1 + g5 + g4.x;   // q 4, 5, 6, 7
+        c[2] = g0b + g2b.y + g6 + g4.y;  // q 8, 11, 10, 9
+    } else {
+#pragma unroll
+        for (int a = 0; a < 3; a++) c[a] = j_raw(wj, o, sx, sy, a, CORR);
+    }
+    if (!CORR) {
+        if (phys) {
+            if (i == 1 && f.per[0]) {
+                c[1] += j_raw(wj, o + (int64_t)g.n[0] * sx, sx, sy, 1, CORR);
+                c[2] += j_raw(wj, o + (int64_t)g.n[0] * sx, sx, sy, 2, CORR);
+            }
+            if (j == 1 && f.per[1]) {
+                c[0] += j_raw(wj, o + (int64_t)g.n[1] * sy, sx, sy, 0, CORR);
+                c[2] += j_raw(wj, o + (int64_t)g.n[1] * sy, sx, sy, 2, CORR);
+            }
+            if (k == 1 && f.per[2]) {
+                c[0] += j_raw(wj, o + g.n[2], sx, sy, 0, CORR);
+                c[1] += j_raw(wj, o + g.n[2], sx, sy, 1, CORR);
+            }
+        }
+    } else if (i <= 2 || i >= g.n[0] || j <= 2 || j >= g.n[1] || k <= 2 || k >= g.n[2]) {
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            int sa[4], sb[4], sc[4], ga[4], gb[4], gc[4];
+            const int na = fold_sources(g, f, 0, a, i, sa, ga), nb = fold_sources(g, f, 1, a, j, sb, gb),
+                      nc = fold_sources(g, f, 2, a, k, sc, gc);
+            if (na * nb * nc == 1) continue;
+            unsigned long long sum = 0ull;
+            for (int x = 0; x < na; x++)
+                for (int y = 0; y < nb; y++)
+                    for (int z = 0; z < nc; z++) {
+                        const unsigned long long v =
+                            j_raw(wj, (int64_t)sa[x] * g.sx + (int64_t)sb[y] * g.sy + sc[z], sx, sy, a, CORR);
+                        sum += ga[x] * gb[y] * gc[z] < 0 ? 0ull - v : v;
+                    }
+            c[a] = sum;
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) J.p[a][o] = (long long)c[a];
+    if (!phys) return;
+    const float jx = __ll2float_rn((long long)c[0]) * q0, jy = __ll2float_rn((long long)c[1]) * q0,
+                jz = __ll2float_rn((long long)c[2]) * q0;
+    if (es) {
+        E.p[0][o] = -dt * (FOURPI_F * jx);
+        E.p[1][o] = -dt * (FOURPI_F * jy);
+        E.p[2][o] = -dt * (FOURPI_F * jz);
+        return;
+    }
+    const float *Tx = T.p[0], *Ty = T.p[1], *Tz = T.p[2];
+    E.p[0][o] -= dt * ((Ty[o] - Ty[o - 1]) * g.idf[2] - (Tz[o] - Tz[o - sy]) * g.idf[1] + FOURPI_F * jx);
+    E.p[1][o] -= dt * ((Tz[o] - Tz[o - sx]) * g.idf[0] - (Tx[o] - Tx[o - 1]) * g.idf[2] + FOURPI_F * jy);
+    E.p[2][o] -= dt * ((Tx[o] - Tx[o - sy]) * g.idf[1] - (Ty[o] - Ty[o - sx]) * g.idf[0] + FOURPI_F * jz);
+}
+
 // J (what & 1) and rho (what & 2) at every grid point from the per-cell
 // records: point p gathers slot q of cell p - off(q), the inverse of the
 // deposit table. Integer sums, so the result equals committing every run
@@ -1169,12 +1332,6 @@ __global__ void k_fillf(float *a, int64_t n, float v) {
 
 // ---- FP32 grid kernels ---------------------------------------------------
 
-struct MF3 {
-    float *p[3];
-};
-struct MCF3 {
-    const float *p[3];
-};
 struct MJ3 {
     const long long *p[3];
 };
@@ -1259,51 +1416,85 @@ __global__ void k_fold_m(MGeom g, int d, long long *f0, long long *f1, long long
     F[t] += F[s];
 }
 
-// The corrected policy's periodic fold and ghost fill along dim d over the
-// whole (n+3)^2 plane (dimension by dimension, so edge and corner lines
-// follow), as k_periodic_full of the FP64 form: fold f[n] += f[0],
-// f[1] += f[n+1], f[2] += f[n+2] (exact integer adds) on the fixed-point
-// arrays; ghost f[0] = f[n], f[n+1] = f[1], f[n+2] = f[2] on the FP32 ones.
-// One array per blockIdx.z.
-struct MFix4 {
-    long long *p[4];
-};
-struct MF9 {
-    float *p[9];
-};
-
-template <class T>
-__device__ __forceinline__ void periodic_full_line(const MGeom &g, T *F, int d, int r, int q, bool fold) {
-    const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
-    const int n = g.n[d];
-    int c[3];
-    c[o1] = r;
-    c[o2] = q;
-    auto at = [&](int i) -> T & {
-        c[d] = i;
-        return F[(int64_t)c[0] * g.sx + (int64_t)c[1] * g.sy + c[2]];
-    };
-    if (fold) {
-        at(n) += at(0);
-        at(1) += at(n + 1);
-        at(2) += at(n + 2);
-    } else {
-        at(0) = at(n);
-        at(n + 1) = at(1);
-        at(n + 2) = at(2);
-    }
-}
+// The corrected policy's periodic fold along dim d over the whole (n+3)^2
+// plane (dimension by dimension, so edge and corner lines follow), as
+// k_periodic_full of the FP64 form: f[n] += f[0], f[1] += f[n+1],
+// f[2] += f[n+2] (exact integer adds) on the fixed-point arrays. One array per
+// blockIdx.z.
 
 __global__ void k_fold_full_m(MGeom g, MFix4 fl, int d, int t1, int t2) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y * blockDim.y + threadIdx.y;
     if (q >= t2 || r >= t1) return;
-    periodic_full_line(g, fl.p[blockIdx.z], d, r, q, true);
+    const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
+    const int n = g.n[d];
+    long long *F = fl.p[blockIdx.z];
+    int c[3];
+    c[o1] = r;
+    c[o2] = q;
+    auto at = [&](int i) -> long long & {
+        c[d] = i;
+        return F[(int64_t)c[0] * g.sx + (int64_t)c[1] * g.sy + c[2]];
+    };
+    at(n) += at(0);
+    at(1) += at(n + 1);
+    at(2) += at(n + 2);
 }
 
-__global__ void k_ghost_full_m(MGeom g, MF9 fl, int d, int t1, int t2) {
-    const int q = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y * blockDim.y + threadIdx.y;
-    if (q >= t2 || r >= t1) return;
-    periodic_full_line(g, fl.p[blockIdx.z], d, r, q, false);
+// The corrected policy's B half and ghost copies in one pass. B (B half, with
+// `update`): at the physical points, E's forward neighbours across a periodic
+// boundary taken from the physical points they are images of, so that E's
+// ghost values need not be filled between the two halves. Copies: each
+// physical point writes the first nf arrays' values to its own images in the
+// ghost planes (0 <- n, n + 1 <- 1, n + 2 <- 2 along every periodic dimension,
+// over the whole range of walled ones), which no thread reads here. The values
+// are those of the copies dimension by dimension (six launches a step).
+__global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, MF9 fl, int nf, MF3 B, MCF3 T, MCF3 E, float dt, int update,
+                                                   int t0, int t1, int t2) {
+    int c[3] = {(int)blockIdx.z, (int)(blockIdx.y * 8 + threadIdx.y), (int)(blockIdx.x * 32 + threadIdx.x)};
+    const int t[3] = {t0, t1, t2};
+    const int64_t st[3] = {g.sx, g.sy, 1};
+    bool phys = true, edge = false;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        c[d] += g.wrap[d];  // periodic: the physical points only
+        if (c[d] >= (g.wrap[d] ? g.n[d] + 1 : t[d])) return;
+        phys = phys && c[d] >= 1 && c[d] <= g.n[d];
+        edge = edge || (g.wrap[d] && (c[d] <= 2 || c[d] >= g.n[d]));
+    }
+    const int64_t o = c[0] * st[0] + c[1] * st[1] + c[2];
+    if (update && phys) {
+        const float *Ex = E.p[0], *Ey = E.p[1], *Ez = E.p[2];
+        int64_t up[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) up[d] = o + (g.wrap[d] && c[d] == g.n[d] ? (1 - g.n[d]) * st[d] : st[d]);
+        B.p[0][o] = T.p[0][o] + dt * ((Ey[up[2]] - Ey[o]) * g.idf[2] - (Ez[up[1]] - Ez[o]) * g.idf[1]);
+        B.p[1][o] = T.p[1][o] + dt * ((Ez[up[0]] - Ez[o]) * g.idf[0] - (Ex[up[2]] - Ex[o]) * g.idf[2]);
+        B.p[2][o] = T.p[2][o] + dt * ((Ex[up[1]] - Ex[o]) * g.idf[1] - (Ey[up[0]] - Ey[o]) * g.idf[0]);
+    }
+    if (!edge) return;
+    // image offsets along each dimension, the point itself first
+    int64_t im[3][4];
+    int ni[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const int n = g.n[d];
+        int m = 0;
+        im[d][m++] = 0;
+        if (g.wrap[d]) {
+            if (c[d] == n) im[d][m++] = -n * st[d];
+            if (c[d] == 1) im[d][m++] = n * st[d];
+            if (c[d] == 2 || n == 1) im[d][m++] = (n + 2 - c[d]) * st[d];
+        }
+        ni[d] = m;
+    }
+    for (int q = 0; q < nf; q++) {
+        float *F = fl.p[q] + o;
+        const float v = *F;
+        for (int x = 0; x < ni[0]; x++)
+            for (int y = 0; y < ni[1]; y++)
+                for (int z = 0; z < ni[2]; z++)
+                    if (x + y + z) F[im[0][x] + im[1][y] + im[2][z]] = v;
+    }
 }
 
 struct MPlane {
@@ -2049,10 +2240,10 @@ int mixed_to_f64(emoo_handle *h, int64_t at, int64_t n, double *x, double *y, do
     return EMOO_OK;
 }
 
-static int mixed_ghost_full(emoo_handle *h, bool e_only);
+static int mixed_ghost_full(emoo_handle *h);
 
 int mixed_ghost_fill(emoo_handle *h) {
-    if (h->policy == EMOO_POLICY_CORRECTED) return mixed_ghost_full(h, false);
+    if (h->policy == EMOO_POLICY_CORRECTED) return mixed_ghost_full(h);
     // E/B ghost fill through the fixed storage slots, with LightBC planes for
     // external sides, in the reference's dimension order
     MGeom mg = mgeom(h, h->dtp);
@@ -2138,59 +2329,80 @@ __global__ void k_mirror_fold_m(MGeom g, MFix4 fl, int d, int right, int t1, int
     F[ks] = 0;
 }
 
-// The corrected policy's full-range fold (fixed point) or ghost fill (FP32)
-// of n arrays, dimension by dimension: periodic dimensions as images over the
-// whole range; walled ones fold J (fix with Jx, Jy, Jz first) by mirror at
-// reflecting sides and copy nothing (their field sides are LightBC planes).
-static int mixed_periodic_full(emoo_handle *h, const MFix4 *fix, const MF9 *flt, int n) {
-    MGeom mg = mgeom(h, h->dtp);
-    const Geom &g = h->g;
-    dim3 blk(32, 8);
-    for (int d = 0; d < 3; d++) {
-        const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
-        if (h->bc.fbc[2 * d] != FBC_PERIODIC) {
-            const bool j3 = fix && n >= 3 && fix->p[0] == h->mf->J[0];
-            for (int r = 0; r < 2 && j3; r++) {
-                if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
-                dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
-                h->launches++;
-                k_mirror_fold_m<<<grd, blk, 0, h->stream>>>(mg, *fix, d, r, g.tot[o1], g.tot[o2]);
-            }
-            continue;
-        }
-        dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, n);
-        h->launches++;
-        if (fix) k_fold_full_m<<<grd, blk, 0, h->stream>>>(mg, *fix, d, g.tot[o1], g.tot[o2]);
-        else k_ghost_full_m<<<grd, blk, 0, h->stream>>>(mg, *flt, d, g.tot[o1], g.tot[o2]);
-    }
-    EMOO_CUDA(cudaGetLastError());
-    return EMOO_OK;
-}
-
+// The corrected policy's full-range fold, dimension by dimension: periodic
+// dimensions as images over the whole range; walled ones fold J by mirror at
+// reflecting sides.
 static int mixed_fold_full(emoo_handle *h, int what) {
     MFix4 fl = {};
     int n = 0;
     if (what & FOLD_J)
         for (int c = 0; c < 3; c++) fl.p[n++] = h->mf->J[c];
     if (what & FOLD_RHO) fl.p[n++] = h->mf->J[3];
-    return n ? mixed_periodic_full(h, &fl, nullptr, n) : EMOO_OK;
+    if (!n) return EMOO_OK;
+    MGeom mg = mgeom(h, h->dtp);
+    const Geom &g = h->g;
+    dim3 blk(32, 8);
+    for (int d = 0; d < 3; d++) {
+        const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
+        if (h->bc.fbc[2 * d] != FBC_PERIODIC) {
+            for (int r = 0; r < 2 && (what & FOLD_J); r++) {
+                if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
+                dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
+                h->launches++;
+                k_mirror_fold_m<<<grd, blk, 0, h->stream>>>(mg, fl, d, r, g.tot[o1], g.tot[o2]);
+            }
+            continue;
+        }
+        dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, n);
+        h->launches++;
+        k_fold_full_m<<<grd, blk, 0, h->stream>>>(mg, fl, d, g.tot[o1], g.tot[o2]);
+    }
+    EMOO_CUDA(cudaGetLastError());
+    return EMOO_OK;
 }
 
-// E (3) or E, B and B_tm1 (9) ghost planes, corrected policy, then the
-// LightBC planes of external sides (between the Yee halves too, so that the
-// B half reads E at the new time at the boundary planes as at the wrap)
-static int mixed_ghost_full(emoo_handle *h, bool e_only) {
+// LightBC planes of every external side, one launch a dimension (its sides
+// are both external).
+static int mixed_light_planes(emoo_handle *h) {
+    PlaneSet ps[12];
+    int n = 0;
+    for (int s = 0; s < 6; s++) {
+        if (h->bc.fbc[s] != FBC_EXTERNAL) continue;
+        n += light_planes_public(h, s, ps + n);
+        if (n > 6 || h->g.n[s / 2] < 2) {  // of one cell, both sides set the same plane: in order
+            EMOO_TRY(mixed_plane_sets(h, ps, n));
+            n = 0;
+        }
+    }
+    return n ? mixed_plane_sets(h, ps, n) : EMOO_OK;
+}
+
+// Corrected policy: the periodic copies of the first nf of E, B and B_tm1
+// storage (3: E alone; 9: all), after the B half when `update`.
+static int mixed_b_ghost(emoo_handle *h, double dtp, int nf, bool update) {
+    const MGeom mg = mgeom(h, dtp);
+    const Geom &g = h->g;
     MF9 fl = {};
     for (int c = 0; c < 3; c++) fl.p[c] = h->mf->E[c];
     for (int c = 0; c < 6; c++) fl.p[3 + c] = h->mf->Bslot[c];
-    EMOO_TRY(mixed_periodic_full(h, nullptr, &fl, e_only ? 3 : 9));
-    for (int s = 0; s < 6; s++) {
-        if (h->bc.fbc[s] != FBC_EXTERNAL) continue;
-        PlaneSet ps[6];
-        const int n = light_planes_public(h, s, ps);
-        EMOO_TRY(mixed_plane_sets(h, ps, n));
-    }
+    MF3 B = {{mb_role(h, 0), mb_role(h, 1), mb_role(h, 2)}};
+    MCF3 T = {{mt_role(h, 0), mt_role(h, 1), mt_role(h, 2)}};
+    MCF3 E = {{h->mf->E[0], h->mf->E[1], h->mf->E[2]}};
+    int t[3];
+    for (int d = 0; d < 3; d++) t[d] = mg.wrap[d] ? g.n[d] : g.tot[d];
+    dim3 blk(32, 8), grd((t[2] + 31) / 32, (t[1] + 7) / 8, t[0]);
+    h->launches++;
+    k_b_ghost_m<<<grd, blk, 0, h->stream>>>(mg, fl, nf, B, T, E, (float)dtp, update ? 1 : 0, g.tot[0], g.tot[1],
+                                            g.tot[2]);
+    EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
+}
+
+// E, B and B_tm1 ghost planes, corrected policy, then the LightBC planes of
+// external sides.
+static int mixed_ghost_full(emoo_handle *h) {
+    EMOO_TRY(mixed_b_ghost(h, h->dtp, 9, false));
+    return mixed_light_planes(h);
 }
 
 // what: FOLD_J (the two transverse J components), FOLD_RHO, or both
@@ -2224,6 +2436,17 @@ static int mixed_deposit_zero(emoo_handle *h, int mode) {
     const size_t n = (size_t)h->g.npts * sizeof(unsigned long long);
     if (mode != DEP_RHO) EMOO_CUDA(cudaMemsetAsync(h->mf->wj, 0, n * DEP_JSLOTS, h->stream));
     if (mode != DEP_J) EMOO_CUDA(cudaMemsetAsync(h->mf->wr, 0, n * DEP_RSLOTS, h->stream));
+    return EMOO_OK;
+}
+
+// The J records before a step's deposit: the pack that precedes it zeroes the
+// interior cells', so only ghost cells' values that a walled move left (or an
+// empty particle store, which packs nothing) need the fill.
+static int mixed_records_zero(emoo_handle *h) {
+    if (h->np == 0 || !h->mf->wj_ghosts_zero) EMOO_TRY(mixed_deposit_zero(h, DEP_J));
+    bool walled = false;
+    for (int s = 0; s < 6; s++) walled = walled || h->bc.fbc[s] != FBC_PERIODIC;
+    h->mf->wj_ghosts_zero = !(walled && h->policy == EMOO_POLICY_CORRECTED);
     return EMOO_OK;
 }
 
@@ -2273,7 +2496,7 @@ static int mixed_fused(emoo_handle *h, double dtp, int mode, bool push = true, b
                        int store_pre = 0) {
     const int with_rho = mode != DEP_J ? 1 : 0;
     if (h->np > (int64_t)UINT32_MAX - FUSED_BLOCK) return EMOO_ERR_UNSUPPORTED;  // k_fused_m's 32-bit index
-    if (h->np == 0) return mixed_finish_deposit(h, mode);
+    if (h->np == 0) return push ? EMOO_OK : mixed_finish_deposit(h, mode);
     MGeom mg = mgeom(h, dtp);
     MSpecies st = mspecies(h, dtp);
     MGather P;
@@ -2317,8 +2540,9 @@ static int mixed_fused(emoo_handle *h, double dtp, int mode, bool push = true, b
         dim3 blk(32, 8);
         dim3 pg((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
         h->launches++;
-        if (corr) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack);
-        else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack);
+        uint4 *zero = reinterpret_cast<uint4 *>(h->mf->wj);
+        if (corr) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, zero);
+        else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, zero);
         EMOO_CUDA(cudaGetLastError());
     }
     h->launches++;
@@ -2355,10 +2579,54 @@ static int mixed_fused(emoo_handle *h, double dtp, int mode, bool push = true, b
     }
     // g0 stays allocated for later loads; it is read only while first_push is set
     if (first) h->first_push = 0;
-    return mixed_finish_deposit(h, mode);
+    return EMOO_OK;
 }
 
-static int mixed_yee(emoo_handle *h, double dtp, int es) {
+// One step's current and fields from the particles' deposit in the J records
+// (mixed_fused with push): J folded and E, then B, ghost values and LightBC
+// planes. fold_what: FOLD_J, or FOLD_ALL to fold the rho the grid holds too.
+static int mixed_step_fields(emoo_handle *h, double dtp, int fold_what) {
+    const bool corr = h->policy == EMOO_POLICY_CORRECTED;
+    const int es = h->info.electrostatic == 1;
+    const MGeom mg = mgeom(h, dtp);
+    const Geom &g = h->g;
+    MFold f;
+    for (int d = 0; d < 3; d++) f.per[d] = h->bc.fbc[2 * d] == FBC_PERIODIC;
+    for (int s = 0; s < 6; s++) f.mirror[s] = corr && !f.per[s / 2] && h->bc.pbc[s] == PBC_REFLECTING;
+    MFix4 J = {};
+    for (int c = 0; c < 3; c++) J.p[c] = h->mf->J[c];
+    MF3 E = {{h->mf->E[0], h->mf->E[1], h->mf->E[2]}};
+    if (!es) h->bswap ^= 1;  // the member-pointer swap of evolveFields
+    MCF3 T = {{mt_role(h, 0), mt_role(h, 1), mt_role(h, 2)}};
+    dim3 blk(32, 8), all((g.tot[2] + 31) / 32, (g.tot[1] + 7) / 8, g.tot[0]);
+    h->launches++;
+    if (corr)
+        k_current_e_m<true><<<all, blk, 0, h->stream>>>(mg, f, h->mf->wj, J, E, T, (float)dtp, (float)h->mf->q0, es,
+                                                        g.tot[1], g.tot[2]);
+    else
+        k_current_e_m<false><<<all, blk, 0, h->stream>>>(mg, f, h->mf->wj, J, E, T, (float)dtp, (float)h->mf->q0, es,
+                                                         g.tot[1], g.tot[2]);
+    EMOO_CUDA(cudaGetLastError());
+    if (fold_what & FOLD_RHO) EMOO_TRY(mixed_fold(h, FOLD_RHO));
+    if (corr) {
+        // E's planes at the new time before the B half reads them
+        if (!es) EMOO_TRY(mixed_light_planes(h));
+        EMOO_TRY(mixed_b_ghost(h, dtp, 9, !es));
+        return mixed_light_planes(h);
+    }
+    if (!es) {
+        MF3 B = {{mb_role(h, 0), mb_role(h, 1), mb_role(h, 2)}};
+        MCF3 Ec = {{E.p[0], E.p[1], E.p[2]}};
+        dim3 grd((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
+        h->launches++;
+        k_yee_b_m<<<grd, blk, 0, h->stream>>>(mg, B, T, Ec, (float)dtp);
+        EMOO_CUDA(cudaGetLastError());
+    }
+    return mixed_ghost_fill(h);
+}
+
+// emoo_evolve_fields: the Yee update alone, on the J the grid holds.
+int mixed_yee_public(emoo_handle *h, double dtp, int es) {
     MGeom mg = mgeom(h, dtp);
     const Geom &g = h->g;
     dim3 blk(32, 8);
@@ -2375,7 +2643,10 @@ static int mixed_yee(emoo_handle *h, double dtp, int es) {
         k_yee_e_m<<<grd, blk, 0, h->stream>>>(mg, E, T, J, (float)dtp, (float)h->mf->q0);
         // the B half reads E at plane n+1: refreshed first under the corrected
         // policy (time-centred at the periodic wrap, as yee_f64)
-        if (h->policy == EMOO_POLICY_CORRECTED) EMOO_TRY(mixed_ghost_full(h, true));
+        if (h->policy == EMOO_POLICY_CORRECTED) {
+            EMOO_TRY(mixed_b_ghost(h, dtp, 3, false));
+            EMOO_TRY(mixed_light_planes(h));
+        }
         MF3 B = {{mb_role(h, 0), mb_role(h, 1), mb_role(h, 2)}};
         MCF3 Ec = {{E.p[0], E.p[1], E.p[2]}};
         h->launches++;
@@ -2392,22 +2663,15 @@ static int mixed_yee(emoo_handle *h, double dtp, int es) {
 // history row of this step).
 int mixed_step_host(emoo_handle *h, double dtp, int fold_what, int store_pre) {
     if (!h->mhost || (h->info.relativity != 0 && h->first_push)) return EMOO_ERR_STATE;
-    EMOO_TRY(mixed_deposit_zero(h, DEP_J));
+    EMOO_TRY(mixed_records_zero(h));
     EMOO_TRY(mixed_fused(h, dtp, DEP_J, true, true, store_pre));
-    EMOO_TRY(mixed_fold(h, fold_what));
-    EMOO_TRY(mixed_yee(h, dtp, h->info.electrostatic == 1));
-    EMOO_TRY(mixed_ghost_fill(h));
-    return EMOO_OK;
+    return mixed_step_fields(h, dtp, fold_what);
 }
 
-int mixed_step(emoo_handle *h, double dtp, int with_rho, int fold_what) {
-    const int mode = with_rho ? DEP_J_RHO : DEP_J;
-    EMOO_TRY(mixed_deposit_zero(h, mode));
-    EMOO_TRY(mixed_fused(h, dtp, mode));
-    EMOO_TRY(mixed_fold(h, fold_what));
-    EMOO_TRY(mixed_yee(h, dtp, h->info.electrostatic == 1));
-    EMOO_TRY(mixed_ghost_fill(h));
-    return EMOO_OK;
+int mixed_step(emoo_handle *h, double dtp, int fold_what) {
+    EMOO_TRY(mixed_records_zero(h));
+    EMOO_TRY(mixed_fused(h, dtp, DEP_J));
+    return mixed_step_fields(h, dtp, fold_what);
 }
 
 int mixed_sort_keys(emoo_handle *h) {
@@ -2661,8 +2925,8 @@ int mixed_interpolate(emoo_handle *h) {
     dim3 blk(32, 8);
     dim3 pg((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
     h->launches += 2;
-    if (h->policy == EMOO_POLICY_CORRECTED) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack);
-    else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack);
+    if (h->policy == EMOO_POLICY_CORRECTED) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, nullptr);
+    else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, nullptr);
     if (h->np > 0)
         k_interpolate_m<<<nblk(h->np), 256, 0, h->stream>>>(h->mf->pack, mstate(h), h->np, h->cap, h->fcache);
     EMOO_CUDA(cudaGetLastError());
@@ -2687,7 +2951,6 @@ int mixed_materialize_rho(emoo_handle *h) {
 
 int mixed_fold_public(emoo_handle *h) { return mixed_fold(h, FOLD_ALL); }
 
-int mixed_yee_public(emoo_handle *h, double dtp, int es) { return mixed_yee(h, dtp, es); }
 
 // FP32 E, B, B_tm1 and fixed-point J / rho into the FP64 slots (for the FP64
 // diagnostics: Gauss-law residual).
@@ -2740,8 +3003,8 @@ int mixed_ad_particles(emoo_handle *h, const MSnapView &S, const int32_t *cell_a
         dim3 blk(32, 8);
         dim3 pg((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
         h->launches++;
-        if (h->policy == EMOO_POLICY_CORRECTED) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack);
-        else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack);
+        if (h->policy == EMOO_POLICY_CORRECTED) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, nullptr);
+        else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, nullptr);
         EMOO_CUDA(cudaGetLastError());
     }
     MSnapC SC{S.cell, {S.o[0], S.o[1], S.o[2]}, {S.u[0], S.u[1], S.u[2]}};
