@@ -60,6 +60,7 @@ struct MState {
 struct MSpecies {
     int nspec;
     int64_t off[EMOO_NSPEC + 1];
+    uint32_t end[EMOO_NSPEC];  // off[s + 1] for the fused kernel's 32-bit particle index
     float qp[EMOO_NSPEC];    // ((0.5 dt q)/m) UNIT_ACC
     float qdep[EMOO_NSPEC];  // (UNIT_RHOJ q / V) / q0: fixed-point units per unit weight and speed
     float m[EMOO_NSPEC];
@@ -69,6 +70,12 @@ struct MSpecies {
 __device__ __forceinline__ int species_of_m(const MSpecies &st, int64_t p) {
     int s = 0;
     while (s + 1 < st.nspec && p >= st.off[s + 1]) s++;
+    return s;
+}
+
+__device__ __forceinline__ int species_of_m32(const MSpecies &st, uint32_t p) {
+    int s = 0;
+    while (s + 1 < st.nspec && p >= st.end[s]) s++;
     return s;
 }
 
@@ -209,6 +216,18 @@ __host__ __device__ __forceinline__ int dep_pos(int q) {
     return q < 12 ? (int)((DEP_JPOS >> (4 * q)) & 15ull) : (int)((DEP_RPOS >> (4 * (q - 12))) & 15ull);
 }
 
+// The inverse: the contribution q (J: 0..11, rho: 12..19) at a record's slot.
+constexpr unsigned long long DEP_JROW =  // slot 0..11
+    (0ull << 0) | (4ull << 4) | (8ull << 8) | (1ull << 12) | (3ull << 16) | (11ull << 20) | (5ull << 24) |
+    (2ull << 28) | (6ull << 32) | (10ull << 36) | (7ull << 40) | (9ull << 44);
+constexpr unsigned long long DEP_RROW =  // slot 0..7, q - 12
+    (0ull << 0) | (3ull << 4) | (7ull << 8) | (4ull << 12) | (6ull << 16) | (2ull << 20) | (1ull << 24) |
+    (5ull << 28);
+
+__host__ __device__ __forceinline__ int dep_row(bool j, int pos) {
+    return (int)(((j ? DEP_JROW : DEP_RROW) >> (4 * pos)) & 15ull);
+}
+
 // The record layouts and the gather in k_cells_to_points must agree with the
 // deposit table: every slot feeds the point offset of the q placed in it.
 // Checked once per handle.
@@ -223,6 +242,7 @@ bool dep_tables_agree() {
         if (pos < 0 || pos >= (j ? DEP_JSLOTS : DEP_RSLOTS)) return false;
         bool &used = j ? usedj[pos] : usedr[pos];
         if (used || (j ? joff[pos] : roff[pos]) != dep_offset(q, sx, sy)) return false;
+        if (dep_row(j, pos) != (j ? q : q - 12)) return false;
         used = true;
     }
     return true;
@@ -377,6 +397,19 @@ __device__ __forceinline__ int axis_bc(const BCTab &bc, int d, int n, int &i, fl
     return mask;
 }
 
+// rsqrtf and __fdividef(1, x) of a normal x >= 1, the instruction alone: the
+// functions' denormal scaling (four instructions each) has nothing to do there.
+__device__ __forceinline__ float rsqrt_ge1(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_ge1(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
 // The push of k_fused_m on one particle: Vay's pusher (REL) on u = gamma v,
 // or Boris's; u is updated in place and v receives the new velocity. The
 // adjoint kernel recomputes the step with this same function.
@@ -393,7 +426,7 @@ __device__ __forceinline__ void push_m(const float f[6], const float qp, const f
             float g = g0[p];
             mx0 = g * ux; my0 = g * uy; mz0 = g * uz;
         } else {
-            float iv = rsqrtf(1.0f + ux * ux + uy * uy + uz * uz);
+            float iv = rsqrt_ge1(1.0f + ux * ux + uy * uy + uz * uz);
             v0x = ux * iv; v0y = uy * iv; v0z = uz * iv;
             mx0 = ux; my0 = uy; mz0 = uz;
         }
@@ -410,11 +443,11 @@ __device__ __forceinline__ void push_m(const float f[6], const float qp, const f
         float ust = upx * tx + upy * ty + upz * tz;
         // sigma >= 1 (gps >= 1 + tau2), so both radicands are >= 1
         float rad = sigma * sigma + 4.0f * (tau2 + ust * ust);
-        float igi = rsqrtf(0.5f * (sigma + rad * rsqrtf(rad)));
+        float igi = rsqrt_ge1(0.5f * (sigma + rad * rsqrt_ge1(rad)));
         tx *= igi;
         ty *= igi;
         tz *= igi;
-        float sfac = __fdividef(1.0f, 1.0f + tx * tx + ty * ty + tz * tz);
+        float sfac = rcp_ge1(1.0f + tx * tx + ty * ty + tz * tz);
         float ud = ust * igi;
         ux = sfac * (upx + ud * tx + (upy * tz - upz * ty));
         uy = sfac * (upy + ud * ty + (upz * tx - upx * tz));
@@ -691,25 +724,124 @@ __device__ __forceinline__ void vb_pieces_list(const MGeom &g, const BCTab &bc, 
     }
 }
 
+// The 12 J contributions of a particle with weights a, b per axis
+// (src/particles/deposit.cpp:12-62) into column w of the transpose; jx, jy, jz
+// in fixed-point units.
+__device__ __forceinline__ void j_terms(float jx, float jy, float jz, const float a[3], const float b[3], float *w) {
+    w[0 * COL_STRIDE] = jx * a[1] * a[2];
+    w[1 * COL_STRIDE] = jx * b[1] * a[2];
+    w[2 * COL_STRIDE] = jx * b[1] * b[2];
+    w[3 * COL_STRIDE] = jx * a[1] * b[2];
+    w[4 * COL_STRIDE] = jy * a[2] * a[0];
+    w[5 * COL_STRIDE] = jy * b[2] * a[0];
+    w[6 * COL_STRIDE] = jy * b[2] * b[0];
+    w[7 * COL_STRIDE] = jy * a[2] * b[0];
+    w[8 * COL_STRIDE] = jz * a[0] * a[1];
+    w[9 * COL_STRIDE] = jz * b[0] * a[1];
+    w[10 * COL_STRIDE] = jz * b[0] * b[1];
+    w[11 * COL_STRIDE] = jz * a[0] * b[1];
+}
+
+// Commits a warp's columns (col: NQ rows of the transpose; 12: J, 8: rho) to
+// the cells' records `rec`: the FP32 sum, in particle order, of each run of
+// consecutive active particles that share a cell, rounded once to the
+// fixed-point quantum and added with one integer atomic per slot. SPLIT: a run
+// that spans particles 15 and 16 is committed as two parts (two half-warps
+// then walk at once). Called by the whole warp.
+//
+// Either way a record's slots are written by consecutive lanes, so that one
+// instruction touches each of its three (two) sectors once: committing each
+// lane's particle by itself, 12 instructions of 32 scattered words, took 237
+// instead of 183 us a launch (8.4 M particles 19 steps after the sort), L2
+// processing four times the requests.
+//  - Runs of one or two particles (particles that have drifted apart, unsorted
+//    input): pairs are summed in their first column, then all 32 lanes commit
+//    (column, slot) pairs, NQ rounds, skipping the columns that head no run.
+//  - Longer runs: lane q (and q + 16 with SPLIT) walks row q in particle order
+//    and commits at each run's end.
+template <int NQ, bool SPLIT, bool GUARD>
+__device__ __forceinline__ void commit_runs(float *col, int *keys, bool active, int cell, unsigned long long *rec) {
+    constexpr int Q0 = NQ == 12 ? 0 : 12;
+    const int lane = threadIdx.x & 31;
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    if (act == 0u) return;
+    // runs of equal cells (inactive lanes get unique negative keys)
+    const int key = active ? cell : -1 - lane;
+    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != key);
+    if (heads == 0xffffffffu) {
+        keys[lane] = active ? cell : -1;
+        __syncwarp();
+        constexpr int T = NQ == 12 ? 3 : 1;  // the (column, slot) pattern repeats every T rounds
+        constexpr int STEP = 32 * T / NQ;    // columns T rounds cover
+#pragma unroll
+        for (int t = 0; t < T; t++) {
+            const int item = t * 32 + lane, r = item / NQ, pos = item % NQ;
+            unsigned long long *dst = rec + pos;
+            const float *v = col + dep_row(NQ == 12, pos) * COL_STRIDE + r;
+            const int *kk = keys + r;
+#pragma unroll
+            for (int u = 0; u < 32; u += STEP) {
+                const int k = kk[u];
+                if (k >= 0) atomicAdd(dst + (size_t)k * NQ, (unsigned long long)f2ll_rn<GUARD>(v[u]));
+            }
+        }
+        __syncwarp();
+        return;
+    }
+    keys[lane] = active ? cell : -1;
+    if (!active) {
+#pragma unroll
+        for (int q = 0; q < NQ; q++) col[q * COL_STRIDE + lane] = 0.0f;
+    }
+    __syncwarp();
+    // Only the ends of active runs commit: an inactive particle is a run of
+    // its own with a zero column, so skipping its end adds 0 to the next run.
+    const unsigned ends32 = ((heads >> 1) | 0x80000000u | (SPLIT ? 0x8000u : 0u)) & act;
+    const int q = SPLIT ? lane & 15 : lane, half = SPLIT ? lane >> 4 : 0;
+    if (q < NQ) {
+        unsigned long long *dst = rec + dep_pos(Q0 + q);
+        float acc = 0.0f;
+#pragma unroll
+        for (int h = 0; h < (SPLIT ? 1 : 2); h++) {
+            const int first = 16 * (half + h);
+            const float4 *row = reinterpret_cast<const float4 *>(col + q * COL_STRIDE + first);
+            const int *hkeys = keys + first;
+            const unsigned ends = ends32 >> first;
+            float r[16];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 v = row[i];
+                r[4 * i] = v.x, r[4 * i + 1] = v.y, r[4 * i + 2] = v.z, r[4 * i + 3] = v.w;
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i++) {
+                acc += r[i];
+                if ((ends >> i) & 1u) {
+                    atomicAdd(dst + (size_t)hkeys[i] * NQ, (unsigned long long)f2ll_rn<GUARD>(acc));
+                    acc = 0.0f;
+                }
+            }
+        }
+    }
+    __syncwarp();
+}
+
 // Fused gather + push + boundaries + deposit, one thread per particle.
 //
-// Deposit: each lane writes its particle's 20 contributions as a column of a
-// per-warp 20 x 32 shared array; then lane q walks row q, summing the
-// contributions of each run of consecutive particles that share a cell in
-// particle order, and adds each run total, in int64 fixed point, to slot q of
-// the run's cell. The order of every FP32 sum is fixed by the particle order,
-// so the slots are bit-reproducible. A warp whose particles are all in
-// different cells (before the first sort) commits each particle directly.
+// Deposit: each lane writes its particle's 12 J contributions as a column of a
+// per-warp shared array, and commit_runs adds the run totals to the cells'
+// records in int64 fixed point. The order of every FP32 sum is fixed by the
+// particle order, so the slots are bit-reproducible.
 //
 // Division and square roots use the hardware approximations (rsqrtf,
 // __fdividef, relative error a few 2^-24): the form's accuracy is FP32. No
 // conversion instruction runs per particle (see f2ll_rn, cell_step).
 //
-// CORR: the corrected policy - the pack holds true-vertex coefficients, the
-// deposit at the current state uses the weights 1 - o and o, and the time
-// loop's current is the charge-conserving one of vb_pieces_list.
+// CORR: the corrected policy - the pack holds true-vertex coefficients and the
+// current is the charge-conserving one of vb_pieces_list.
 //
-// HOST (with PUSH, after the first push): the particle state is read from and
+// HOST (after the first push): the particle state is read from and
 // written back to the caller's FP64 arrays (Hp) instead of the device store,
 // converted as the loader and readback convert (f64_to_m, m_to_f64), so one
 // launch moves every particle over the host link in both directions at once.
@@ -727,14 +859,13 @@ constexpr int fused_min_blocks() {
     return 256 / FUSED_BLOCK * (CORR || HOST ? 4 : 6);
 }
 
-template <bool REL, bool FIRST, bool PUSH, bool CORR = false, bool HOST = false>
+template <bool REL, bool FIRST, bool CORR = false, bool HOST = false>
 __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
     k_fused_m(MGeom g, Div3 dv, MSpecies st, BCTab bc, const float4 *__restrict__ pack, MState S, int64_t np,
-              MDeposit D, int with_rho, const float *g0, DevCounters *ctr, const MHost *__restrict__ Hp,
-              int store_pre) {
-    __shared__ __align__(16) float s_w[FUSED_WARPS][20 * COL_STRIDE];
+              MDeposit D, const float *g0, DevCounters *ctr, const MHost *__restrict__ Hp, int store_pre) {
+    __shared__ __align__(16) float s_w[FUSED_WARPS][DEP_JSLOTS * COL_STRIDE];
     __shared__ int s_key[FUSED_WARPS][32];
-    constexpr bool VBL = CORR && PUSH;  // the corrected policy's pieces go through a list
+    constexpr bool VBL = CORR;  // the corrected policy's pieces go through a list
     __shared__ float s_pl[VBL ? FUSED_WARPS : 1][DEP_JSLOTS][DEP_LIST + 1];
     __shared__ int s_plk[VBL ? FUSED_WARPS : 1][DEP_LIST];
     // a 32-bit product (mixed_fused refuses 2^32 particles or more): the state
@@ -781,7 +912,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
             c = S.cell[p];
         }
         if (c >= 0) {
-            const int s = species_of_m(st, p);
+            const int s = species_of_m32(st, (uint32_t)p);
             if (!HOST) {
                 ox = S.ox[p], oy = S.oy[p], oz = S.oz[p];
                 ux = S.ux[p], uy = S.uy[p], uz = S.uz[p];
@@ -792,14 +923,8 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
             const int ix0 = ix, iy0 = iy, iz0 = iz;
             const float so[3] = {ox, oy, oz};
             float mv[3] = {0.0f, 0.0f, 0.0f};
-            if (!PUSH) {
-                // deposit at the current state (Particle_Handler::depositRhoJ)
-                float iga = 1.0f;
-                if (REL && !FIRST) iga = rsqrtf(1.0f + ux * ux + uy * uy + uz * uz);
-                vx = ux * iga;
-                vy = uy * iga;
-                vz = uz * iga;
-            } else {
+            bool outside = false;  // of the box, after the boundaries
+            {
                 float f[6];
                 gather_pack(pack + (int64_t)c * PACK_F4, ox, oy, oz, f);
                 push_m<REL, FIRST>(f, st.qp[s], g0, p, ux, uy, uz, vx, vy, vz);
@@ -808,12 +933,30 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
                 mv[0] = nx;
                 mv[1] = ny;
                 mv[2] = nz;
-                cell_step(nx, ix, ox);
-                cell_step(ny, iy, oy);
-                cell_step(nz, iz, oz);
-                mask |= axis_bc(bc, 0, g.n[0], ix, ox, ux, vx);
-                if (!(mask & 64)) mask |= axis_bc(bc, 1, g.n[1], iy, oy, uy, vy);
-                if (!(mask & 64)) mask |= axis_bc(bc, 2, g.n[2], iz, oz, uz, vz);
+                // All three axes by comparisons; a move past a neighbour cell, an
+                // offset that rounds to 1, or a NaN takes cell_step.
+                ox = nx, oy = ny, oz = nz;
+                if (nx >= 1.0f) ox = nx - 1.0f, ix++;
+                if (nx < 0.0f) ox = nx + 1.0f, ix--;
+                if (ny >= 1.0f) oy = ny - 1.0f, iy++;
+                if (ny < 0.0f) oy = ny + 1.0f, iy--;
+                if (nz >= 1.0f) oz = nz - 1.0f, iz++;
+                if (nz < 0.0f) oz = nz + 1.0f, iz--;
+                if (!(nx >= -1.0f && nx < 2.0f && ny >= -1.0f && ny < 2.0f && nz >= -1.0f && nz < 2.0f && ox < 1.0f &&
+                      oy < 1.0f && oz < 1.0f)) {
+                    ix = ix0, iy = iy0, iz = iz0;
+                    cell_step(nx, ix, ox);
+                    cell_step(ny, iy, oy);
+                    cell_step(nz, iz, oz);
+                }
+                outside = (unsigned)(ix - 1) >= (unsigned)g.n[0] || (unsigned)(iy - 1) >= (unsigned)g.n[1] ||
+                          (unsigned)(iz - 1) >= (unsigned)g.n[2];
+                if (outside) {
+                    mask |= axis_bc(bc, 0, g.n[0], ix, ox, ux, vx);
+                    if (!(mask & 64)) mask |= axis_bc(bc, 1, g.n[1], iy, oy, uy, vy);
+                    if (!(mask & 64)) mask |= axis_bc(bc, 2, g.n[2], iz, oz, uz, vz);
+                    outside = ix < 1 || ix > g.n[0] || iy < 1 || iy > g.n[1] || iz < 1 || iz > g.n[2];
+                }
             }
             if (VBL && (mask & 64) && st.deposit[s]) {
                 // an absorbing wall removed the particle: the current of its
@@ -827,7 +970,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
             if (mask & 64) {
                 if (HOST) host_dead(*Hp, hs, hi);
                 else S.cell[p] = -1;
-            } else if (ix < 1 || ix > g.n[0] || iy < 1 || iy > g.n[1] || iz < 1 || iz > g.n[2]) {
+            } else if (outside) {
                 // moved more than a box length in one step: record, drop
                 atomicOr(&ctr->err, (unsigned long long)ERR_BOUNDS);
                 if (HOST) host_dead(*Hp, hs, hi);
@@ -835,7 +978,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
                 mask |= 64;
             } else {
                 onew = ix * (int)g.sx + iy * (int)g.sy + iz;  // < npts < 2^31 (checked in mixed_alloc)
-                if (PUSH && HOST) {
+                if (HOST) {
                     const float o3[3] = {ox, oy, oz}, u3[3] = {ux, uy, uz};
                     double out[7];
                     m_to_f64<false>(Hp->g, dv, onew, o3, u3, Hp->rel, out);
@@ -846,7 +989,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
                     Hp->vy[hs][hi] = out[4];
                     Hp->vz[hs][hi] = out[5];
                     if (Hp->gam[hs]) Hp->gam[hs][hi] = out[6];
-                } else if (PUSH) {
+                } else {
                     S.cell[p] = onew;
                     S.ox[p] = ox;
                     S.oy[p] = oy;
@@ -855,62 +998,20 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
                     S.uy[p] = uy;
                     S.uz[p] = uz;
                 }
-                if (CORR && PUSH && st.deposit[s]) {
+                if (CORR && st.deposit[s]) {
                     active = true;
                     vb_dep = true;
                     vb_i[0] = ix0, vb_i[1] = iy0, vb_i[2] = iz0;
 #pragma unroll
                     for (int a = 0; a < 3; a++) vb_s[a] = so[a], vb_e[a] = mv[a];
                     vb_qd = st.qdep[s];
-                    float *w = col + lane;
-                    if (with_rho) {  // rho at the new position, true-vertex weights
-                        const float qd = st.qdep[s];
-                        const float a[3] = {1.0f - ox, 1.0f - oy, 1.0f - oz}, b[3] = {ox, oy, oz};
-                        w[12 * COL_STRIDE] = qd * a[0] * a[1] * a[2];
-                        w[13 * COL_STRIDE] = qd * b[0] * a[1] * a[2];
-                        w[14 * COL_STRIDE] = qd * b[0] * b[1] * a[2];
-                        w[15 * COL_STRIDE] = qd * a[0] * b[1] * a[2];
-                        w[16 * COL_STRIDE] = qd * a[0] * b[1] * b[2];
-                        w[17 * COL_STRIDE] = qd * b[0] * b[1] * b[2];
-                        w[18 * COL_STRIDE] = qd * b[0] * a[1] * b[2];
-                        w[19 * COL_STRIDE] = qd * a[0] * a[1] * b[2];
-                    }
                 } else if (st.deposit[s]) {
                     active = true;
-                    // deposit weights (src/particles/deposit.cpp:12-62) in
-                    // fixed-point units: (UNIT_RHOJ q / V) v_i (2 - o_j)(2 - o_k) etc.;
-                    // over the true vertex (CORR) 1 - o and o
-                    float a[3] = {2.0f - ox, 2.0f - oy, 2.0f - oz};
-                    float b[3] = {ox - 1.0f, oy - 1.0f, oz - 1.0f};
-                    if (CORR) {
-                        a[0] = 1.0f - ox, a[1] = 1.0f - oy, a[2] = 1.0f - oz;
-                        b[0] = ox, b[1] = oy, b[2] = oz;
-                    }
+                    // in fixed-point units: (UNIT_RHOJ q / V) v_i (2 - o_j)(2 - o_k) etc.
+                    const float a[3] = {2.0f - ox, 2.0f - oy, 2.0f - oz};
+                    const float b[3] = {ox - 1.0f, oy - 1.0f, oz - 1.0f};
                     const float qd = st.qdep[s];
-                    float jx = qd * vx, jy = qd * vy, jz = qd * vz;
-                    float *w = col + lane;
-                    w[0 * COL_STRIDE] = jx * a[1] * a[2];
-                    w[1 * COL_STRIDE] = jx * b[1] * a[2];
-                    w[2 * COL_STRIDE] = jx * b[1] * b[2];
-                    w[3 * COL_STRIDE] = jx * a[1] * b[2];
-                    w[4 * COL_STRIDE] = jy * a[2] * a[0];
-                    w[5 * COL_STRIDE] = jy * b[2] * a[0];
-                    w[6 * COL_STRIDE] = jy * b[2] * b[0];
-                    w[7 * COL_STRIDE] = jy * a[2] * b[0];
-                    w[8 * COL_STRIDE] = jz * a[0] * a[1];
-                    w[9 * COL_STRIDE] = jz * b[0] * a[1];
-                    w[10 * COL_STRIDE] = jz * b[0] * b[1];
-                    w[11 * COL_STRIDE] = jz * a[0] * b[1];
-                    if (with_rho) {
-                        w[12 * COL_STRIDE] = qd * a[0] * a[1] * a[2];
-                        w[13 * COL_STRIDE] = qd * b[0] * a[1] * a[2];
-                        w[14 * COL_STRIDE] = qd * b[0] * b[1] * a[2];
-                        w[15 * COL_STRIDE] = qd * a[0] * b[1] * a[2];
-                        w[16 * COL_STRIDE] = qd * a[0] * b[1] * b[2];
-                        w[17 * COL_STRIDE] = qd * b[0] * b[1] * b[2];
-                        w[18 * COL_STRIDE] = qd * b[0] * a[1] * b[2];
-                        w[19 * COL_STRIDE] = qd * a[0] * a[1] * b[2];
-                    }
+                    j_terms(qd * vx, qd * vy, qd * vz, a, b, col + lane);
                 }
             }
         }
@@ -923,106 +1024,65 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
 #pragma unroll
         for (int q = 0; q < DEP_JSLOTS; q++) wv[q] = 0.0f;
         // a particle the boundaries removed has no new cell: all its pieces go to the list
-        vb_pieces_list<true>(g, bc, PL, D, lane, vb_dep, vb_i[0], vb_i[1], vb_i[2], vb_s, vb_e, vb_qd,
+        vb_pieces_list<!REL>(g, bc, PL, D, lane, vb_dep, vb_i[0], vb_i[1], vb_i[2], vb_s, vb_e, vb_qd,
                              active ? onew : -1, wv);
-        if (PL.n) list_flush<true>(PL, D, lane);
+        if (PL.n) list_flush<!REL>(PL, D, lane);
         if (vb_dep && active) {
 #pragma unroll
             for (int q = 0; q < DEP_JSLOTS; q++) col[q * COL_STRIDE + lane] = wv[q];
         }
     }
     if (__any_sync(0xffffffffu, mask & 63)) count_cross(ctr, mask & 63);
-    const unsigned act = __ballot_sync(0xffffffffu, active);
-    if (act == 0u) return;
-    // runs of equal cells (inactive lanes get unique negative keys)
-    const int key = active ? onew : -1 - lane;
-    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
-    const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != key);
-    keys[lane] = active ? onew : -1;
-    if (!active) {
-#pragma unroll
-        for (int q = 0; q < DEP_SLOTS; q++) col[q * COL_STRIDE + lane] = 0.0f;
-    }
-    __syncwarp();
-    const int nq = with_rho ? DEP_SLOTS : 12;
-    if (heads == 0xffffffffu) {
-        // every particle in a cell of its own (unsorted input)
+    commit_runs<12, true, !REL>(col, keys, active, onew, D.wj);
+}
+
+// Particle_Handler::depositRhoJ at the current state: J (what & 1) and rho
+// (what & 2). gam: the momentum slots hold u = gamma v (else v).
+template <bool CORR>
+__global__ void __launch_bounds__(256) k_deposit_m(MGeom g, Div3 dv, MSpecies st, MState S, int64_t np, MDeposit D, int what,
+                                                   int gam) {
+    __shared__ __align__(16) float s_w[8][20 * COL_STRIDE];
+    __shared__ int s_key[8][32];
+    const int64_t p = (int64_t)(blockIdx.x * blockDim.x + threadIdx.x);
+    const int lane = threadIdx.x & 31;
+    float *col = s_w[threadIdx.x >> 5];
+    int *keys = s_key[threadIdx.x >> 5];
+    bool active = false;
+    int c = -1;
+    if (p < np) {
+        c = S.cell[p];
+        const int s = species_of_m32(st, (uint32_t)p);
+        active = c >= 0 && st.deposit[s];
         if (active) {
-            unsigned long long *dj = D.wj + (size_t)onew * DEP_JSLOTS, *dr = D.wr + (size_t)onew * DEP_RSLOTS;
-#pragma unroll
-            for (int q = 0; q < DEP_SLOTS; q++) {
-                if (q >= nq) break;
-                long long fx = f2ll_rn(col[q * COL_STRIDE + lane]);
-                if (fx != 0) atomicAdd((q < 12 ? dj : dr) + dep_pos(q), (unsigned long long)fx);
+            const float ox = S.ox[p], oy = S.oy[p], oz = S.oz[p], qd = st.qdep[s];
+            float a[3] = {2.0f - ox, 2.0f - oy, 2.0f - oz}, b[3] = {ox - 1.0f, oy - 1.0f, oz - 1.0f};
+            if (CORR) {
+                a[0] = 1.0f - ox, a[1] = 1.0f - oy, a[2] = 1.0f - oz;
+                b[0] = ox, b[1] = oy, b[2] = oz;
             }
-        }
-        return;
-    }
-    const unsigned ends32 = (heads >> 1) | 0x80000000u;  // bit i: particle i ends its run
-    if (nq == DEP_JSLOTS) {
-        // J only (the time loop): lanes 0..11 walk rows 0..11 over particles
-        // 0..15 while lanes 16..27 walk them over particles 16..31, each in
-        // particle order, committing at each run end; a run that spans
-        // particles 15 and 16 is committed as two parts.
-        // Only the ends of active runs commit: an inactive particle is a run of
-        // its own with a zero column, so skipping its end adds 0 to the next run.
-        // With |velocity| < 1 (relativistic), a run total is below 2^39 quanta.
-        const int q = lane & 15, half = lane >> 4;
-        if (q < DEP_JSLOTS) {
-            unsigned long long *dst = D.wj + dep_pos(q);
-            const float4 *row = reinterpret_cast<const float4 *>(col + q * COL_STRIDE + 16 * half);
-            const int *hkeys = keys + 16 * half;
-            const unsigned hact = (act >> (16 * half)) & 0xffffu;
-            const unsigned ends = (((ends32 >> (16 * half)) & 0xffffu) | 0x8000u) & hact;
-            float r[16];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 v = row[i];
-                r[4 * i] = v.x, r[4 * i + 1] = v.y, r[4 * i + 2] = v.z, r[4 * i + 3] = v.w;
+            float *w = col + lane;
+            if (what & 1) {
+                const float ux = S.ux[p], uy = S.uy[p], uz = S.uz[p];
+                float iga = 1.0f;
+                if (gam) iga = rsqrtf(1.0f + ux * ux + uy * uy + uz * uz);
+                j_terms(qd * (ux * iga), qd * (uy * iga), qd * (uz * iga), a, b, w);
             }
-            float acc = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                acc += r[i];
-                if ((ends >> i) & 1u) {
-                    atomicAdd(dst + (size_t)hkeys[i] * DEP_JSLOTS, (unsigned long long)f2ll_rn<!REL>(acc));
-                    acc = 0.0f;
-                }
-            }
-        }
-        return;
-    }
-    if (lane < nq) {
-        // row `lane`: one pass in particle order, committing at each run end;
-        // lanes 0..11 commit one cell's J record together, lanes 12..19 its rho record
-        const bool jrow = lane < 12;
-        unsigned long long *dst = (jrow ? D.wj : D.wr) + dep_pos(lane);
-        const int stride = jrow ? DEP_JSLOTS : DEP_RSLOTS;
-        const float4 *row = reinterpret_cast<const float4 *>(col + lane * COL_STRIDE);
-        const unsigned ends = ends32;
-        float acc = 0.0f;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            float r[16];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const float4 v = row[4 * h + i];
-                r[4 * i] = v.x, r[4 * i + 1] = v.y, r[4 * i + 2] = v.z, r[4 * i + 3] = v.w;
-            }
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                acc += r[i];
-                if ((ends >> (16 * h + i)) & 1u) {  // warp-uniform
-                    const int kk = keys[16 * h + i];
-                    if (kk >= 0) {
-                        // zero totals are committed too: testing costs more than the atomic
-                        atomicAdd(dst + (size_t)kk * stride, (unsigned long long)f2ll_rn(acc));
-                    }
-                    acc = 0.0f;
-                }
+            if (what & 2) {
+                w[12 * COL_STRIDE] = qd * a[0] * a[1] * a[2];
+                w[13 * COL_STRIDE] = qd * b[0] * a[1] * a[2];
+                w[14 * COL_STRIDE] = qd * b[0] * b[1] * a[2];
+                w[15 * COL_STRIDE] = qd * a[0] * b[1] * a[2];
+                w[16 * COL_STRIDE] = qd * a[0] * b[1] * b[2];
+                w[17 * COL_STRIDE] = qd * b[0] * b[1] * b[2];
+                w[18 * COL_STRIDE] = qd * b[0] * a[1] * b[2];
+                w[19 * COL_STRIDE] = qd * a[0] * a[1] * b[2];
             }
         }
     }
+    if (what == 1) commit_runs<12, true, true>(col, keys, active, c, D.wj);
+    if (what == 3) commit_runs<12, false, true>(col, keys, active, c, D.wj);
+    // |rho term| <= 8 quanta 2^32 a particle: a run total is below 2^43
+    if (what & 2) commit_runs<8, false, false>(col + 12 * COL_STRIDE, keys, active, c, D.wr);
 }
 
 struct MF3 {
@@ -1633,7 +1693,7 @@ __global__ void k_compact_keys_m(MSpecies st, const int32_t *cell, int64_t np, i
 
 // ---- differentiation of the mixed step --------------------------------------
 //
-// The adjoint of one step of the loop (k_fused_m<REL, false, true> with J
+// The adjoint of one step of the loop (k_fused_m<REL, false> with J
 // only, then fold, Yee, executeBC(-1)) for one particle, given the particle
 // state before the step (S) and the pack built from the fields before it.
 // The forward is recomputed with k_fused_m's own functions (gather_pack,
@@ -2061,6 +2121,7 @@ MSpecies mspecies(emoo_handle *h, double dtp) {
     st.nspec = t.nspec;
     for (int s = 0; s <= EMOO_NSPEC; s++) st.off[s] = t.off[s];
     for (int s = 0; s < EMOO_NSPEC; s++) {
+        st.end[s] = (uint32_t)t.off[s + 1];
         st.qp[s] = (float)t.qp[s];
         st.qdep[s] = (float)((t.uq[s] / h->g.vol) / h->mf->q0);
         st.m[s] = (float)t.m[s];
@@ -2494,7 +2555,6 @@ static int mixed_finish_deposit(emoo_handle *h, int mode) {
 // sums must have been zeroed (mixed_deposit_zero).
 static int mixed_fused(emoo_handle *h, double dtp, int mode, bool push = true, bool host = false,
                        int store_pre = 0) {
-    const int with_rho = mode != DEP_J ? 1 : 0;
     if (h->np > (int64_t)UINT32_MAX - FUSED_BLOCK) return EMOO_ERR_UNSUPPORTED;  // k_fused_m's 32-bit index
     if (h->np == 0) return push ? EMOO_OK : mixed_finish_deposit(h, mode);
     MGeom mg = mgeom(h, dtp);
@@ -2518,20 +2578,11 @@ static int mixed_fused(emoo_handle *h, double dtp, int mode, bool push = true, b
     dim3 grd((unsigned)nb);
     const bool corr = h->policy == EMOO_POLICY_CORRECTED;
     if (!push) {
+        const int what = mode == DEP_J ? 1 : mode == DEP_RHO ? 2 : 3, gam = rel && !first ? 1 : 0;
+        const unsigned db = (unsigned)((h->np + 255) / 256);
         h->launches++;
-#define EMOO_DEPOSIT_M(R, F, C)                                                                                  \
-    k_fused_m<R, F, false, C><<<grd, FUSED_BLOCK, 0, h->stream>>>(mg, dv, st, h->bc, pk, S, h->np, D, with_rho, g0, \
-                                                                  h->ctr, nullptr, 0)
-        if (corr) {
-            if (rel && first) EMOO_DEPOSIT_M(true, true, true);
-            else if (rel) EMOO_DEPOSIT_M(true, false, true);
-            else EMOO_DEPOSIT_M(false, false, true);
-        } else {
-            if (rel && first) EMOO_DEPOSIT_M(true, true, false);
-            else if (rel) EMOO_DEPOSIT_M(true, false, false);
-            else EMOO_DEPOSIT_M(false, false, false);
-        }
-#undef EMOO_DEPOSIT_M
+        if (corr) k_deposit_m<true><<<db, 256, 0, h->stream>>>(mg, dv, st, S, h->np, D, what, gam);
+        else k_deposit_m<false><<<db, 256, 0, h->stream>>>(mg, dv, st, S, h->np, D, what, gam);
         EMOO_CUDA(cudaGetLastError());
         return mixed_finish_deposit(h, mode);
     }
@@ -2548,11 +2599,10 @@ static int mixed_fused(emoo_handle *h, double dtp, int mode, bool push = true, b
     h->launches++;
     if (h->prof_on) EMOO_CUDA(cudaEventRecord(h->prof_ev[0], h->stream));
 #define EMOO_FUSED_M(R, F, C)                                                                                   \
-    k_fused_m<R, F, true, C><<<grd, FUSED_BLOCK, 0, h->stream>>>(mg, dv, st, h->bc, pk, S, h->np, D, with_rho, g0, \
-                                                                 h->ctr, nullptr, 0)
-#define EMOO_FUSED_HOST(R, C)                                                                                    \
-    k_fused_m<R, false, true, C, true><<<grd, FUSED_BLOCK, 0, h->stream>>>(mg, dv, st, h->bc, pk, S, h->np, D, 0, \
-                                                                           g0, h->ctr, h->mhost, store_pre)
+    k_fused_m<R, F, C><<<grd, FUSED_BLOCK, 0, h->stream>>>(mg, dv, st, h->bc, pk, S, h->np, D, g0, h->ctr, nullptr, 0)
+#define EMOO_FUSED_HOST(R, C)                                                                                      \
+    k_fused_m<R, false, C, true><<<grd, FUSED_BLOCK, 0, h->stream>>>(mg, dv, st, h->bc, pk, S, h->np, D, g0, h->ctr, \
+                                                                     h->mhost, store_pre)
     if (host) {  // the host-resident step: after the first push, J only
         if (corr) {
             if (rel) EMOO_FUSED_HOST(true, true);
