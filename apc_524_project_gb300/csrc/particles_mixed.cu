@@ -610,9 +610,9 @@ __device__ __forceinline__ void list_append(DepList &L, const MDeposit &D, int l
 // and mid-offsets m adds, for each axis a with transverse axes j, k, to its
 // cell's slots 4a .. 4a+3
 //   qd (D_a d_a / dt) ((1-m_j)(1-m_k) + D_j D_k/12, m_j (1-m_k) - .., m_j m_k + .., (1-m_j) m_k - ..).
-// Pieces in the particle's new cell `onew` are summed into w (the run
-// reduction commits them); the others are appended to the warp's list. All
-// lanes of the warp call it (dep false: no pieces).
+// Pieces in the particle's new cell `onew` are summed into its column w of the
+// transpose (the run reduction commits them); the others are appended to the
+// warp's list. All lanes of the warp call it (dep false: no pieces).
 // Crossing times come from comparisons and one fast divide; the cell of a
 // piece from comparisons (no conversion instruction).
 // One straight piece of a path inside one cell, endpoints ua -> ub in the
@@ -638,17 +638,9 @@ __device__ __forceinline__ int vb_piece_cell(const MGeom &g, const int io[3], co
     return ct;
 }
 
-__device__ __forceinline__ void vb_piece(const MGeom &g, const int io[3], const float ua[3], const float ub[3],
-                                         float qd, int &ct, float W[DEP_JSLOTS]) {
-    float m[3], Dd[3];
-    int c[3];
-    ct = vb_piece_cell(g, io, ua, ub, c);
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const float mid = 0.5f * (ua[a] + ub[a]);
-        m[a] = mid - (c[a] < 0 ? -1.0f : (c[a] > 0 ? 1.0f : 0.0f));  // no int-to-float conversion (FP64 pipe)
-        Dd[a] = ub[a] - ua[a];
-    }
+// The twelve terms of a piece of extent Dd and mid-offsets m in its cell.
+__device__ __forceinline__ void vb_terms(const MGeom &g, const float m[3], const float Dd[3], float qd,
+                                         float W[DEP_JSLOTS]) {
 #pragma unroll
     for (int a = 0; a < 3; a++) {
         const int jb = (a + 1) % 3, kb = (a + 2) % 3;
@@ -661,10 +653,42 @@ __device__ __forceinline__ void vb_piece(const MGeom &g, const int io[3], const 
     }
 }
 
+__device__ __forceinline__ void vb_piece(const MGeom &g, const int io[3], const float ua[3], const float ub[3],
+                                         float qd, int &ct, float W[DEP_JSLOTS]) {
+    float m[3], Dd[3];
+    int c[3];
+    ct = vb_piece_cell(g, io, ua, ub, c);
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const float mid = 0.5f * (ua[a] + ub[a]);
+        m[a] = mid - (c[a] < 0 ? -1.0f : (c[a] > 0 ? 1.0f : 0.0f));  // no int-to-float conversion (FP64 pipe)
+        Dd[a] = ub[a] - ua[a];
+    }
+    vb_terms(g, m, Dd, qd, W);
+}
+
+// The whole move of a particle that stays in its cell (s and e in [0, 1)): one
+// piece. False where rounding puts the piece's mid-point on the far face (the
+// general path decides then).
+__device__ __forceinline__ bool vb_whole(const MGeom &g, const float s[3], const float e[3], float qd,
+                                         float W[DEP_JSLOTS]) {
+    float m[3], Dd[3];
+    bool in = true;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const float ub = fmaf(1.0f, e[a] - s[a], s[a]);  // the end as the general path forms it
+        m[a] = 0.5f * (s[a] + ub);
+        Dd[a] = ub - s[a];
+        in = in && m[a] >= 0.0f && m[a] < 1.0f;
+    }
+    vb_terms(g, m, Dd, qd, W);
+    return in;
+}
+
 template <bool GUARD>
 __device__ __forceinline__ void vb_pieces_list(const MGeom &g, const BCTab &bc, DepList &L, const MDeposit &D,
                                                int lane, bool dep, int ix, int iy, int iz, const float s[3],
-                                               const float e[3], float qd, int onew, float w[DEP_JSLOTS]) {
+                                               const float e[3], float qd, int onew, float *w) {
     float t[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -693,7 +717,7 @@ __device__ __forceinline__ void vb_pieces_list(const MGeom &g, const BCTab &bc, 
             vb_piece(g, io, ua, ub, qd, ct, W);
             if (ct == onew) {
 #pragma unroll
-                for (int q = 0; q < DEP_JSLOTS; q++) w[q] += W[q];
+                for (int q = 0; q < DEP_JSLOTS; q++) w[q * COL_STRIDE] += W[q];
             }
         }
         list_append<GUARD>(L, D, lane, valid && ct != onew, ct, W);
@@ -846,17 +870,19 @@ __device__ __forceinline__ void commit_runs(float *col, int *keys, bool active, 
 // converted as the loader and readback convert (f64_to_m, m_to_f64), so one
 // launch moves every particle over the host link in both directions at once.
 // Resident blocks per SM the register budget is cut for, counted in blocks of
-// 256 threads and measured over a 20-step sort interval at 256^3: 6 (40
-// registers, no spills) for the reference policy on the device store, where
-// more warps hide the L2 latency that grows as particles drift between sorts
-// (12.59 against 13.06 ms a launch at 5); 4 (64 registers, no spills) for the
-// corrected policy's pieces (19.23 against 20.01 ms at 5 with 148 bytes of
-// spills, 24.6 ms at 6) and for the host-resident conversions (spills at 5).
-// The same warps in blocks of 128 threads, twice as many blocks, take 12.36
-// ms (blocks of 64: 12.60; of 96: 12.63; of 512: 12.92).
+// 256 threads: 6 (40 registers, no spills) for the reference policy on the
+// device store, where more warps hide the L2 latency that grows as particles
+// drift between sorts (536,870,912 particles, means over a 20-step interval
+// with the commits as they were then: 12.59 against 13.06 ms a launch at 5); 5
+// (48 registers) for the corrected policy, whose warps wait at the move list's
+// barriers (10.0 M particles: 336 us; 365 at 4, 342 at 6 with spills); 4 for
+// the host-resident conversions (spills at 5). The same warps in blocks of 128
+// threads, twice as many blocks, took 12.36 ms (blocks of 64: 12.60; of 96:
+// 12.63; of 512: 12.92); under the corrected policy blocks of 256 take 352 us,
+// of 64 429.
 template <bool CORR, bool HOST>
 constexpr int fused_min_blocks() {
-    return 256 / FUSED_BLOCK * (CORR || HOST ? 4 : 6);
+    return 256 / FUSED_BLOCK * (HOST ? 4 : CORR ? 5 : 6);
 }
 
 template <bool REL, bool FIRST, bool CORR = false, bool HOST = false>
@@ -868,6 +894,15 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
     constexpr bool VBL = CORR;  // the corrected policy's pieces go through a list
     __shared__ float s_pl[VBL ? FUSED_WARPS : 1][DEP_JSLOTS][DEP_LIST + 1];
     __shared__ int s_plk[VBL ? FUSED_WARPS : 1][DEP_LIST];
+    // the block's moves that leave their cell: start, end, charge; old cell,
+    // new cell (-1: removed), owner thread
+    __shared__ float s_mv[VBL ? 7 : 1][VBL ? FUSED_BLOCK : 1];
+    __shared__ int s_mvi[VBL ? 3 : 1][VBL ? FUSED_BLOCK : 1];
+    __shared__ int s_nmv;
+    if (VBL) {
+        if (threadIdx.x == 0) s_nmv = 0;
+        __syncthreads();
+    }
     // a 32-bit product (mixed_fused refuses 2^32 particles or more): the state
     // arrays are then addressed with one wide multiply-add each
     const int64_t p = (int64_t)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -879,7 +914,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
     int onew = 0;
     // the corrected policy's move, for its pieces after the divergent part
     bool vb_dep = false;
-    int vb_i[3] = {0, 0, 0};
+    int vb_c = 0;
     float vb_s[3] = {0.0f, 0.0f, 0.0f}, vb_e[3] = {0.0f, 0.0f, 0.0f}, vb_qd = 0.0f;
     if (p < np) {
         int32_t c;
@@ -962,7 +997,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
                 // an absorbing wall removed the particle: the current of its
                 // whole move still goes in (pieces after the branch)
                 vb_dep = true;
-                vb_i[0] = ix0, vb_i[1] = iy0, vb_i[2] = iz0;
+                vb_c = c;
 #pragma unroll
                 for (int a = 0; a < 3; a++) vb_s[a] = so[a], vb_e[a] = mv[a];
                 vb_qd = st.qdep[s];
@@ -1001,7 +1036,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
                 if (CORR && st.deposit[s]) {
                     active = true;
                     vb_dep = true;
-                    vb_i[0] = ix0, vb_i[1] = iy0, vb_i[2] = iz0;
+                    vb_c = c;
 #pragma unroll
                     for (int a = 0; a < 3; a++) vb_s[a] = so[a], vb_e[a] = mv[a];
                     vb_qd = st.qdep[s];
@@ -1017,20 +1052,60 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
         }
     }
     if (VBL) {
-        // Villasenor-Buneman pieces with the whole warp present: the new
-        // cell's into the column, the others through the warp's list
-        DepList PL{s_pl[threadIdx.x >> 5], s_plk[threadIdx.x >> 5], 0};
-        float wv[DEP_JSLOTS];
+        // A move inside its cell is one piece, into the column at once. The
+        // others - a few lanes of nearly every warp - are listed and split by
+        // the block's first warps together: split in place, every warp issues
+        // the splitting for its few (353 us a launch for 10.0 M particles,
+        // 336 so).
+        bool listed = false;
+        if (vb_dep) {
+            float W[DEP_JSLOTS];
+            listed = true;
+            if (vb_e[0] >= 0.0f && vb_e[0] < 1.0f && vb_e[1] >= 0.0f && vb_e[1] < 1.0f && vb_e[2] >= 0.0f &&
+                vb_e[2] < 1.0f && active)
+                listed = !vb_whole(g, vb_s, vb_e, vb_qd, W);
+            if (!listed) {
 #pragma unroll
-        for (int q = 0; q < DEP_JSLOTS; q++) wv[q] = 0.0f;
-        // a particle the boundaries removed has no new cell: all its pieces go to the list
-        vb_pieces_list<!REL>(g, bc, PL, D, lane, vb_dep, vb_i[0], vb_i[1], vb_i[2], vb_s, vb_e, vb_qd,
-                             active ? onew : -1, wv);
-        if (PL.n) list_flush<!REL>(PL, D, lane);
-        if (vb_dep && active) {
-#pragma unroll
-            for (int q = 0; q < DEP_JSLOTS; q++) col[q * COL_STRIDE + lane] = wv[q];
+                for (int q = 0; q < DEP_JSLOTS; q++) col[q * COL_STRIDE + lane] = W[q];
+            }
         }
+        const unsigned lm = __ballot_sync(0xffffffffu, listed);
+        if (lm) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&s_nmv, __popc(lm));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(lm & lanemask_lt());
+            if (listed) {
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    s_mv[a][at] = vb_s[a];
+                    s_mv[3 + a][at] = vb_e[a];
+                }
+                s_mv[6][at] = vb_qd;
+                s_mvi[0][at] = vb_c;
+                s_mvi[1][at] = active ? onew : -1;  // a removed particle has no new cell: all its pieces go to the list
+                s_mvi[2][at] = threadIdx.x;
+            }
+        }
+        __syncthreads();
+        const int nmv = s_nmv;
+        if ((threadIdx.x & ~31u) < nmv) {  // the whole warp
+            const bool dep = threadIdx.x < nmv;
+            const int at = dep ? threadIdx.x : 0;
+            const float sv[3] = {s_mv[0][at], s_mv[1][at], s_mv[2][at]};
+            const float ev[3] = {s_mv[3][at], s_mv[4][at], s_mv[5][at]};
+            int ix, iy, iz;
+            split_cell(g, dv, s_mvi[0][at], ix, iy, iz);
+            DepList PL{s_pl[threadIdx.x >> 5], s_plk[threadIdx.x >> 5], 0};
+            const int own = s_mvi[2][at];
+            float *w = s_w[own >> 5] + (own & 31);  // the owner's column takes the new cell's pieces
+            if (dep) {
+#pragma unroll
+                for (int q = 0; q < DEP_JSLOTS; q++) w[q * COL_STRIDE] = 0.0f;
+            }
+            vb_pieces_list<!REL>(g, bc, PL, D, lane, dep, ix, iy, iz, sv, ev, s_mv[6][at], s_mvi[1][at], w);
+            if (PL.n) list_flush<!REL>(PL, D, lane);
+        }
+        __syncthreads();
     }
     if (__any_sync(0xffffffffu, mask & 63)) count_cross(ctr, mask & 63);
     commit_runs<12, true, !REL>(col, keys, active, onew, D.wj);
