@@ -3,7 +3,7 @@
 Each CUDA translation unit is compiled separately, in parallel, with the flags it
 needs: the FP64 parity kernels and the sampler with --fmad=false (every multiply
 and add separately rounded, as in the reference's x86-64 build), the mixed-precision
-kernels with contraction allowed.
+kernels and the derivatives with contraction allowed.
 """
 import os
 import shutil
@@ -30,7 +30,7 @@ CUDA_UNITS = [
     ("loader.cu", ["--fmad=false"]),
     ("sort.cu", []),
     ("particles_mixed.cu", ["--fmad=true"]),
-    ("adjoint_f64.cu", ["--fmad=false"]),
+    ("adjoint_f64.cu", []),
     ("adjoint_mixed.cu", []),
 ]
 HOST_UNITS = ["api.cpp", "loader_host.cpp", "input_parser.cpp", "io.cpp"]

@@ -43,23 +43,40 @@ struct Dual {
     double v, d;
 };
 
+// Products and sums of primal values, separately rounded on the device also
+// where the translation unit allows contraction: the step's own words.
+AD_HD double rmul(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    return __dmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+AD_HD double radd(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    return __dadd_rn(a, b);
+#else
+    return a + b;
+#endif
+}
+
 AD_HD Dual mk(double v, double d = 0.0) { return Dual{v, d}; }
 AD_HD double val(double x) { return x; }
 AD_HD double val(const Dual &x) { return x.v; }
-AD_HD Dual operator+(Dual a, Dual b) { return {a.v + b.v, a.d + b.d}; }
-AD_HD Dual operator-(Dual a, Dual b) { return {a.v - b.v, a.d - b.d}; }
+AD_HD Dual operator+(Dual a, Dual b) { return {radd(a.v, b.v), a.d + b.d}; }
+AD_HD Dual operator-(Dual a, Dual b) { return {radd(a.v, -b.v), a.d - b.d}; }
 AD_HD Dual operator-(Dual a) { return {-a.v, -a.d}; }
-AD_HD Dual operator*(Dual a, Dual b) { return {a.v * b.v, a.d * b.v + a.v * b.d}; }
+AD_HD Dual operator*(Dual a, Dual b) { return {rmul(a.v, b.v), a.d * b.v + a.v * b.d}; }
 AD_HD Dual operator/(Dual a, Dual b) {
     const double q = a.v / b.v;
     return {q, (a.d - q * b.d) / b.v};
 }
-AD_HD Dual operator+(Dual a, double b) { return {a.v + b, a.d}; }
-AD_HD Dual operator+(double a, Dual b) { return {a + b.v, b.d}; }
-AD_HD Dual operator-(Dual a, double b) { return {a.v - b, a.d}; }
-AD_HD Dual operator-(double a, Dual b) { return {a - b.v, -b.d}; }
-AD_HD Dual operator*(Dual a, double b) { return {a.v * b, a.d * b}; }
-AD_HD Dual operator*(double a, Dual b) { return {a * b.v, a * b.d}; }
+AD_HD Dual operator+(Dual a, double b) { return {radd(a.v, b), a.d}; }
+AD_HD Dual operator+(double a, Dual b) { return {radd(a, b.v), b.d}; }
+AD_HD Dual operator-(Dual a, double b) { return {radd(a.v, -b), a.d}; }
+AD_HD Dual operator-(double a, Dual b) { return {radd(a, -b.v), -b.d}; }
+AD_HD Dual operator*(Dual a, double b) { return {rmul(a.v, b), a.d * b}; }
+AD_HD Dual operator*(double a, Dual b) { return {rmul(a, b.v), a * b.d}; }
 AD_HD Dual operator/(Dual a, double b) { return {a.v / b, a.d / b}; }
 AD_HD Dual operator/(double a, Dual b) {
     const double q = a / b.v;
@@ -286,7 +303,7 @@ AD_HD void vay_eval(double qp, const T f[6], double dt, T x[3], T v[3], T &gamma
 
 // The intermediates of one Vay step, for its reverse.
 struct VayTape {
-    double up[3], tau[3], tsq, sigma, ustar, gi1, gi, tt[3], s, udott, w[3], vout[3];
+    double up[3], tau[3], tsq, sigma, ustar, gi1, igi, tt[3], s, udott, w[3], vout[3];
 };
 
 // vay_eval<double> keeping its intermediates: the same operations in the
@@ -304,22 +321,23 @@ AD_HD void vay_fwd(double qp, const double f[6], double dt, double x[3], double 
     T.sigma = gps - T.tsq;
     T.ustar = T.up[0] * T.tau[0] + T.up[1] * T.tau[1] + T.up[2] * T.tau[2];
     T.gi1 = ::sqrt(T.sigma * T.sigma + 4.0 * (T.tsq + T.ustar * T.ustar));
-    T.gi = ::sqrt(0.5 * (T.sigma + T.gi1));
+    const double gi = ::sqrt(0.5 * (T.sigma + T.gi1));
+    T.igi = 1.0 / gi;
     AD_UNROLL
-    for (int a = 0; a < 3; a++) T.tt[a] = T.tau[a] / T.gi;
+    for (int a = 0; a < 3; a++) T.tt[a] = T.tau[a] / gi;
     T.s = 1.0 / (1.0 + T.tt[0] * T.tt[0] + T.tt[1] * T.tt[1] + T.tt[2] * T.tt[2]);
-    T.udott = T.ustar / T.gi;
+    T.udott = T.ustar / gi;
     double cr[3];
     cross3(T.up, T.tt, cr);
     AD_UNROLL
     for (int a = 0; a < 3; a++) T.w[a] = T.up[a] + T.udott * T.tt[a] + cr[a];
     AD_UNROLL
     for (int a = 0; a < 3; a++) {
-        T.vout[a] = T.s * T.w[a] / T.gi;
+        T.vout[a] = T.s * T.w[a] / gi;
         v[a] = T.vout[a];
         x[a] = x[a] + dt * v[a];
     }
-    gamma = T.gi;
+    gamma = gi;
 }
 
 // Adjoint of vay_eval from its tape (inputs v_in, g_in, fields f): lx, lv,
@@ -329,9 +347,9 @@ AD_HD void vay_fwd(double qp, const double f[6], double dt, double x[3], double 
 AD_HD void vay_rev_tape(const VayTape &T, double qp, const double f[6], double dt, const double v_in[3], double g_in,
                         double lx[3], double lv[3], double &lg, double lf[6]) {
     const double b[3] = {f[3], f[4], f[5]};
-    const double igi = 1.0 / T.gi, igi1 = 1.0 / T.gi1;
+    const double igi = T.igi, igi1 = 1.0 / T.gi1;
     const double *up = T.up, *tau = T.tau, *tt = T.tt, *w = T.w, *vout = T.vout;
-    const double gi = T.gi, gi1 = T.gi1, s = T.s, udott = T.udott, sigma = T.sigma, ustar = T.ustar;
+    const double s = T.s, udott = T.udott, sigma = T.sigma, ustar = T.ustar;
     double lvo[3];
     AD_UNROLL
     for (int a = 0; a < 3; a++) lvo[a] = lv[a] + dt * lx[a];
@@ -411,8 +429,6 @@ AD_HD void vay_rev_tape(const VayTape &T, double qp, const double f[6], double d
         lf[a] += le[a];
         lf[3 + a] += lb[a];
     }
-    (void)gi;
-    (void)gi1;
 }
 
 // Adjoint of vay_eval at inputs (f, v, gamma): lx, lv, lg hold the output

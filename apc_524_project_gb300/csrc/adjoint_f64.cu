@@ -25,9 +25,11 @@
 //    every `checkpoint_every` steps; each segment is recomputed forward,
 //    storing the state before each of its steps, then reversed.
 //
-// Compiled with --fmad=false like the FP64 kernels, so the dual numbers'
-// primal values and the adjoint's recomputed forward are bit-identical to the
-// primal step, and every cell and boundary decision agrees with it.
+// The dual numbers' primal values and the adjoint's recomputed forward are
+// bit-identical to the primal step, so every cell and boundary decision agrees
+// with it: they use separately rounded operations (ad::rmul / radd, and the
+// step's own functions in f64_particle.cuh). The derivatives may be contracted,
+// which halves their FP64 instructions.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,6 +40,7 @@
 #include "adjoint_fields.cuh"
 #include "dev_common.cuh"
 #include "emoo_internal.h"
+#include "f64_particle.cuh"
 
 namespace emoo {
 
@@ -58,9 +61,7 @@ struct PArr {
 struct CPArr {
     const double *p[7];
 };
-struct FPtrs {
-    const double *E[3], *B[3], *T[3];  // E, B role, B_tm1 role
-};
+using FPtrs = GatherPtrs;  // E, B role, B_tm1 role
 using FOut = adf::FOutT<double>;
 using JPtrs = adf::JPtrsT<double>;
 using Slots6 = adf::Slots6T<double>;
@@ -279,13 +280,13 @@ __global__ void k_tlm_particles(Geom g, SpeciesTab st, BCTab bc, CPArr P, FPtrs 
     }
     const Dual p0[3] = {pos[0], pos[1], pos[2]};
     const int ic[3] = {ix, iy, iz};
-    for (int a = 0; a < 3; a++) ds[a] = pos[a] - (g.x0[a] + g.d[a] * (ic[a] - g.vshift));
+    for (int a = 0; a < 3; a++) ds[a] = pos[a] - ad::radd(g.x0[a], ad::rmul(g.d[a], ic[a] - g.vshift));
     ad::gather_eval(cg, v18, ds, f);
     Dual gam = mk(REL ? P.p[6][p] : 1.0, REL ? dP.p[6][p] : 0.0);
     if (REL) ad::vay_eval(st.qp[s], f, dt, pos, vel, gam);
     else ad::boris_eval(st.qp[s], f, dt, pos, vel);
     if (CORR && st.deposit[s] && dt > 0.0) {
-        const double coef = st.uq[s] / g.vol / dt;
+        const double coef = st.vbc[s];
         vb_tlm(g, dJ, p0, pos, coef);
         exit_tlm(g, bc, dJ, pos, coef);
     }
@@ -299,7 +300,7 @@ __global__ void k_tlm_particles(Geom g, SpeciesTab st, BCTab bc, CPArr P, FPtrs 
             const int64_t o2 = gidx(g, ix, iy, iz);
             const int jc[3] = {ix, iy, iz};
             Dual r[3], c12[12];
-            for (int a = 0; a < 3; a++) r[a] = pos[a] - (g.x0[a] + g.d[a] * jc[a]);
+            for (int a = 0; a < 3; a++) r[a] = pos[a] - ad::radd(g.x0[a], ad::rmul(g.d[a], jc[a]));
             ad::jterms_eval(cg, st.uq[s], r, vel, c12);
             for (int q = 0; q < 12; q++) atomicAdd(dJ.J[q >> 2] + jpoint(g, o2, q), c12[q].d);
         }
@@ -313,96 +314,230 @@ __global__ void k_tlm_particles(Geom g, SpeciesTab st, BCTab bc, CPArr P, FPtrs 
 
 // ---- adjoint particle kernel ---------------------------------------------
 //
+// Adjoint of the current of a move that stays in its cell, the one piece of
+// ad::vb_rev with ta = 0 and tb = 1: o the cell's grid point, m and D its
+// mid-offsets and extent, cd[a] = coef d_a; the derivatives of the ends (cell
+// units) into l0, l1. With A = l0 n_j + l1 m_j, B = l2 n_j + l3 m_j and X =
+// l0 - l1 - l2 + l3 over the axis's four edges (n = 1 - m), the weights'
+// adjoint is n_k A + m_k B + cr X.
+__device__ __forceinline__ void vb_whole_adj(const Geom &g, const JPtrs &LJ, int64_t o, const double m[3],
+                                             const double D[3], const double cd[3], double l0[3], double l1[3]) {
+    const int64_t st[3] = {g.sx, g.sy, 1};
+    double n[3], D12[3], lD[3] = {0.0, 0.0, 0.0}, lm[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        n[a] = 1.0 - m[a];
+        D12[a] = D[a] * (1.0 / 12.0);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const int j = (a + 1) % 3, k = (a + 2) % 3;
+        const double *J = LJ.J[a] + o;
+        const double e0 = J[0], e1 = J[st[j]], e2 = J[st[k]], e3 = J[st[j] + st[k]];
+        const double A = e0 * n[j] + e1 * m[j], B = e2 * n[j] + e3 * m[j];
+        const double d10 = e1 - e0, d32 = e3 - e2, X = d32 - d10;
+        const double w = cd[a] * D[a], wX = w * X;
+        lD[a] += cd[a] * (n[k] * A + m[k] * B + D[j] * D12[k] * X);
+        lD[j] += wX * D12[k];
+        lD[k] += wX * D12[j];
+        lm[j] += w * (n[k] * d10 + m[k] * d32);
+        lm[k] += w * (B - A);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        l0[a] = 0.5 * lm[a] - lD[a];
+        l1[a] = 0.5 * lm[a] + lD[a];
+    }
+}
+
 // P, F: the primal state before the step (from the tape). L: the particle
 // adjoints, after the step on entry, before it on exit. LJ: the adjoint of
 // the deposited current. LF: field adjoints that receive the gather's
-// adjoint (atomics). CORR as in k_tlm_particles.
-template <bool REL, bool CORR>
-__global__ void k_adj_particles(Geom g, SpeciesTab st, BCTab bc, CPArr P, FPtrs F, PArr L, int64_t np, double dt,
-                                JPtrs LJ, FOut LF) {
+// adjoint (atomics). CORR as in k_tlm_particles; UNIT: unit cells at the
+// origin.
+//
+// Bound by the FP64 pipe. The forward is the step's own (f64_particle.cuh),
+// the reverse uses fused multiply-adds. Under the corrected policy a move
+// inside its cell takes vb_whole_adj; the others are listed and worked off by
+// the block together, as k_fused_vb does, and hand their derivatives back.
+// Laser box of 32^3 cells, 262,144 particles in load order, corrected: 338 us
+// a launch, 565 with every path split in place, divisions by gamma, and no
+// fused operations.
+constexpr int ADJ_BLOCK = 128;
+
+template <bool REL, bool CORR, bool UNIT>
+__global__ void __launch_bounds__(ADJ_BLOCK) k_adj_particles(Geom g, SpeciesTab st, BCTab bc, CPArr P, FPtrs F, PArr L,
+                                                             int64_t np, double dt, JPtrs LJ, FOut LF) {
+    __shared__ double s_move[CORR ? 7 : 1][CORR ? ADJ_BLOCK : 1];  // in: ends and coef; out: their derivatives
+    __shared__ int s_n;
+    if (CORR) {
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+    }
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= np) return;
-    const double x = P.p[0][p];
-    if (x != x) return;
-    const int s = species_of(st, p);
-    int ix, iy, iz;
-    cell_of(g, x, P.p[1][p], P.p[2][p], ix, iy, iz);
-    if (!cell_ok(g, ix, iy, iz)) return;
-    const int64_t o = gidx(g, ix, iy, iz);
-    int64_t pt[18];
-    gather_points(g, o, pt);
-    double v18[18];
-    for (int k = 0; k < 12; k++) v18[k] = F.E[k >> 2][pt[k]];
-    for (int k = 12; k < 18; k++) {
-        const int c = (k - 12) >> 1;
-        v18[k] = (F.T[c][pt[k]] + F.B[c][pt[k]]) / 2;
+    int ci[3] = {0, 0, 0}, s = 0;
+    double pos[3] = {0.0, 0.0, 0.0};
+    bool live = false;
+    if (p < np) {
+        pos[0] = P.p[0][p];
+        if (alive(pos[0])) {
+            pos[1] = P.p[1][p], pos[2] = P.p[2][p];
+            locate<UNIT>(g, pos, ci);
+            live = cell_ok(g, ci[0], ci[1], ci[2]);
+        }
     }
-    const CellGeo cg = cell_geo(g);
-    const int ic[3] = {ix, iy, iz};
-    double pos[3], vel[3], ds[3], f[6], p0[3];
-    for (int a = 0; a < 3; a++) {
-        pos[a] = p0[a] = P.p[a][p];
-        vel[a] = P.p[3 + a][p];
-        ds[a] = pos[a] - (g.x0[a] + g.d[a] * (ic[a] - g.vshift));
-    }
-    ad::gather_eval(cg, v18, ds, f);
-    const double v_in[3] = {vel[0], vel[1], vel[2]};
-    const double g_in = REL ? P.p[6][p] : 1.0;
-    double gam = g_in;
-    ad::VayTape vt;
-    if (REL) ad::vay_fwd(st.qp[s], f, dt, pos, vel, gam, vt);
-    else ad::boris_eval(st.qp[s], f, dt, pos, vel);
-    const double p1[3] = {pos[0], pos[1], pos[2]};  // the end of the move, before the boundaries
-    const int flips = bc_t(bc, pos, vel);
-    double lx[3], lv[3], lg = REL ? L.p[6][p] : 0.0;
-    for (int a = 0; a < 3; a++) {
-        lx[a] = L.p[a][p];
-        lv[a] = L.p[3 + a][p];
-    }
-    if (flips < 0) {  // removed: nothing after the step depends on it
-        for (int a = 0; a < 3; a++) lx[a] = lv[a] = 0.0;
-        lg = 0.0;
-    } else {
-        if (!CORR && st.deposit[s]) {
-            int jx, jy, jz;
-            cell_of(g, pos[0], pos[1], pos[2], jx, jy, jz);
-            if (cell_ok(g, jx, jy, jz)) {
-                const int64_t o2 = gidx(g, jx, jy, jz);
-                const int jc[3] = {jx, jy, jz};
-                double r[3], l12[12];
-                for (int a = 0; a < 3; a++) r[a] = pos[a] - (g.x0[a] + g.d[a] * jc[a]);
-                for (int q = 0; q < 12; q++) l12[q] = LJ.J[q >> 2][jpoint(g, o2, q)];
-                ad::jterms_rev(cg, st.uq[s], r, vel, l12, lx, lv);
+    if (!CORR && !live) return;
+    int64_t o = 0;
+    double vel[3], ds[3], e[3], b2[3], E12[12], S6[6], v_in[3], g_in = 1.0;
+    VayStep vs;
+    int flips = 0, at = -1;
+    double lx[3], lv[3], lg = 0.0, lp0[3] = {0.0, 0.0, 0.0};
+    if (live) {
+        s = species_of(st, p);
+        o = gidx(g, ci[0], ci[1], ci[2]);
+        from_vertex<UNIT>(g, ci, pos, ds);
+        gather_cell<UNIT>(g, F, o, ds, e, b2, E12, S6);
+        const double p0[3] = {pos[0], pos[1], pos[2]};
+#pragma unroll
+        for (int a = 0; a < 3; a++) v_in[a] = vel[a] = P.p[3 + a][p];
+        if (REL) {
+            double gam = g_in = P.p[6][p];
+            vay_push<ANY>(st.qp[s], st.hqp[s], e, b2, dt, pos, vel, gam, vs);
+        } else {
+            boris_push<ANY>(st.qp[s], st.hqp[s], e, b2, dt, pos, vel);
+        }
+        const double p1[3] = {pos[0], pos[1], pos[2]};  // the end of the move, before the boundaries
+        const bool hit = maybe_crossed(bc, pos);
+        double vb[3] = {vel[0], vel[1], vel[2]};  // after the boundaries
+        if (hit) flips = bc_t(bc, pos, vb);
+        if (REL) lg = L.p[6][p];
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            lx[a] = L.p[a][p];
+            lv[a] = L.p[3 + a][p];
+        }
+        if (flips < 0) {  // removed: nothing after the step depends on it
+#pragma unroll
+            for (int a = 0; a < 3; a++) lx[a] = lv[a] = 0.0;
+            lg = 0.0;
+        } else {
+            if (!CORR && st.deposit[s]) {
+                int jc[3];
+                locate<UNIT>(g, pos, jc);
+                if (cell_ok(g, jc[0], jc[1], jc[2])) {
+                    const int64_t o2 = gidx(g, jc[0], jc[1], jc[2]);
+                    double r[3], l12[12];
+                    from_vertex<UNIT>(g, jc, pos, r);
+#pragma unroll
+                    for (int q = 0; q < 12; q++) l12[q] = LJ.J[q >> 2][jpoint(g, o2, q)];
+                    ad::jterms_rev(cell_geo(g), st.uq[s], r, vb, l12, lx, lv);
+                }
+            }
+#pragma unroll
+            for (int a = 0; a < 3; a++)
+                if ((flips >> a) & 1) {
+                    lx[a] = -lx[a];
+                    lv[a] = -lv[a];
+                }
+        }
+        if (CORR && st.deposit[s] && dt > 0.0) {  // the current of the move, also for a removed particle
+            const double coef = st.vbc[s];
+            double u0[3], u1[3];
+            if (leaves_cell<UNIT>(g, ci, p0, p1, u0, u1) || hit) {
+                at = atomicAdd(&s_n, 1);
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    s_move[a][at] = p0[a];
+                    s_move[3 + a][at] = p1[a];
+                }
+                s_move[6][at] = coef;
+            } else {
+                double m[3], D[3], cd[3], l1[3];
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    D[a] = u1[a] - u0[a];
+                    m[a] = 0.5 * D[a] + (UNIT ? ds[a] : u0[a] - f64_of_int(ci[a] - 1));
+                    cd[a] = UNIT ? coef : coef * g.d[a];
+                }
+                vb_whole_adj(g, LJ, o, m, D, cd, lp0, l1);
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    if (!UNIT) lp0[a] *= g.id[a];
+                    lx[a] += UNIT ? l1[a] : l1[a] * g.id[a];
+                }
             }
         }
-        for (int a = 0; a < 3; a++)
-            if ((flips >> a) & 1) {
-                lx[a] = -lx[a];
-                lv[a] = -lv[a];
+    }
+    if (CORR) {
+        __syncthreads();
+        if ((int)threadIdx.x < s_n) {
+            const int i = threadIdx.x;
+            const double a0[3] = {s_move[0][i], s_move[1][i], s_move[2][i]};
+            const double a1[3] = {s_move[3][i], s_move[4][i], s_move[5][i]};
+            double l0[3] = {0.0, 0.0, 0.0}, l1[3] = {0.0, 0.0, 0.0};
+            vb_adj(g, LJ, a0, a1, s_move[6][i], l0, l1);
+            exit_adj(g, bc, LJ, a1, s_move[6][i], l1);
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                s_move[a][i] = l0[a];
+                s_move[3 + a][i] = l1[a];
             }
+        }
+        __syncthreads();
+        if (!live) return;
+        if (at >= 0) {
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                lp0[a] = s_move[a][at];
+                lx[a] += s_move[3 + a][at];
+            }
+        }
     }
-    double lp0[3] = {0.0, 0.0, 0.0};
-    if (CORR && st.deposit[s] && dt > 0.0) {  // the current of the move, also for a removed particle
-        const double coef = st.uq[s] / g.vol / dt;
-        double lp1[3] = {0.0, 0.0, 0.0};
-        vb_adj(g, LJ, p0, p1, coef, lp0, lp1);
-        exit_adj(g, bc, LJ, p1, coef, lp1);
-        for (int a = 0; a < 3; a++) lx[a] += lp1[a];
-    }
+    const double f[6] = {e[0], e[1], e[2], 0.5 * b2[0], 0.5 * b2[1], 0.5 * b2[2]};
     double lf[6] = {0, 0, 0, 0, 0, 0};
-    if (REL) ad::vay_rev_tape(vt, st.qp[s], f, dt, v_in, g_in, lx, lv, lg, lf);
-    else ad::boris_rev(st.qp[s], f, dt, v_in, lx, lv, lf);
-    double l18[18] = {0}, lds[3] = {0, 0, 0};
-    ad::gather_rev(cg, v18, ds, lf, l18, lds);
-    for (int k = 0; k < 12; k++)
-        if (l18[k] != 0.0) atomicAdd(LF.E[k >> 2] + pt[k], l18[k]);
-    for (int k = 12; k < 18; k++) {
-        const int c = (k - 12) >> 1;
-        if (l18[k] != 0.0) {
-            atomicAdd(LF.B[c] + pt[k], 0.5 * l18[k]);
-            atomicAdd(LF.T[c] + pt[k], 0.5 * l18[k]);
+    if (REL) {
+        ad::VayTape vt;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            vt.up[a] = vs.up[a], vt.tau[a] = vs.tau[a], vt.tt[a] = vs.tt[a], vt.w[a] = vs.w[a];
+            vt.vout[a] = vel[a];
         }
+        vt.tsq = vs.tsq, vt.sigma = vs.sigma, vt.ustar = vs.ustar, vt.gi1 = vs.gi1, vt.igi = vs.igi;
+        vt.s = vs.s, vt.udott = vs.udott;
+        ad::vay_rev_tape(vt, st.qp[s], f, dt, v_in, g_in, lx, lv, lg, lf);
+    } else {
+        ad::boris_rev(st.qp[s], f, dt, v_in, lx, lv, lf);
     }
+    // the gather: its field inputs by atomics, the offsets into lx
+    const int64_t str[3] = {g.sx, g.sy, 1};
+    double w[3], lds[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < 3; i++) w[i] = (UNIT ? 1.0 : g.d[i]) - ds[i];
+    auto add = [](double *to, double v) {
+        if ((unsigned long long)__double_as_longlong(v) << 1) atomicAdd(to, v);  // v != 0
+    };
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int j = (i + 1) % 3, k = (i + 2) % 3;
+        const double *v = E12 + 4 * i, *S = S6 + 2 * i;
+        const double ls = UNIT ? lf[i] : lf[i] * g.iarea[i];
+        const double tw = ls * w[k], tr = ls * ds[k];
+        double *E = LF.E[i] + o;
+        add(E, tw * w[j]);
+        add(E + str[j], tw * ds[j]);
+        add(E + str[j] + str[k], tr * ds[j]);
+        add(E + str[k], tr * w[j]);
+        lds[j] += tw * (v[1] - v[0]) + tr * (v[2] - v[3]);
+        lds[k] += ls * (w[j] * (v[3] - v[0]) + ds[j] * (v[2] - v[1]));
+        const double lb = 0.5 * (UNIT ? lf[3 + i] : lf[3 + i] * g.id[i]);  // half for B, half for B_tm1
+        const double b0 = lb * w[i], b1 = lb * ds[i];
+        add(LF.B[i] + o, b0);
+        add(LF.T[i] + o, b0);
+        add(LF.B[i] + o + str[i], b1);
+        add(LF.T[i] + o + str[i], b1);
+        lds[i] += lb * (S[1] - S[0]);
+    }
+#pragma unroll
     for (int a = 0; a < 3; a++) {
         L.p[a][p] = lx[a] + lds[a] + lp0[a];
         L.p[3 + a][p] = lv[a];
@@ -848,11 +983,18 @@ static int periodic_full_adj(emoo_handle *h, double *const *lslot, const int *id
 template <bool REL>
 static void launch_adj(emoo_handle *h, bool corr, const SpeciesTab &st, CPArr P, FPtrs F, PArr LP, int64_t np,
                        JPtrs LJ, FOut LF) {
-    const int nb = pblocks_all(np);
-    if (corr)
-        k_adj_particles<REL, true><<<nb, 256, 0, h->stream>>>(h->g, st, h->bc, P, F, LP, np, h->dtp, LJ, LF);
-    else
-        k_adj_particles<REL, false><<<nb, 256, 0, h->stream>>>(h->g, st, h->bc, P, F, LP, np, h->dtp, LJ, LF);
+    const int nb = (int)((np + ADJ_BLOCK - 1) / ADJ_BLOCK);
+    if (np == 0) return;
+#define EMOO_ADJ(C, U) \
+    k_adj_particles<REL, C, U><<<nb, ADJ_BLOCK, 0, h->stream>>>(h->g, st, h->bc, P, F, LP, np, h->dtp, LJ, LF)
+    if (corr) {
+        if (h->g.unit) EMOO_ADJ(true, true);
+        else EMOO_ADJ(true, false);
+    } else {
+        if (h->g.unit) EMOO_ADJ(false, true);
+        else EMOO_ADJ(false, false);
+    }
+#undef EMOO_ADJ
 }
 
 // adjoint of one step, given the state before it (snapshot S)

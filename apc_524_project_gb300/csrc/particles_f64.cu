@@ -23,7 +23,7 @@
 
 #include "dev_common.cuh"
 #include "emoo_internal.h"
-#include "f64_ops.cuh"
+#include "f64_particle.cuh"
 
 namespace emoo {
 
@@ -31,12 +31,6 @@ double *role_b(emoo_handle *h, int c);
 double *role_t(emoo_handle *h, int c);
 
 namespace {
-
-struct GatherPtrs {
-    const double *E[3];
-    const double *B[3];  // current B role
-    const double *T[3];  // B_tm1 role
-};
 
 struct DepositPtrs {
     double *J[3];
@@ -46,119 +40,6 @@ struct DepositPtrs {
 struct PState {
     double *x, *y, *z, *vx, *vy, *vz, *g;
 };
-
-// A position's cell index (dev_common's cell_of, getCellID's truncation) on
-// each axis, and the position relative to the cell's vertex x0 + d (i -
-// vshift). UNIT: unit cells at the origin.
-template <bool UNIT>
-__device__ __forceinline__ void locate(const Geom &g, const double p[3], int c[3]) {
-#pragma unroll
-    for (int a = 0; a < 3; a++) c[a] = f64_trunc(UNIT ? p[a] : (p[a] - g.x0[a]) * g.id[a]) + 1;
-}
-
-template <bool UNIT>
-__device__ __forceinline__ void from_vertex(const Geom &g, const int c[3], const double p[3], double ds[3]) {
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        const double i = f64_of_int(c[a] - g.vshift);
-        ds[a] = p[a] - (UNIT ? i : g.x0[a] + g.d[a] * i);
-    }
-}
-
-// Grid::getFieldInterpolatorVec (src/grid/oGrid.cpp:153-197) and
-// Interpolator::interpolate_fields (src/particles/interpolate.cpp:11-47) for a
-// particle in the cell at grid point o, ds from its vertex. e: the electric
-// field; b2: twice the magnetic field (the halves of the averages of B and
-// B_tm1 are exact, so the pushers take them where they cost nothing).
-template <bool UNIT>
-__device__ __forceinline__ void gather_cell(const Geom &g, const GatherPtrs &P, int64_t o, const double ds[3],
-                                            double e[3], double b2[3]) {
-    const int64_t st[3] = {g.sx, g.sy, 1};
-    double w[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) w[i] = (UNIT ? 1.0 : g.d[i]) - ds[i];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const int j = (i + 1) % 3, k = (i + 2) % 3;
-        const double *E = P.E[i] + o, *B = P.B[i] + o, *T = P.T[i] + o;
-        double s = w[j] * w[k] * E[0];
-        s += ds[j] * w[k] * E[st[j]];
-        s += ds[j] * ds[k] * E[st[j] + st[k]];
-        s += w[j] * ds[k] * E[st[k]];
-        const double b = w[i] * (T[0] + B[0]) + ds[i] * (T[st[i]] + B[st[i]]);
-        e[i] = UNIT ? s : ddiv(s, g.area[i], g.iarea[i], g.area_p2[i]);
-        b2[i] = UNIT ? b : ddiv(b, g.d[i], g.id[i], g.p2[i]);
-    }
-}
-
-// What a kernel's instance may take for granted: unit cells at the origin,
-// and with them a time step that is a power of two.
-enum { ANY = 0, UNIT_CELLS = 1, UNIT_DT2 = 2 };
-
-// x + dt v; with dt a power of two the product is exact and one fused
-// instruction gives the same sum.
-template <int MODE>
-__device__ __forceinline__ double advance(double x, double dt, double v) {
-    return MODE == UNIT_DT2 ? __fma_rn(dt, v, x) : x + dt * v;
-}
-
-// Boris::Step, src/pusher/boris.cpp:33-85 (q_p precomputed per species, hq
-// half of it), on e and b2 = 2 B: hq b2 = q_p B, and 2 / (1 + q_p q_p B^2)
-// from the same scaled words.
-template <int MODE>
-__device__ __forceinline__ void boris_push(double q_p, double hq, const double e[3], const double b2[3], double dt,
-                                           double p[3], double v[3]) {
-    const double ex = e[0], ey = e[1], ez = e[2];
-    double tx = hq * b2[0], ty = hq * b2[1], tz = hq * b2[2];
-    double bsqr4 = b2[0] * b2[0] + b2[1] * b2[1] + b2[2] * b2[2];
-    double tsqr = 2.0 / (1.0 + hq * hq * bsqr4);
-    double sx = tsqr * tx, sy = tsqr * ty, sz = tsqr * tz;
-    const double qex = q_p * ex, qey = q_p * ey, qez = q_p * ez;
-    double v_mx = v[0] + qex, v_my = v[1] + qey, v_mz = v[2] + qez;
-    double v_ix = v_mx + v_my * tz - v_mz * ty;
-    double v_iy = v_my + v_mz * tx - v_mx * tz;
-    double v_iz = v_mz + v_mx * ty - v_my * tx;
-    double v_px = v_mx + v_iy * sz - v_iz * sy;
-    double v_py = v_my + v_iz * sx - v_ix * sz;
-    double v_pz = v_mz + v_ix * sy - v_iy * sx;
-    v[0] = v_px + qex;
-    v[1] = v_py + qey;
-    v[2] = v_pz + qez;
-#pragma unroll
-    for (int a = 0; a < 3; a++) p[a] = advance<MODE>(p[a], dt, v[a]);
-}
-
-// Relativistic_Boris::Step (Vay), src/pusher/relativisticBoris.cpp:53-140, on
-// e and b2 = 2 B: hq b2 = q_p B; e + v x B as one fused instruction with the
-// exact half of v x b2; sigma^2 + 4 (..) likewise.
-template <int MODE>
-__device__ __forceinline__ void vay_push(double q_p, double hq, const double e[3], const double b2[3], double dt,
-                                         double p[3], double v[3], double &gamma) {
-    const double bx = b2[0], by = b2[1], bz = b2[2];
-    double vXbx = v[1] * bz - v[2] * by, vXby = v[2] * bx - v[0] * bz, vXbz = v[0] * by - v[1] * bx;
-    double uhx = gamma * v[0] + q_p * __fma_rn(0.5, vXbx, e[0]);
-    double uhy = gamma * v[1] + q_p * __fma_rn(0.5, vXby, e[1]);
-    double uhz = gamma * v[2] + q_p * __fma_rn(0.5, vXbz, e[2]);
-    double upx = uhx + q_p * e[0], upy = uhy + q_p * e[1], upz = uhz + q_p * e[2];
-    double gammap_sq = 1.0 + upx * upx + upy * upy + upz * upz;
-    double taux = hq * bx, tauy = hq * by, tauz = hq * bz;
-    double tau_sq = taux * taux + tauy * tauy + tauz * tauz;
-    double sigma = gammap_sq - tau_sq;
-    double ustar = upx * taux + upy * tauy + upz * tauz;
-    double gi = sqrt(__fma_rn(4.0, tau_sq + ustar * ustar, sigma * sigma));
-    gi = sqrt(f64_half(sigma + gi));
-    const F64Quot dg = f64_divisor(gi);
-    double tx = f64_quot(taux, dg), ty = f64_quot(tauy, dg), tz = f64_quot(tauz, dg);
-    double s = 1.0 / (1.0 + tx * tx + ty * ty + tz * tz);
-    double udott = f64_quot(ustar, dg);
-    double upXt_x = upy * tz - upz * ty, upXt_y = upz * tx - upx * tz, upXt_z = upx * ty - upy * tx;
-    v[0] = f64_quot(s * (upx + udott * tx + upXt_x), dg);
-    v[1] = f64_quot(s * (upy + udott * ty + upXt_y), dg);
-    v[2] = f64_quot(s * (upz + udott * tz + upXt_z), dg);
-#pragma unroll
-    for (int a = 0; a < 3; a++) p[a] = advance<MODE>(p[a], dt, v[a]);
-    gamma = gi;
-}
 
 // The six particle boundaries applied to one particle in the reference's
 // side order (src/particles/particle_handler.cpp:287-295). A periodic side's
@@ -327,19 +208,6 @@ __device__ __forceinline__ void commit_deposit(const Geom &g, const DepositPtrs 
     __syncwarp();
 }
 
-// Whether apply_bc may find a side crossed, from integer comparisons: true
-// for every crossing, and for a -0 against a wall at 0 or a NaN, where
-// apply_bc then finds none.
-__device__ __forceinline__ bool maybe_crossed(const BCTab &bc, const double p[3]) {
-    bool hit = false;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const long long k = f64_key(p[d]);
-        hit = hit || k < f64_key(bc.xmin[d]) || k > f64_key(bc.xmax[d]);
-    }
-    return hit;
-}
-
 __device__ __forceinline__ void count_crossings(DevCounters *ctr, int mask) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -348,8 +216,6 @@ __device__ __forceinline__ void count_crossings(DevCounters *ctr, int mask) {
         if (lane == 0 && b) atomicAdd(&ctr->cross[s], (unsigned long long)__popc(b));
     }
 }
-
-__device__ __forceinline__ bool alive(double x) { return f64_not_nan(x); }
 
 // emoo_interpolate: per-particle field cache (Particle::field).
 __global__ void k_interpolate(Geom g, GatherPtrs P, PState S, int64_t np, int64_t cap, double *fc, DevCounters *ctr) {
@@ -363,9 +229,9 @@ __global__ void k_interpolate(Geom g, GatherPtrs P, PState S, int64_t np, int64_
         atomicOr(&ctr->err, (unsigned long long)ERR_BOUNDS);
         return;
     }
-    double ds[3], e[3], b2[3];
+    double ds[3], e[3], b2[3], E12[12], S6[6];
     from_vertex<false>(g, c, pos, ds);
-    gather_cell<false>(g, P, gidx(g, c[0], c[1], c[2]), ds, e, b2);
+    gather_cell<false>(g, P, gidx(g, c[0], c[1], c[2]), ds, e, b2, E12, S6);
 #pragma unroll
     for (int q = 0; q < 3; q++) {
         fc[q * cap + p] = e[q];
@@ -390,7 +256,8 @@ __global__ void k_push_cached(SpeciesTab st, PState S, int64_t np, int64_t cap, 
     double v[3] = {S.vx[p], S.vy[p], S.vz[p]};
     if (rel) {
         double ga = S.g[p];
-        vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga);
+        VayStep vt;
+        vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga, vt);
         S.g[p] = ga;
     } else {
         boris_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v);
@@ -574,16 +441,17 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, 
             if (!cell_ok(g, ci[0], ci[1], ci[2])) {
                 atomicOr(&ctr->err, (unsigned long long)ERR_BOUNDS);
             } else {
-                double ds[3], e[3], b2[3];
+                double ds[3], e[3], b2[3], E12[12], S6[6];
                 from_vertex<UNIT>(g, ci, pos, ds);
                 o = gidx(g, ci[0], ci[1], ci[2]);
-                gather_cell<UNIT>(g, P, o, ds, e, b2);
+                gather_cell<UNIT>(g, P, o, ds, e, b2, E12, S6);
                 double v[3] = {S.vx[p], S.vy[p], S.vz[p]};
 #pragma unroll
                 for (int a = 0; a < 3; a++) p0[a] = pos[a];
                 if (REL) {
                     double ga = S.g[p];
-                    vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga);
+                    VayStep vt;
+                    vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga, vt);
                     S.g[p] = ga;
                 } else {
                     boris_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v);
@@ -593,16 +461,8 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, 
                 const bool hit = maybe_crossed(bc, pos);
                 if (st.deposit[s] && dt > 0.0) {
                     coef = st.vbc[s];
-                    // a face crossed on some axis: the cells of the ends (as
-                    // vb_deposit's floors) differ
                     double u0[3], u1[3];
-                    listed = hit;
-#pragma unroll
-                    for (int a = 0; a < 3; a++) {
-                        u0[a] = UNIT ? p0[a] : (p0[a] - g.x0[a]) * g.id[a];
-                        u1[a] = UNIT ? p1[a] : (p1[a] - g.x0[a]) * g.id[a];
-                        listed = listed || f64_sign(u0[a]) || f64_sign(u1[a]) || f64_trunc(u1[a]) + 1 != ci[a];
-                    }
+                    listed = leaves_cell<UNIT>(g, ci, p0, p1, u0, u1) || hit;
                     if (!listed) {
                         active = true;
                         double m[3], Dd[3], n[3];
@@ -685,13 +545,14 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused(Geom g, SpeciesTab st, BCT
             if (!cell_ok(g, ci[0], ci[1], ci[2])) {
                 atomicOr(&ctr->err, (unsigned long long)ERR_BOUNDS);
             } else {
-                double ds[3], e[3], b2[3];
+                double ds[3], e[3], b2[3], E12[12], S6[6];
                 from_vertex<UNIT>(g, ci, pos, ds);
-                gather_cell<UNIT>(g, P, gidx(g, ci[0], ci[1], ci[2]), ds, e, b2);
+                gather_cell<UNIT>(g, P, gidx(g, ci[0], ci[1], ci[2]), ds, e, b2, E12, S6);
                 double v[3] = {S.vx[p], S.vy[p], S.vz[p]};
                 if (REL) {
                     double ga = S.g[p];
-                    vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga);
+                    VayStep vt;
+                    vay_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v, ga, vt);
                     S.g[p] = ga;
                 } else {
                     boris_push<MODE>(st.qp[s], st.hqp[s], e, b2, dt, pos, v);
