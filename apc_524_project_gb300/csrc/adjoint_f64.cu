@@ -67,7 +67,6 @@ using JPtrs = adf::JPtrsT<double>;
 using Slots6 = adf::Slots6T<double>;
 using adf::k_fold_adj;
 using adf::k_ghost_adj;
-using adf::k_plane_adj;
 using adf::k_yee_b_adj;
 using adf::k_yee_e_adj;
 
@@ -926,59 +925,7 @@ static int tlm_step(emoo_handle *h, AdRun &R, double **dP, double *const *dslot,
     return EMOO_OK;
 }
 
-// The plane sets met by the adjoint steps, in reverse order, with the
-// device sums (sum LF, sum LF t1 t2) each one left in `sums`; the wave
-// parameter gradient is formed from them on the host at the end.
-struct PlaneLedger {
-    std::vector<AdBcOp> ops;
-    double *sums = nullptr;
-    size_t cap = 0;
-};
-
-// adjoint of one step, given the state before it (snapshot S)
-// Adjoints of plane sets, last first, each recorded in the ledger.
-static int planes_adj(emoo_handle *h, const std::vector<AdBcOp> &ops, double *const *lslot, PlaneLedger &pl) {
-    for (auto it = ops.rbegin(); it != ops.rend(); ++it) {
-        const AdBcOp &op = *it;
-        if (op.kind != 1) continue;
-        if (pl.ops.size() >= pl.cap) return EMOO_ERR_STATE;
-        double *sums = pl.sums + 2 * adf::PLANE_BLOCKS * pl.ops.size();
-        pl.ops.push_back(op);
-        h->launches++;
-        k_plane_adj<<<adf::PLANE_BLOCKS, 256, 0, h->stream>>>(h->g, lslot[op.slot], op.dim, op.idx, op.t1, op.t2,
-                                                              sums);
-    }
-    EMOO_CUDA(cudaGetLastError());
-    return EMOO_OK;
-}
-
-// Adjoint of the corrected policy's whole-range periodic copies (fold = 0) or
-// folds (fold = 1) of the slots `ids`, with the mirror folds of J at
-// reflecting walls (fold = 1 on the J slots): dimensions and sides reversed.
-static int periodic_full_adj(emoo_handle *h, double *const *lslot, const int *ids, int nids, int fold) {
-    const Geom &g = h->g;
-    adf::Slots9T<double> fl{};
-    for (int k = 0; k < nids; k++) fl.p[k] = lslot[ids[k]];
-    dim3 blk(32, 8);
-    for (int d = 2; d >= 0; d--) {
-        const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
-        if (h->bc.fbc[2 * d] != FBC_PERIODIC) {
-            if (!fold) continue;
-            for (int r = 1; r >= 0; r--) {
-                if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
-                dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
-                h->launches++;
-                adf::k_mirror_fold_adj<double><<<grd, blk, 0, h->stream>>>(g, fl, d, r);
-            }
-            continue;
-        }
-        dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, nids);
-        h->launches++;
-        adf::k_periodic_full_adj<double><<<grd, blk, 0, h->stream>>>(g, fl, d, fold);
-    }
-    EMOO_CUDA(cudaGetLastError());
-    return EMOO_OK;
-}
+using adf::PlaneLedger;
 
 template <bool REL>
 static void launch_adj(emoo_handle *h, bool corr, const SpeciesTab &st, CPArr P, FPtrs F, PArr LP, int64_t np,
@@ -1024,24 +971,25 @@ static int adj_step(emoo_handle *h, AdRun &R, const Snapshot &S, double **L, dou
         static const int ids9[9] = {EMOO_EX, EMOO_EY, EMOO_EZ, EMOO_BX, EMOO_BY, EMOO_BZ,
                                     EMOO_BX_TM1, EMOO_BY_TM1, EMOO_BZ_TM1};
         static const int ids_j[3] = {EMOO_JX, EMOO_JY, EMOO_JZ};
-        EMOO_TRY(planes_adj(h, ops, lslot, pl));
-        EMOO_TRY(periodic_full_adj(h, lslot, ids9, 9, 0));
+        EMOO_TRY(adf::planes_adj<double>(h, ops, 0, ops.size(), lslot, pl));
+        EMOO_TRY(adf::copy_images_adj<double>(h, lslot, ids9, 9));
         h->launches += 2;
         k_yee_b_adj<<<grid_all(g, blk), blk, 0, h->stream>>>(g, yc, A);
         // the B half overwrote the B role's physical points: the values the
         // planes set there between the halves reach nothing
         adf::Slots9T<double> lb{{A.B[0], A.B[1], A.B[2]}};
         adf::k_clear_phys<double><<<dim3((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]), blk, 0, h->stream>>>(g, lb);
-        EMOO_TRY(planes_adj(h, ops, lslot, pl));
-        EMOO_TRY(periodic_full_adj(h, lslot, ids_e, 3, 0));
+        EMOO_TRY(adf::planes_adj<double>(h, ops, 0, ops.size(), lslot, pl));
+        EMOO_TRY(adf::copy_images_adj<double>(h, lslot, ids_e, 3));
         h->launches++;
         k_yee_e_adj<<<grid_all(g, blk), blk, 0, h->stream>>>(g, yc, A, LJ);
-        EMOO_TRY(periodic_full_adj(h, lslot, ids_j, 3, 1));
+        EMOO_TRY(adf::periodic_fold_adj<double>(h, lslot, ids_j, 3));
     } else {
         // 1. executeBC(-1), in reverse
-        for (auto it = ops.rbegin(); it != ops.rend(); ++it) {
-            const AdBcOp &op = *it;
+        for (size_t i = ops.size(); i > 0;) {
+            const AdBcOp &op = ops[i - 1];
             if (op.kind == 0) {
+                i--;
                 Slots6 fl{{lslot[EMOO_EX], lslot[EMOO_EY], lslot[EMOO_EZ], lslot[EMOO_BX], lslot[EMOO_BY],
                            lslot[EMOO_BZ]}};
                 for (int d = 2; d >= 0; d--) {
@@ -1054,8 +1002,10 @@ static int adj_step(emoo_handle *h, AdRun &R, const Snapshot &S, double **L, dou
                     }
                 }
             } else {
-                const std::vector<AdBcOp> one(1, op);
-                EMOO_TRY(planes_adj(h, one, lslot, pl));
+                size_t first = i - 1;  // the stretch of plane sets that ends here
+                while (first > 0 && ops[first - 1].kind == 1) first--;
+                EMOO_TRY(adf::planes_adj<double>(h, ops, first, i, lslot, pl));
+                i = first;
             }
         }
         EMOO_CUDA(cudaGetLastError());

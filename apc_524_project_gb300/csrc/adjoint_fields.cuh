@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "dev_common.cuh"
 #include "emoo_internal.h"
 
@@ -159,13 +161,11 @@ __global__ void k_ghost_adj(Geom g, Slots6T<R> fl, int d, int side) {
 
 // ---- corrected policy ------------------------------------------------------
 //
-// Adjoint of the whole-range periodic operations along d, per transverse
-// point of the (n+3)^2 plane, the forward steps reversed (so any n is exact):
-// fold = 1 reverses f[n] += f[0], f[1] += f[n+1], f[2] += f[n+2];
-// fold = 0 reverses f[0] = f[n], f[n+1] = f[1], f[n+2] = f[2].
-// One field per blockIdx.z.
+// Adjoint of the whole-range periodic fold along d (f[n] += f[0], f[1] +=
+// f[n+1], f[2] += f[n+2]), per transverse point of the (n+3)^2 plane, the
+// forward steps reversed (so any n is exact). One field per blockIdx.z.
 template <class R>
-__global__ void k_periodic_full_adj(Geom g, Slots9T<R> fl, int d, int fold) {
+__global__ void k_periodic_full_adj(Geom g, Slots9T<R> fl, int d) {
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y * blockDim.y + threadIdx.y;
@@ -179,17 +179,32 @@ __global__ void k_periodic_full_adj(Geom g, Slots9T<R> fl, int d, int fold) {
         c[d] = i;
         return F[gidx(g, c[0], c[1], c[2])];
     };
-    if (fold) {
-        at(n + 2) += at(2);
-        at(n + 1) += at(1);
-        at(0) += at(n);
-    } else {
-        at(2) += at(n + 2);
-        at(n + 2) = (R)0;
-        at(1) += at(n + 1);
-        at(n + 1) = (R)0;
-        at(n) += at(0);
-        at(0) = (R)0;
+    at(n + 2) += at(2);
+    at(n + 1) += at(1);
+    at(0) += at(n);
+}
+
+struct WrapDims {
+    int w[3];
+};
+
+// Adjoint of the whole-range ghost copies of nf fields: each point takes in
+// its periodic images' adjoints and clears them.
+template <class R>
+__global__ void k_copy_images_adj(Geom g, Slots9T<R> fl, int nf, WrapDims w) {
+    int c[3];
+    if (!image_point(g.n, w.w, c) || !has_images(g.n, w.w, c)) return;
+    const int64_t st[3] = {g.sx, g.sy, 1}, o = gidx(g, c[0], c[1], c[2]);
+    Images im;
+    images_of(g.n, w.w, st, c, im);
+    for (int q = 0; q < nf; q++) {
+        R *F = fl.p[q] + o;
+        R v = *F;
+        for_images(im, [&](int64_t d) {
+            v += F[d];
+            F[d] = (R)0;
+        });
+        *F = v;
     }
 }
 
@@ -238,9 +253,23 @@ __global__ void k_clear_phys(Geom g, Slots9T<R> fl) {
 // The plane's adjoint is cleared.
 constexpr int PLANE_BLOCKS = 64;
 
+// A launch takes the planes of up to 12 sets (blockIdx.y), none of which
+// share a point; entry e's partials follow entry e - 1's.
 template <class R>
-__global__ void k_plane_adj(Geom g, R *F, int d, int idx, const double *t1, const double *t2, double *sums2) {
+struct PlaneAdjList {
+    R *f[12];
+    int idx[12];
+    const double *t1[12], *t2[12];
+    int dim, n;
+};
+
+template <class R>
+__global__ void k_plane_adj(Geom g, PlaneAdjList<R> pl, double *sums) {
     __shared__ double s_u[32], s_s[32];
+    const int entry = blockIdx.y, d = pl.dim, idx = pl.idx[entry];
+    R *F = pl.f[entry];
+    const double *t1 = pl.t1[entry], *t2 = pl.t2[entry];
+    double *sums2 = sums + 2 * (size_t)PLANE_BLOCKS * entry;
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     double su = 0.0, ss = 0.0;
     const int64_t m = (int64_t)g.tot[o1] * g.tot[o2];
@@ -274,6 +303,91 @@ __global__ void k_plane_adj(Geom g, R *F, int d, int idx, const double *t1, cons
         sums2[2 * blockIdx.x] = a;
         sums2[2 * blockIdx.x + 1] = b;
     }
+}
+
+// The plane sets met by the adjoint steps, in reverse order, with the device
+// sums (sum LF, sum LF t1 t2) each one left in `sums`; the wave parameter
+// gradient is formed from them on the host at the end.
+struct PlaneLedger {
+    std::vector<AdBcOp> ops;
+    double *sums = nullptr;
+    size_t cap = 0;
+};
+
+// Adjoints of the plane sets among ops [first, last), last first, each
+// recorded in the ledger; one launch for those of a dimension, whose planes
+// are disjoint (unless it has one cell: both sides set the same plane).
+template <class R>
+int planes_adj(emoo_handle *h, const std::vector<AdBcOp> &ops, size_t first, size_t last, R *const *lslot,
+               PlaneLedger &pl) {
+    PlaneAdjList<R> list = {};
+    size_t start = pl.ops.size();
+    auto flush = [&]() -> int {
+        if (!list.n) return EMOO_OK;
+        h->launches++;
+        k_plane_adj<R><<<dim3(PLANE_BLOCKS, list.n), 256, 0, h->stream>>>(h->g, list,
+                                                                          pl.sums + 2 * (size_t)PLANE_BLOCKS * start);
+        EMOO_CUDA(cudaGetLastError());
+        list.n = 0;
+        start = pl.ops.size();
+        return EMOO_OK;
+    };
+    for (size_t i = last; i-- > first;) {
+        const AdBcOp &op = ops[i];
+        if (op.kind != 1) continue;
+        if (pl.ops.size() >= pl.cap) return EMOO_ERR_STATE;
+        bool apart = list.n < 12 && (!list.n || op.dim == list.dim);
+        for (int e = 0; e < list.n; e++) apart = apart && !(list.f[e] == lslot[op.slot] && list.idx[e] == op.idx);
+        if (!apart) EMOO_TRY(flush());
+        list.dim = op.dim;
+        list.f[list.n] = lslot[op.slot];
+        list.idx[list.n] = op.idx;
+        list.t1[list.n] = op.t1;
+        list.t2[list.n] = op.t2;
+        list.n++;
+        pl.ops.push_back(op);
+    }
+    return flush();
+}
+
+// Adjoint of the corrected policy's whole-range folds (J with its mirror folds
+// at reflecting walls), dimensions and sides reversed.
+template <class R>
+int periodic_fold_adj(emoo_handle *h, R *const *lslot, const int *ids, int nids) {
+    const Geom &g = h->g;
+    Slots9T<R> fl{};
+    for (int k = 0; k < nids; k++) fl.p[k] = lslot[ids[k]];
+    dim3 blk(32, 8);
+    for (int d = 2; d >= 0; d--) {
+        const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
+        if (h->bc.fbc[2 * d] != FBC_PERIODIC) {
+            for (int r = 1; r >= 0; r--) {
+                if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
+                dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
+                h->launches++;
+                k_mirror_fold_adj<R><<<grd, blk, 0, h->stream>>>(g, fl, d, r);
+            }
+            continue;
+        }
+        dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, nids);
+        h->launches++;
+        k_periodic_full_adj<R><<<grd, blk, 0, h->stream>>>(g, fl, d);
+    }
+    EMOO_CUDA(cudaGetLastError());
+    return EMOO_OK;
+}
+
+// Adjoint of the corrected policy's ghost copies.
+template <class R>
+int copy_images_adj(emoo_handle *h, R *const *lslot, const int *ids, int nids) {
+    Slots9T<R> fl{};
+    WrapDims w;
+    for (int k = 0; k < nids; k++) fl.p[k] = lslot[ids[k]];
+    for (int d = 0; d < 3; d++) w.w[d] = h->bc.fbc[2 * d] == FBC_PERIODIC;
+    h->launches++;
+    k_copy_images_adj<R><<<image_grid(h->g, w.w), dim3(32, 8), 0, h->stream>>>(h->g, fl, nids, w);
+    EMOO_CUDA(cudaGetLastError());
+    return EMOO_OK;
 }
 
 }  // namespace adf

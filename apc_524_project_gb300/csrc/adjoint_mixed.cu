@@ -261,62 +261,14 @@ int objective_m(emoo_handle *h, const ObjM &os, double *dev, double *out) {
     return EMOO_OK;
 }
 
-struct LedgerM {
-    std::vector<AdBcOp> ops;
-    double *sums = nullptr;
-    size_t cap = 0;
-};
-
-// Adjoints of plane sets, last first, each recorded in the ledger.
-int planes_adj_m(emoo_handle *h, const std::vector<AdBcOp> &ops, float *const *lslot, LedgerM &pl) {
-    for (auto it = ops.rbegin(); it != ops.rend(); ++it) {
-        const AdBcOp &op = *it;
-        if (op.kind != 1) continue;
-        if (pl.ops.size() >= pl.cap) return EMOO_ERR_STATE;
-        double *sums = pl.sums + 2 * adf::PLANE_BLOCKS * pl.ops.size();
-        pl.ops.push_back(op);
-        h->launches++;
-        adf::k_plane_adj<float><<<adf::PLANE_BLOCKS, 256, 0, h->stream>>>(h->g, lslot[op.slot], op.dim, op.idx, op.t1,
-                                                                          op.t2, sums);
-    }
-    EMOO_CUDA(cudaGetLastError());
-    return EMOO_OK;
-}
-
-// Adjoint of the corrected policy's whole-range periodic copies (fold = 0) or
-// folds (fold = 1) of the float adjoint slots `ids`, with the mirror folds of
-// J at reflecting walls (fold = 1): dimensions and sides reversed.
-int periodic_full_adj_m(emoo_handle *h, float *const *lslot, const int *ids, int nids, int fold) {
-    const Geom &g = h->g;
-    adf::Slots9T<float> fl{};
-    for (int k = 0; k < nids; k++) fl.p[k] = lslot[ids[k]];
-    dim3 blk(32, 8);
-    for (int d = 2; d >= 0; d--) {
-        const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
-        if (h->bc.fbc[2 * d] != FBC_PERIODIC) {
-            if (!fold) continue;
-            for (int r = 1; r >= 0; r--) {
-                if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
-                dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
-                h->launches++;
-                adf::k_mirror_fold_adj<float><<<grd, blk, 0, h->stream>>>(g, fl, d, r);
-            }
-            continue;
-        }
-        dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, nids);
-        h->launches++;
-        adf::k_periodic_full_adj<float><<<grd, blk, 0, h->stream>>>(g, fl, d, fold);
-    }
-    EMOO_CUDA(cudaGetLastError());
-    return EMOO_OK;
-}
+using adf::PlaneLedger;
 
 // The field part of one corrected step in reverse (forward: J fold, E half,
 // E images, planes, B half, E/B/B_tm1 images, planes), the FP64 form's
 // sequence on the float adjoint slots; leaves the current adjoint in the J
 // slots for the particle kernel.
 int adj_fields_corrected_m(emoo_handle *h, const MSnap &S, const std::vector<AdBcOp> &ops, float *const *lslot,
-                           LedgerM &pl) {
+                           PlaneLedger &pl) {
     static const int ids_e[3] = {EMOO_EX, EMOO_EY, EMOO_EZ};
     static const int ids9[9] = {EMOO_EX, EMOO_EY, EMOO_EZ, EMOO_BX, EMOO_BY, EMOO_BZ,
                                 EMOO_BX_TM1, EMOO_BY_TM1, EMOO_BZ_TM1};
@@ -326,18 +278,18 @@ int adj_fields_corrected_m(emoo_handle *h, const MSnap &S, const std::vector<AdB
     JPtrsF LJ{{lslot[EMOO_JX], lslot[EMOO_JY], lslot[EMOO_JZ]}};
     dim3 blk(32, 8);
     const adf::YeeCoef<float> yc = adf::yee_coef<float>(g, h->dtp);
-    EMOO_TRY(planes_adj_m(h, ops, lslot, pl));
-    EMOO_TRY(periodic_full_adj_m(h, lslot, ids9, 9, 0));
+    EMOO_TRY(adf::planes_adj<float>(h, ops, 0, ops.size(), lslot, pl));
+    EMOO_TRY(adf::copy_images_adj<float>(h, lslot, ids9, 9));
     h->launches += 2;
     adf::k_yee_b_adj<float><<<grid_all_m(g, blk), blk, 0, h->stream>>>(g, yc, A);
     // the B half overwrote the B role's physical points
     adf::Slots9T<float> lb{{A.B[0], A.B[1], A.B[2]}};
     adf::k_clear_phys<float><<<dim3((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]), blk, 0, h->stream>>>(g, lb);
-    EMOO_TRY(planes_adj_m(h, ops, lslot, pl));
-    EMOO_TRY(periodic_full_adj_m(h, lslot, ids_e, 3, 0));
+    EMOO_TRY(adf::planes_adj<float>(h, ops, 0, ops.size(), lslot, pl));
+    EMOO_TRY(adf::copy_images_adj<float>(h, lslot, ids_e, 3));
     h->launches++;
     adf::k_yee_e_adj<float><<<grid_all_m(g, blk), blk, 0, h->stream>>>(g, yc, A, LJ);
-    EMOO_TRY(periodic_full_adj_m(h, lslot, ids_j, 3, 1));
+    EMOO_TRY(adf::periodic_fold_adj<float>(h, lslot, ids_j, 3));
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -345,7 +297,7 @@ int adj_fields_corrected_m(emoo_handle *h, const MSnap &S, const std::vector<AdB
 // adjoint of one step, given the state before it (S) and the cell array of
 // the state after it
 int adj_step_m(emoo_handle *h, AdRunM &R, const MSnap &S, const int32_t *cell_after, float *const lo[3],
-               float *const lu[3], float *const *lslot, LedgerM &pl, unsigned long long *mismatch) {
+               float *const lu[3], float *const *lslot, PlaneLedger &pl, unsigned long long *mismatch) {
     const Geom &g = h->g;
     const int b1 = S.bswap ^ 1;  // B roles after the step's Yee update
     std::vector<AdBcOp> ops;
@@ -367,9 +319,10 @@ int adj_step_m(emoo_handle *h, AdRunM &R, const MSnap &S, const int32_t *cell_af
               *lT[3] = {LF.T[0], LF.T[1], LF.T[2]};
         return mixed_ad_particles(h, R.view(S), cell_after, lo, lu, lj, lE, lB, lT, mismatch);
     }
-    for (auto it = ops.rbegin(); it != ops.rend(); ++it) {
-        const AdBcOp &op = *it;
+    for (size_t i = ops.size(); i > 0;) {
+        const AdBcOp &op = ops[i - 1];
         if (op.kind == 0) {
+            i--;
             Slots6F fl{{lslot[EMOO_EX], lslot[EMOO_EY], lslot[EMOO_EZ], lslot[EMOO_BX], lslot[EMOO_BY], lslot[EMOO_BZ]}};
             for (int d = 2; d >= 0; d--) {
                 if (!((op.mask >> d) & 1)) continue;
@@ -382,12 +335,10 @@ int adj_step_m(emoo_handle *h, AdRunM &R, const MSnap &S, const int32_t *cell_af
                 }
             }
         } else {
-            if (pl.ops.size() >= pl.cap) return EMOO_ERR_STATE;
-            double *sums = pl.sums + 2 * adf::PLANE_BLOCKS * pl.ops.size();
-            pl.ops.push_back(op);
-            h->launches++;
-            adf::k_plane_adj<float><<<adf::PLANE_BLOCKS, 256, 0, h->stream>>>(g, lslot[op.slot], op.dim, op.idx, op.t1,
-                                                                              op.t2, sums);
+            size_t first = i - 1;  // the stretch of plane sets that ends here
+            while (first > 0 && ops[first - 1].kind == 1) first--;
+            EMOO_TRY(adf::planes_adj<float>(h, ops, first, i, lslot, pl));
+            i = first;
         }
     }
     EMOO_CUDA(cudaGetLastError());
@@ -530,7 +481,7 @@ int ad_run_mixed(emoo_handle *h, const emoo_ad_spec *spec, int mode, emoo_ad_res
         float *lu[3] = {lam[3], lam[4], lam[5]};
         EMOO_TRY(mixed_ad_kinetic(h, handle_view(h), os.species, os.xlo, os.xhi, nullptr, lu));
     }
-    LedgerM pl;
+    PlaneLedger pl;
     {
         std::vector<AdBcOp> ops;
         EMOO_TRY(ad_bc_ops(h, ops));

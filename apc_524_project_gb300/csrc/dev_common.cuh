@@ -65,6 +65,71 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
+// The corrected policy's periodic images. Along a periodic dimension of n
+// cells (wrap 1) index c of 1..n has images 0 (of n), n + 1 (of 1) and n + 2
+// (of 2; of 1 when n is 1); a walled one (wrap 0) has none and keeps its whole
+// range. A point's images are the products over the dimensions, itself among
+// them; every ghost point along periodic dimensions is the image of exactly
+// one such point.
+struct Images {
+    int64_t off[3][4];  // offsets along each dimension, 0 first
+    int n[3];
+};
+
+// The point of thread (bx, by, bz) of a launch over `t` = n (periodic) or n + 3
+// (walled) points a dimension; false past the range.
+__device__ __forceinline__ bool image_point(const int n[3], const int wrap[3], int c[3]) {
+    c[0] = (int)blockIdx.z;
+    c[1] = (int)(blockIdx.y * blockDim.y + threadIdx.y);
+    c[2] = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    bool in = true;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        c[d] += wrap[d];
+        in = in && c[d] < (wrap[d] ? n[d] + 1 : n[d] + 3);
+    }
+    return in;
+}
+
+// Whether the point has images besides itself.
+__device__ __forceinline__ bool has_images(const int n[3], const int wrap[3], const int c[3]) {
+    bool edge = false;
+#pragma unroll
+    for (int d = 0; d < 3; d++) edge = edge || (wrap[d] && (c[d] <= 2 || c[d] == n[d]));
+    return edge;
+}
+
+__device__ __forceinline__ void images_of(const int n[3], const int wrap[3], const int64_t st[3], const int c[3],
+                                          Images &im) {
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        int m = 0;
+        im.off[d][m++] = 0;
+        if (wrap[d]) {
+            if (c[d] == n[d]) im.off[d][m++] = -n[d] * st[d];
+            if (c[d] == 1) im.off[d][m++] = n[d] * st[d];
+            if (c[d] == 2 || n[d] == 1) im.off[d][m++] = (n[d] + 2 - c[d]) * st[d];
+        }
+        im.n[d] = m;
+    }
+}
+
+// f(offset) for every image but the point itself
+template <class F>
+__device__ __forceinline__ void for_images(const Images &im, F f) {
+    for (int x = 0; x < im.n[0]; x++)
+        for (int y = 0; y < im.n[1]; y++)
+            for (int z = 0; z < im.n[2]; z++)
+                if (x + y + z) f(im.off[0][x] + im.off[1][y] + im.off[2][z]);
+}
+
+// Launch shape of image_point (blocks of 32 x 8).
+inline dim3 image_grid(const Geom &g, const int wrap[3]) {
+    int t[3];
+    for (int d = 0; d < 3; d++) t[d] = wrap[d] ? g.n[d] : g.tot[d];
+    return dim3((t[2] + 31) / 32, (t[1] + 7) / 8, t[0]);
+}
+
 __device__ __forceinline__ void atomic_max_nonneg(double *addr, double v) {
     // non-negative doubles order like their bit patterns
     atomicMax((unsigned long long *)addr, (unsigned long long)__double_as_longlong(v));

@@ -762,11 +762,10 @@ struct Slots9 {
     double *p[9];
 };
 
-// Along dim d, for every transverse point of the whole (n+3)^2 plane:
-// fold = 1: f[n] += f[0], f[1] += f[n+1], f[2] += f[n+2] (the ghost planes'
-// deposits to their periodic images); fold = 0: f[0] = f[n], f[n+1] = f[1],
-// f[n+2] = f[2] (the ghost planes refreshed). One field per blockIdx.z.
-__global__ void k_periodic_full(Geom g, Slots9 fl, int d, int fold) {
+// Fold along dim d, for every transverse point of the whole (n+3)^2 plane:
+// f[n] += f[0], f[1] += f[n+1], f[2] += f[n+2] (the ghost planes' deposits to
+// their periodic images). One field per blockIdx.z.
+__global__ void k_periodic_full(Geom g, Slots9 fl, int d) {
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y * blockDim.y + threadIdx.y;
@@ -780,14 +779,27 @@ __global__ void k_periodic_full(Geom g, Slots9 fl, int d, int fold) {
         c[d] = i;
         return F[gidx(g, c[0], c[1], c[2])];
     };
-    if (fold) {
-        at(n) += at(0);
-        at(1) += at(n + 1);
-        at(2) += at(n + 2);
-    } else {
-        at(0) = at(n);
-        at(n + 1) = at(1);
-        at(n + 2) = at(2);
+    at(n) += at(0);
+    at(1) += at(n + 1);
+    at(2) += at(n + 2);
+}
+
+struct Wrap {
+    int w[3];
+};
+
+// Ghost copies of nf fields over the whole range in one launch: each point
+// writes its value to its periodic images (no thread reads a ghost value).
+__global__ void k_copy_images(Geom g, Slots9 fl, int nf, Wrap w) {
+    int c[3];
+    if (!image_point(g.n, w.w, c) || !has_images(g.n, w.w, c)) return;
+    const int64_t st[3] = {g.sx, g.sy, 1}, o = gidx(g, c[0], c[1], c[2]);
+    Images im;
+    images_of(g.n, w.w, st, c, im);
+    for (int q = 0; q < nf; q++) {
+        double *F = fl.p[q] + o;
+        const double v = *F;
+        for_images(im, [&](int64_t d) { F[d] = v; });
     }
 }
 
@@ -822,14 +834,12 @@ __global__ void k_mirror_fold(Geom g, Slots9 fl, int d, int right) {
     F[ks] = 0.0;
 }
 
-// The corrected policy's folds (fold = 1, the arrays J and / or rho) or ghost
-// copies (fold = 0), dimension by dimension so edge and corner lines follow:
-// periodic dimensions as images over the whole range; walled dimensions
-// (corrected policy with reflecting or absorbing particle sides) fold J by
-// mirror at reflecting sides only (at absorbing ones the current of the path
-// beyond the wall stays in the ghost layer) and copy nothing (their field
-// sides are LightBC planes).
-static int periodic_full(emoo_handle *h, const int *ids, int nids, int fold) {
+// The corrected policy's folds (J and / or rho), dimension by dimension so edge
+// and corner lines follow: periodic dimensions as images over the whole range;
+// walled dimensions (corrected policy with reflecting or absorbing particle
+// sides) fold J by mirror at reflecting sides only (at absorbing ones the
+// current of the path beyond the wall stays in the ghost layer).
+static int periodic_fold(emoo_handle *h, const int *ids, int nids) {
     const Geom &g = h->g;
     Slots9 fl;
     for (int k = 0; k < nids; k++) fl.p[k] = h->slot[ids[k]];
@@ -837,7 +847,7 @@ static int periodic_full(emoo_handle *h, const int *ids, int nids, int fold) {
     for (int d = 0; d < 3; d++) {
         const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
         if (h->bc.fbc[2 * d] != FBC_PERIODIC) {
-            const bool j3 = fold && nids >= 3 && ids[0] == EMOO_JX && ids[1] == EMOO_JY && ids[2] == EMOO_JZ;
+            const bool j3 = nids >= 3 && ids[0] == EMOO_JX && ids[1] == EMOO_JY && ids[2] == EMOO_JZ;
             for (int r = 0; r < 2 && j3; r++) {
                 if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
                 dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
@@ -848,7 +858,7 @@ static int periodic_full(emoo_handle *h, const int *ids, int nids, int fold) {
         }
         dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, nids);
         h->launches++;
-        k_periodic_full<<<grd, blk, 0, h->stream>>>(g, fl, d, fold);
+        k_periodic_full<<<grd, blk, 0, h->stream>>>(g, fl, d);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -860,34 +870,50 @@ int fold_full_f64(emoo_handle *h, int what) {
     if (what & FOLD_J)
         for (int c = 0; c < 3; c++) ids[n++] = EMOO_JX + c;
     if (what & FOLD_RHO) ids[n++] = EMOO_RHO;
-    return periodic_full(h, ids, n, 1);
+    return periodic_fold(h, ids, n);
 }
 
-// LightBC planes of every external side (E and B roles through the slots).
+// LightBC planes of every external side (E and B roles through the slots), one
+// launch a dimension (its sides are both external).
 static int light_all_f64(emoo_handle *h) {
+    PlaneSet ps[12];
+    int n = 0;
     for (int s = 0; s < 6; s++) {
         if (h->bc.fbc[s] != FBC_EXTERNAL) continue;
-        PlaneSet ps[6];
-        const int n = light_planes_slots(h, s, ps);
-        EMOO_TRY(plane_set_f64(h, ps, n));
+        n += light_planes_slots(h, s, ps + n);
+        if (n > 6 || h->g.n[s / 2] < 2) {  // of one cell, both sides set the same plane: in order
+            EMOO_TRY(plane_set_f64(h, ps, n));
+            n = 0;
+        }
     }
-    return EMOO_OK;
+    return n ? plane_set_f64(h, ps, n) : EMOO_OK;
 }
 
 // E's boundary values between the Yee halves (corrected policy): periodic
 // images and LightBC planes, so the B half reads E at the new time everywhere.
 int ghost_e_full_f64(emoo_handle *h) {
     static const int ids[3] = {EMOO_EX, EMOO_EY, EMOO_EZ};
-    EMOO_TRY(periodic_full(h, ids, 3, 0));
+    EMOO_TRY(periodic_copies_f64(h, ids, 3));
     return light_all_f64(h);
 }
 
-int periodic_copies_f64(emoo_handle *h, const int *ids, int nids) { return periodic_full(h, ids, nids, 0); }
+// The corrected policy's ghost copies; walled dimensions copy nothing (their
+// field sides are LightBC planes).
+int periodic_copies_f64(emoo_handle *h, const int *ids, int nids) {
+    Slots9 fl;
+    Wrap w;
+    for (int k = 0; k < nids; k++) fl.p[k] = h->slot[ids[k]];
+    for (int d = 0; d < 3; d++) w.w[d] = h->bc.fbc[2 * d] == FBC_PERIODIC;
+    h->launches++;
+    k_copy_images<<<image_grid(h->g, w.w), dim3(32, 8), 0, h->stream>>>(h->g, fl, nids, w);
+    EMOO_CUDA(cudaGetLastError());
+    return EMOO_OK;
+}
 
 int ghost_full_f64(emoo_handle *h) {
     static const int ids[9] = {EMOO_EX, EMOO_EY, EMOO_EZ, EMOO_BX, EMOO_BY, EMOO_BZ, EMOO_BX_TM1, EMOO_BY_TM1,
                                EMOO_BZ_TM1};
-    EMOO_TRY(periodic_full(h, ids, 9, 0));
+    EMOO_TRY(periodic_copies_f64(h, ids, 9));
     return light_all_f64(h);
 }
 

@@ -1583,19 +1583,14 @@ __global__ void k_fold_full_m(MGeom g, MFix4 fl, int d, int t1, int t2) {
 // ghost planes (0 <- n, n + 1 <- 1, n + 2 <- 2 along every periodic dimension,
 // over the whole range of walled ones), which no thread reads here. The values
 // are those of the copies dimension by dimension (six launches a step).
-__global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, MF9 fl, int nf, MF3 B, MCF3 T, MCF3 E, float dt, int update,
-                                                   int t0, int t1, int t2) {
-    int c[3] = {(int)blockIdx.z, (int)(blockIdx.y * 8 + threadIdx.y), (int)(blockIdx.x * 32 + threadIdx.x)};
-    const int t[3] = {t0, t1, t2};
+__global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, MF9 fl, int nf, MF3 B, MCF3 T, MCF3 E, float dt,
+                                                   int update) {
+    int c[3];
+    if (!image_point(g.n, g.wrap, c)) return;
     const int64_t st[3] = {g.sx, g.sy, 1};
-    bool phys = true, edge = false;
+    bool phys = true;
 #pragma unroll
-    for (int d = 0; d < 3; d++) {
-        c[d] += g.wrap[d];  // periodic: the physical points only
-        if (c[d] >= (g.wrap[d] ? g.n[d] + 1 : t[d])) return;
-        phys = phys && c[d] >= 1 && c[d] <= g.n[d];
-        edge = edge || (g.wrap[d] && (c[d] <= 2 || c[d] >= g.n[d]));
-    }
+    for (int d = 0; d < 3; d++) phys = phys && c[d] >= 1 && c[d] <= g.n[d];
     const int64_t o = c[0] * st[0] + c[1] * st[1] + c[2];
     if (update && phys) {
         const float *Ex = E.p[0], *Ey = E.p[1], *Ez = E.p[2];
@@ -1606,29 +1601,13 @@ __global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, MF9 fl, int nf, MF3 
         B.p[1][o] = T.p[1][o] + dt * ((Ez[up[0]] - Ez[o]) * g.idf[0] - (Ex[up[2]] - Ex[o]) * g.idf[2]);
         B.p[2][o] = T.p[2][o] + dt * ((Ex[up[1]] - Ex[o]) * g.idf[1] - (Ey[up[0]] - Ey[o]) * g.idf[0]);
     }
-    if (!edge) return;
-    // image offsets along each dimension, the point itself first
-    int64_t im[3][4];
-    int ni[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        const int n = g.n[d];
-        int m = 0;
-        im[d][m++] = 0;
-        if (g.wrap[d]) {
-            if (c[d] == n) im[d][m++] = -n * st[d];
-            if (c[d] == 1) im[d][m++] = n * st[d];
-            if (c[d] == 2 || n == 1) im[d][m++] = (n + 2 - c[d]) * st[d];
-        }
-        ni[d] = m;
-    }
+    if (!has_images(g.n, g.wrap, c)) return;
+    Images im;
+    images_of(g.n, g.wrap, st, c, im);
     for (int q = 0; q < nf; q++) {
         float *F = fl.p[q] + o;
         const float v = *F;
-        for (int x = 0; x < ni[0]; x++)
-            for (int y = 0; y < ni[1]; y++)
-                for (int z = 0; z < ni[2]; z++)
-                    if (x + y + z) F[im[0][x] + im[1][y] + im[2][z]] = v;
+        for_images(im, [&](int64_t d) { F[d] = v; });
     }
 }
 
@@ -2517,19 +2496,15 @@ static int mixed_light_planes(emoo_handle *h) {
 // storage (3: E alone; 9: all), after the B half when `update`.
 static int mixed_b_ghost(emoo_handle *h, double dtp, int nf, bool update) {
     const MGeom mg = mgeom(h, dtp);
-    const Geom &g = h->g;
     MF9 fl = {};
     for (int c = 0; c < 3; c++) fl.p[c] = h->mf->E[c];
     for (int c = 0; c < 6; c++) fl.p[3 + c] = h->mf->Bslot[c];
     MF3 B = {{mb_role(h, 0), mb_role(h, 1), mb_role(h, 2)}};
     MCF3 T = {{mt_role(h, 0), mt_role(h, 1), mt_role(h, 2)}};
     MCF3 E = {{h->mf->E[0], h->mf->E[1], h->mf->E[2]}};
-    int t[3];
-    for (int d = 0; d < 3; d++) t[d] = mg.wrap[d] ? g.n[d] : g.tot[d];
-    dim3 blk(32, 8), grd((t[2] + 31) / 32, (t[1] + 7) / 8, t[0]);
     h->launches++;
-    k_b_ghost_m<<<grd, blk, 0, h->stream>>>(mg, fl, nf, B, T, E, (float)dtp, update ? 1 : 0, g.tot[0], g.tot[1],
-                                            g.tot[2]);
+    k_b_ghost_m<<<image_grid(h->g, mg.wrap), dim3(32, 8), 0, h->stream>>>(mg, fl, nf, B, T, E, (float)dtp,
+                                                                          update ? 1 : 0);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
