@@ -188,24 +188,65 @@ struct WrapDims {
     int w[3];
 };
 
-// Adjoint of the whole-range ghost copies of nf fields: each point takes in
-// its periodic images' adjoints and clears them.
+// Adjoint of the whole-range ghost copies of the fields: each point with images
+// takes in their adjoints and clears them; blockIdx.y = field. 32^3 cells, nine
+// fields: 3.5 us (26 us with a thread a point of the grid for all fields).
 template <class R>
-__global__ void k_copy_images_adj(Geom g, Slots9T<R> fl, int nf, WrapDims w) {
-    int c[3];
-    if (!image_point(g.n, w.w, c) || !has_images(g.n, w.w, c)) return;
-    const int64_t st[3] = {g.sx, g.sy, 1}, o = gidx(g, c[0], c[1], c[2]);
-    Images im;
-    images_of(g.n, w.w, st, c, im);
-    for (int q = 0; q < nf; q++) {
-        R *F = fl.p[q] + o;
-        R v = *F;
-        for_images(im, [&](int64_t d) {
-            v += F[d];
-            F[d] = (R)0;
-        });
-        *F = v;
+__global__ void k_copy_images_adj(Geom g, Slots9T<R> fl, WrapDims w, Slabs S) {
+    int d, c[3];
+    if (!slab_point(S, blockIdx.x * blockDim.x + threadIdx.x, d, c)) return;
+    unsigned m[3];  // images along each dimension: bit 0 the point itself, 1, 2, 3 index 0, n + 1, n + 2
+    bool one = true;
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        const int n = g.n[e];
+        m[e] = 1u;
+        if (!w.w[e]) continue;
+        // listed: 1, 2, n; the rest of a periodic dimension: 3 .. n - 1
+        if (e < d) c[e] += 3;
+        else if (e == d) c[e] = c[e] < 2 ? c[e] + 1 : n;
+        else c[e] += 1;
+        m[e] |= (c[e] == n ? 2u : 0u) | (c[e] == 1 ? 4u : 0u) | (c[e] == 2 || n == 1 ? 8u : 0u);
+        one = one && n >= 3;
     }
+    auto index = [&](int e, int b) { return b == 0 ? c[e] : b == 1 ? 0 : g.n[e] + b - 1; };
+    R *F = fl.p[blockIdx.y];
+    R v = (R)0;
+    if (one) {  // at most one image along each dimension: all loads at once
+        int at[3][2];
+        bool has[3][2];
+#pragma unroll
+        for (int e = 0; e < 3; e++) {
+            at[e][0] = c[e];
+            at[e][1] = m[e] > 1u ? index(e, 31 - __clz(m[e])) : c[e];
+            has[e][0] = true;
+            has[e][1] = m[e] > 1u;
+        }
+        R x[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            const int i = q >> 2, j = (q >> 1) & 1, k = q & 1;
+            if (has[0][i] && has[1][j] && has[2][k]) x[q] = F[gidx(g, at[0][i], at[1][j], at[2][k])];
+        }
+        v = x[0];
+#pragma unroll
+        for (int q = 1; q < 8; q++) {
+            const int i = q >> 2, j = (q >> 1) & 1, k = q & 1;
+            if (has[0][i] && has[1][j] && has[2][k]) {
+                v += x[q];
+                F[gidx(g, at[0][i], at[1][j], at[2][k])] = (R)0;
+            }
+        }
+    } else {
+        for (unsigned x = m[0]; x; x &= x - 1)
+            for (unsigned y = m[1]; y; y &= y - 1)
+                for (unsigned z = m[2]; z; z &= z - 1) {
+                    R *p = F + gidx(g, index(0, __ffs(x) - 1), index(1, __ffs(y) - 1), index(2, __ffs(z) - 1));
+                    v += *p;
+                    *p = (R)0;
+                }
+    }
+    F[gidx(g, c[0], c[1], c[2])] = v;
 }
 
 // Adjoint of the mirror fold at a reflecting wall (dst += s src, src = 0, s =
@@ -384,8 +425,15 @@ int copy_images_adj(emoo_handle *h, R *const *lslot, const int *ids, int nids) {
     WrapDims w;
     for (int k = 0; k < nids; k++) fl.p[k] = lslot[ids[k]];
     for (int d = 0; d < 3; d++) w.w[d] = h->bc.fbc[2 * d] == FBC_PERIODIC;
+    Slabs S;  // the points with images
+    for (int d = 0; d < 3; d++) {
+        S.listed[d] = w.w[d] ? std::min(3, h->g.n[d]) : 0;
+        S.rest[d] = (w.w[d] ? h->g.n[d] : h->g.tot[d]) - S.listed[d];
+    }
+    const int64_t points = slab_size(S);
+    if (!points) return EMOO_OK;
     h->launches++;
-    k_copy_images_adj<R><<<image_grid(h->g, w.w), dim3(32, 8), 0, h->stream>>>(h->g, fl, nids, w);
+    k_copy_images_adj<R><<<dim3((unsigned)((points + 127) / 128), nids), 128, 0, h->stream>>>(h->g, fl, w, S);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }

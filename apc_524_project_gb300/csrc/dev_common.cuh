@@ -71,63 +71,71 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // range. A point's images are the products over the dimensions, itself among
 // them; every ghost point along periodic dimensions is the image of exactly
 // one such point.
-struct Images {
-    int64_t off[3][4];  // offsets along each dimension, 0 first
-    int n[3];
+//
+// The few points with images, and the ghost points, have threads of their own,
+// numbered densely over the slabs they form: in a launch over the whole grid
+// every warp holds some (rows are two to six warps long), and pays for them.
+
+// A set of points: dimension by dimension, those whose index is one of
+// `listed[d]` there and none of the listed ones in the dimensions before.
+struct Slabs {
+    int listed[3], rest[3];  // counts per dimension
 };
 
-// The point of thread (bx, by, bz) of a launch over `t` = n (periodic) or n + 3
-// (walled) points a dimension; false past the range.
-__device__ __forceinline__ bool image_point(const int n[3], const int wrap[3], int c[3]) {
-    c[0] = (int)blockIdx.z;
-    c[1] = (int)(blockIdx.y * blockDim.y + threadIdx.y);
-    c[2] = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    bool in = true;
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        c[d] += wrap[d];
-        in = in && c[d] < (wrap[d] ? n[d] + 1 : n[d] + 3);
-    }
-    return in;
-}
-
-// Whether the point has images besides itself.
-__device__ __forceinline__ bool has_images(const int n[3], const int wrap[3], const int c[3]) {
-    bool edge = false;
-#pragma unroll
-    for (int d = 0; d < 3; d++) edge = edge || (wrap[d] && (c[d] <= 2 || c[d] == n[d]));
-    return edge;
-}
-
-__device__ __forceinline__ void images_of(const int n[3], const int wrap[3], const int64_t st[3], const int c[3],
-                                          Images &im) {
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-        int m = 0;
-        im.off[d][m++] = 0;
-        if (wrap[d]) {
-            if (c[d] == n[d]) im.off[d][m++] = -n[d] * st[d];
-            if (c[d] == 1) im.off[d][m++] = n[d] * st[d];
-            if (c[d] == 2 || n[d] == 1) im.off[d][m++] = (n[d] + 2 - c[d]) * st[d];
+// Point `id` of the slabs as (dimension it is listed in, place in each: of the
+// listed in that dimension, of the rest before it, of all after it).
+__device__ __forceinline__ bool slab_point(const Slabs &S, uint32_t id, int &d, int at[3]) {
+    const uint32_t t1 = S.listed[1] + S.rest[1], t2 = S.listed[2] + S.rest[2];
+    uint32_t size = S.listed[0] * t1 * t2;
+    uint32_t n1 = t1, n2 = t2;
+    d = 0;
+    if (id >= size) {
+        id -= size;
+        d = 1;
+        n1 = S.listed[1];
+        size = S.rest[0] * n1 * t2;
+        if (id >= size) {
+            id -= size;
+            d = 2;
+            n1 = S.rest[1];
+            n2 = S.listed[2];
+            if (id >= S.rest[0] * n1 * n2) return false;
         }
-        im.n[d] = m;
     }
+    const uint32_t q = id / n2;
+    at[2] = (int)(id - q * n2);
+    at[0] = (int)(q / n1);
+    at[1] = (int)(q - at[0] * n1);
+    return true;
 }
 
-// f(offset) for every image but the point itself
-template <class F>
-__device__ __forceinline__ void for_images(const Images &im, F f) {
-    for (int x = 0; x < im.n[0]; x++)
-        for (int y = 0; y < im.n[1]; y++)
-            for (int z = 0; z < im.n[2]; z++)
-                if (x + y + z) f(im.off[0][x] + im.off[1][y] + im.off[2][z]);
+inline int64_t slab_size(const Slabs &S) {
+    const int64_t t1 = S.listed[1] + S.rest[1], t2 = S.listed[2] + S.rest[2];
+    return S.listed[0] * t1 * t2 + (int64_t)S.rest[0] * (S.listed[1] * t2 + (int64_t)S.rest[1] * S.listed[2]);
 }
 
-// Launch shape of image_point (blocks of 32 x 8).
-inline dim3 image_grid(const Geom &g, const int wrap[3]) {
-    int t[3];
-    for (int d = 0; d < 3; d++) t[d] = wrap[d] ? g.n[d] : g.tot[d];
-    return dim3((t[2] + 31) / 32, (t[1] + 7) / 8, t[0]);
+// The ghost points along the periodic dimensions.
+inline Slabs ghost_slabs(const int n[3], const int wrap[3]) {
+    Slabs S;
+    for (int d = 0; d < 3; d++) {
+        S.listed[d] = wrap[d] ? 3 : 0;
+        S.rest[d] = wrap[d] ? n[d] : n[d] + 3;
+    }
+    return S;
+}
+
+// Ghost point `id`: its indices c and those of the point it is an image of.
+__device__ __forceinline__ bool ghost_point(const Slabs &S, const int n[3], const int wrap[3], uint32_t id, int c[3],
+                                            int of[3]) {
+    int d;
+    if (!slab_point(S, id, d, c)) return false;
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+        if (e == d) c[e] = c[e] ? n[e] + c[e] : 0;
+        else if (e < d) c[e] += wrap[e];
+        of[e] = !wrap[e] || (c[e] >= 1 && c[e] <= n[e]) ? c[e] : c[e] == 0 ? n[e] : c[e] == n[e] + 1 || n[e] == 1 ? 1 : 2;
+    }
+    return true;
 }
 
 __device__ __forceinline__ void atomic_max_nonneg(double *addr, double v) {
