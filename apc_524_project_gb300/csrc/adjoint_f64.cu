@@ -367,6 +367,7 @@ constexpr int ADJ_BLOCK = 128;
 template <bool REL, bool CORR, bool UNIT>
 __global__ void __launch_bounds__(ADJ_BLOCK) k_adj_particles(Geom g, SpeciesTab st, BCTab bc, CPArr P, FPtrs F, PArr L,
                                                              int64_t np, double dt, JPtrs LJ, FOut LF) {
+    after_previous<false>();
     __shared__ double s_move[CORR ? 7 : 1][CORR ? ADJ_BLOCK : 1];  // in: ends and coef; out: their derivatives
     __shared__ int s_n;
     if (CORR) {
@@ -933,7 +934,7 @@ static void launch_adj(emoo_handle *h, bool corr, const SpeciesTab &st, CPArr P,
     const int nb = (int)((np + ADJ_BLOCK - 1) / ADJ_BLOCK);
     if (np == 0) return;
 #define EMOO_ADJ(C, U) \
-    k_adj_particles<REL, C, U><<<nb, ADJ_BLOCK, 0, h->stream>>>(h->g, st, h->bc, P, F, LP, np, h->dtp, LJ, LF)
+    launch_after(k_adj_particles<REL, C, U>, nb, ADJ_BLOCK, 0, h->stream)(h->g, st, h->bc, P, F, LP, np, h->dtp, LJ, LF)
     if (corr) {
         if (h->g.unit) EMOO_ADJ(true, true);
         else EMOO_ADJ(true, false);
@@ -974,15 +975,15 @@ static int adj_step(emoo_handle *h, AdRun &R, const Snapshot &S, double **L, dou
         EMOO_TRY(adf::planes_adj<double>(h, ops, 0, ops.size(), lslot, pl));
         EMOO_TRY(adf::copy_images_adj<double>(h, lslot, ids9, 9));
         h->launches += 2;
-        k_yee_b_adj<<<grid_all(g, blk), blk, 0, h->stream>>>(g, yc, A);
+        launch_after(k_yee_b_adj<double>, grid_all(g, blk), blk, 0, h->stream)(g, yc, A);
         // the B half overwrote the B role's physical points: the values the
         // planes set there between the halves reach nothing
         adf::Slots9T<double> lb{{A.B[0], A.B[1], A.B[2]}};
-        adf::k_clear_phys<double><<<dim3((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]), blk, 0, h->stream>>>(g, lb);
+        launch_after(adf::k_clear_phys<double>, dim3((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]), blk, 0, h->stream)(g, lb);
         EMOO_TRY(adf::planes_adj<double>(h, ops, 0, ops.size(), lslot, pl));
         EMOO_TRY(adf::copy_images_adj<double>(h, lslot, ids_e, 3));
         h->launches++;
-        k_yee_e_adj<<<grid_all(g, blk), blk, 0, h->stream>>>(g, yc, A, LJ);
+        launch_after(k_yee_e_adj<double>, grid_all(g, blk), blk, 0, h->stream)(g, yc, A, LJ);
         EMOO_TRY(adf::periodic_fold_adj<double>(h, lslot, ids_j, 3));
     } else {
         // 1. executeBC(-1), in reverse
@@ -998,7 +999,7 @@ static int adj_step(emoo_handle *h, AdRun &R, const Snapshot &S, double **L, dou
                     dim3 grd((g.n[o2] + 31) / 32, (g.n[o1] + 7) / 8, 6);
                     for (int side = 1; side >= 0; side--) {
                         h->launches++;
-                        k_ghost_adj<<<grd, blk, 0, h->stream>>>(g, fl, d, side);
+                        launch_after(k_ghost_adj<double>, grd, blk, 0, h->stream)(g, fl, d, side);
                     }
                 }
             } else {
@@ -1011,8 +1012,8 @@ static int adj_step(emoo_handle *h, AdRun &R, const Snapshot &S, double **L, dou
         EMOO_CUDA(cudaGetLastError());
         // 2. Yee update, in reverse (B then E), roles after the step
         h->launches += 2;
-        k_yee_b_adj<<<grid_all(g, blk), blk, 0, h->stream>>>(g, yc, A);
-        k_yee_e_adj<<<grid_all(g, blk), blk, 0, h->stream>>>(g, yc, A, LJ);
+        launch_after(k_yee_b_adj<double>, grid_all(g, blk), blk, 0, h->stream)(g, yc, A);
+        launch_after(k_yee_e_adj<double>, grid_all(g, blk), blk, 0, h->stream)(g, yc, A, LJ);
         // 3. the J fold, in reverse
         for (int d = 2; d >= 0; d--) {
             if (h->bc.fbc[2 * d] != FBC_PERIODIC) continue;
@@ -1021,7 +1022,7 @@ static int adj_step(emoo_handle *h, AdRun &R, const Snapshot &S, double **L, dou
             const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
             dim3 grd((g.n[o2] + 31) / 32, (g.n[o1] + 7) / 8, 2);
             h->launches++;
-            k_fold_adj<<<grd, blk, 0, h->stream>>>(g, d, lslot[f0], lslot[f1]);
+            launch_after(k_fold_adj<double>, grd, blk, 0, h->stream)(g, d, lslot[f0], lslot[f1]);
         }
     }
     // particles: deposit, boundaries, push, gather, in reverse

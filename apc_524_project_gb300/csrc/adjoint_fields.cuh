@@ -57,6 +57,7 @@ YeeCoef<R> yee_coef(const Geom &g, double dt) {
 // gather form over every grid point: LT += LB (physical), LE += dt C_E^T LB.
 template <class R>
 __global__ void k_yee_b_adj(Geom g, YeeCoef<R> yc, FOutT<R> A) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = blockIdx.z;
@@ -91,6 +92,7 @@ __global__ void k_yee_b_adj(Geom g, YeeCoef<R> yc, FOutT<R> A) {
 // cleared.
 template <class R>
 __global__ void k_yee_e_adj(Geom g, YeeCoef<R> yc, FOutT<R> A, JPtrsT<R> LJ) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y * blockDim.y + threadIdx.y;
     const int i = blockIdx.z;
@@ -124,6 +126,7 @@ __global__ void k_yee_e_adj(Geom g, YeeCoef<R> yc, FOutT<R> A, JPtrsT<R> LJ) {
 // range, the two transverse J components): LF[n+1] += LF[1].
 template <class R>
 __global__ void k_fold_adj(Geom g, int d, R *f0, R *f1) {
+    after_previous();
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int r = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -142,6 +145,7 @@ __global__ void k_fold_adj(Geom g, int d, R *f0, R *f1) {
 // transverse physical range): LF[src] += LF[dst], LF[dst] = 0.
 template <class R>
 __global__ void k_ghost_adj(Geom g, Slots6T<R> fl, int d, int side) {
+    after_previous();
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int r = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -166,6 +170,7 @@ __global__ void k_ghost_adj(Geom g, Slots6T<R> fl, int d, int side) {
 // forward steps reversed (so any n is exact). One field per blockIdx.z.
 template <class R>
 __global__ void k_periodic_full_adj(Geom g, Slots9T<R> fl, int d) {
+    after_previous();
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y * blockDim.y + threadIdx.y;
@@ -193,6 +198,7 @@ struct WrapDims {
 // fields: 3.5 us (26 us with a thread a point of the grid for all fields).
 template <class R>
 __global__ void k_copy_images_adj(Geom g, Slots9T<R> fl, WrapDims w, Slabs S) {
+    after_previous();
     int d, c[3];
     if (!slab_point(S, blockIdx.x * blockDim.x + threadIdx.x, d, c)) return;
     unsigned m[3];  // images along each dimension: bit 0 the point itself, 1, 2, 3 index 0, n + 1, n + 2
@@ -254,6 +260,7 @@ __global__ void k_copy_images_adj(Geom g, Slots9T<R> fl, WrapDims w, Slabs S) {
 // shape as the forward; blockIdx.z = component.
 template <class R>
 __global__ void k_mirror_fold_adj(Geom g, Slots9T<R> fl, int d, int right) {
+    after_previous();
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y * blockDim.y + threadIdx.y;
@@ -278,6 +285,7 @@ __global__ void k_mirror_fold_adj(Geom g, Slots9T<R> fl, int d, int right) {
 // overwrites there).
 template <class R>
 __global__ void k_clear_phys(Geom g, Slots9T<R> fl) {
+    after_previous();
     const int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     const int i = blockIdx.z + 1;
@@ -306,6 +314,7 @@ struct PlaneAdjList {
 
 template <class R>
 __global__ void k_plane_adj(Geom g, PlaneAdjList<R> pl, double *sums) {
+    after_previous();
     __shared__ double s_u[32], s_s[32];
     const int entry = blockIdx.y, d = pl.dim, idx = pl.idx[entry];
     R *F = pl.f[entry];
@@ -366,7 +375,7 @@ int planes_adj(emoo_handle *h, const std::vector<AdBcOp> &ops, size_t first, siz
     auto flush = [&]() -> int {
         if (!list.n) return EMOO_OK;
         h->launches++;
-        k_plane_adj<R><<<dim3(PLANE_BLOCKS, list.n), 256, 0, h->stream>>>(h->g, list,
+        launch_after(k_plane_adj<R>, dim3(PLANE_BLOCKS, list.n), 256, 0, h->stream)(h->g, list,
                                                                           pl.sums + 2 * (size_t)PLANE_BLOCKS * start);
         EMOO_CUDA(cudaGetLastError());
         list.n = 0;
@@ -406,13 +415,13 @@ int periodic_fold_adj(emoo_handle *h, R *const *lslot, const int *ids, int nids)
                 if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
                 dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
                 h->launches++;
-                k_mirror_fold_adj<R><<<grd, blk, 0, h->stream>>>(g, fl, d, r);
+                launch_after(k_mirror_fold_adj<R>, grd, blk, 0, h->stream)(g, fl, d, r);
             }
             continue;
         }
         dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, nids);
         h->launches++;
-        k_periodic_full_adj<R><<<grd, blk, 0, h->stream>>>(g, fl, d);
+        launch_after(k_periodic_full_adj<R>, grd, blk, 0, h->stream)(g, fl, d);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -433,7 +442,7 @@ int copy_images_adj(emoo_handle *h, R *const *lslot, const int *ids, int nids) {
     const int64_t points = slab_size(S);
     if (!points) return EMOO_OK;
     h->launches++;
-    k_copy_images_adj<R><<<dim3((unsigned)((points + 127) / 128), nids), 128, 0, h->stream>>>(h->g, fl, w, S);
+    launch_after(k_copy_images_adj<R>, dim3((unsigned)((points + 127) / 128), nids), 128, 0, h->stream)(h->g, fl, w, S);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }

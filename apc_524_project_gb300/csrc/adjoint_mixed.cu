@@ -281,14 +281,14 @@ int adj_fields_corrected_m(emoo_handle *h, const MSnap &S, const std::vector<AdB
     EMOO_TRY(adf::planes_adj<float>(h, ops, 0, ops.size(), lslot, pl));
     EMOO_TRY(adf::copy_images_adj<float>(h, lslot, ids9, 9));
     h->launches += 2;
-    adf::k_yee_b_adj<float><<<grid_all_m(g, blk), blk, 0, h->stream>>>(g, yc, A);
+    launch_after(adf::k_yee_b_adj<float>, grid_all_m(g, blk), blk, 0, h->stream)(g, yc, A);
     // the B half overwrote the B role's physical points
     adf::Slots9T<float> lb{{A.B[0], A.B[1], A.B[2]}};
-    adf::k_clear_phys<float><<<dim3((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]), blk, 0, h->stream>>>(g, lb);
+    launch_after(adf::k_clear_phys<float>, dim3((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]), blk, 0, h->stream)(g, lb);
     EMOO_TRY(adf::planes_adj<float>(h, ops, 0, ops.size(), lslot, pl));
     EMOO_TRY(adf::copy_images_adj<float>(h, lslot, ids_e, 3));
     h->launches++;
-    adf::k_yee_e_adj<float><<<grid_all_m(g, blk), blk, 0, h->stream>>>(g, yc, A, LJ);
+    launch_after(adf::k_yee_e_adj<float>, grid_all_m(g, blk), blk, 0, h->stream)(g, yc, A, LJ);
     EMOO_TRY(adf::periodic_fold_adj<float>(h, lslot, ids_j, 3));
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -331,7 +331,7 @@ int adj_step_m(emoo_handle *h, AdRunM &R, const MSnap &S, const int32_t *cell_af
                 dim3 grd((g.n[o2] + 31) / 32, (g.n[o1] + 7) / 8, 6);
                 for (int side = 1; side >= 0; side--) {
                     h->launches++;
-                    adf::k_ghost_adj<float><<<grd, blk, 0, h->stream>>>(g, fl, d, side);
+                    launch_after(adf::k_ghost_adj<float>, grd, blk, 0, h->stream)(g, fl, d, side);
                 }
             }
         } else {
@@ -347,8 +347,8 @@ int adj_step_m(emoo_handle *h, AdRunM &R, const MSnap &S, const int32_t *cell_af
     dim3 blk(32, 8);
     h->launches += 2;
     const adf::YeeCoef<float> yc = adf::yee_coef<float>(g, h->dtp);
-    adf::k_yee_b_adj<float><<<grid_all_m(g, blk), blk, 0, h->stream>>>(g, yc, A);
-    adf::k_yee_e_adj<float><<<grid_all_m(g, blk), blk, 0, h->stream>>>(g, yc, A, LJ);
+    launch_after(adf::k_yee_b_adj<float>, grid_all_m(g, blk), blk, 0, h->stream)(g, yc, A);
+    launch_after(adf::k_yee_e_adj<float>, grid_all_m(g, blk), blk, 0, h->stream)(g, yc, A, LJ);
     for (int d = 2; d >= 0; d--) {
         if (h->bc.fbc[2 * d] != FBC_PERIODIC) continue;
         const int f0 = (d == 0) ? EMOO_JY : EMOO_JX;
@@ -356,7 +356,7 @@ int adj_step_m(emoo_handle *h, AdRunM &R, const MSnap &S, const int32_t *cell_af
         const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
         dim3 grd((g.n[o2] + 31) / 32, (g.n[o1] + 7) / 8, 2);
         h->launches++;
-        adf::k_fold_adj<float><<<grd, blk, 0, h->stream>>>(g, d, lslot[f0], lslot[f1]);
+        launch_after(adf::k_fold_adj<float>, grd, blk, 0, h->stream)(g, d, lslot[f0], lslot[f1]);
     }
     EMOO_CUDA(cudaGetLastError());
     const FOutF LF = field_out_f(lslot, S.bswap);

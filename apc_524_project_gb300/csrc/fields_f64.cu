@@ -36,6 +36,7 @@ dim3 phys_grid(const Geom &g, dim3 blk) {
 // Grid::evolveFields, E half (src/grid/oGrid.cpp:23-40): E -= dt (curl-ish of
 // B_tm1 + 4 pi J) over physical points, B_tm1 being the freshly swapped role.
 __global__ void k_yee_e(Geom g, double dt, F3 E, CF3 T, CF3 J) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int i = blockIdx.z + 1;
@@ -57,6 +58,7 @@ __global__ void k_yee_e(Geom g, double dt, F3 E, CF3 T, CF3 J) {
 // Grid::evolveFields, B half (src/grid/oGrid.cpp:43-57): B = B_tm1 + dt curl E.
 // Reads the E ghost planes as they are (refreshed only after the update).
 __global__ void k_yee_b(Geom g, double dt, F3 B, CF3 T, CF3 E) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int i = blockIdx.z + 1;
@@ -74,6 +76,7 @@ __global__ void k_yee_b(Geom g, double dt, F3 B, CF3 T, CF3 E) {
 
 // Grid::evolveFieldsES, src/grid/oGrid.cpp:67-81
 __global__ void k_yee_es(Geom g, double dt, F3 E, CF3 J) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int i = blockIdx.z + 1;
@@ -97,6 +100,7 @@ struct FieldList {
 // physical points and write ghost points, so any set of dims runs at once.
 // blockIdx.z = (field * 3 + dim) * 2 + side.
 __global__ void k_ghost(Geom g, FieldList fl, int dims_mask, const int *skip) {
+    after_previous();
     if (skip && *skip) return;
     int z = blockIdx.z;
     int r = z & 1;
@@ -122,6 +126,7 @@ __global__ void k_ghost(Geom g, FieldList fl, int dims_mask, const int *skip) {
 // side, src/boundaries/b_fields/bc_f_periodic.cpp:40-46): the two transverse
 // J components and rho of ghost plane n+1 are added into plane 1.
 __global__ void k_fold(Geom g, int d, double *f0, double *f1, double *f2) {
+    after_previous();
     int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     int q = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int p = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -143,6 +148,7 @@ struct PlaneList {
 
 // Grid::setFieldInPlane over the whole (n+3)^2 plane, src/grid/oGrid.cpp:446-476.
 __global__ void k_plane_set(Geom g, PlaneList pl, const int *skip) {
+    after_previous();
     if (skip && *skip) return;
     int e = blockIdx.z;
     if (e >= pl.n) return;
@@ -162,6 +168,7 @@ __global__ void k_plane_set(Geom g, PlaneList pl, const int *skip) {
 }
 
 __global__ void k_fill(double *p, int64_t n, double v) {
+    after_previous();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         p[i] = v;
 }
@@ -544,6 +551,7 @@ __global__ void k_jacobi_fused(Geom g, const double *src, double *dst, const dou
 
 // phiToE, src/poisson/convertFields.cpp:20-68 (reads phi1 storage).
 __global__ void k_phi_to_e(Geom g, const double *phi, F3 E) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int i = blockIdx.z + 1;
@@ -557,6 +565,7 @@ __global__ void k_phi_to_e(Geom g, const double *phi, F3 E) {
 // AToB, src/poisson/convertFields.cpp:83-154, including its use of the same
 // A component in both differences.
 __global__ void k_a_to_b(Geom g, const double *Ax, const double *Ay, const double *Az, F3 B) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int i = blockIdx.z + 1;
@@ -573,6 +582,7 @@ __global__ void k_a_to_b(Geom g, const double *Ax, const double *Ay, const doubl
 // Per-block partial sums of the six field energies of the history row
 // (src/IO/output.cpp:98-114; SQR(x) expands to x*x unparenthesised).
 __global__ void k_field_energy(Geom g, CF3 E, CF3 B, double *part) {
+    after_previous();
     double acc[6] = {0, 0, 0, 0, 0, 0};
     int64_t nphys = (int64_t)g.n[0] * g.n[1] * g.n[2];
     double hv = 0.5 * g.vol;
@@ -672,7 +682,7 @@ int yee_f64(emoo_handle *h, double dt) {
     CF3 T = {{role_t(h, 0), role_t(h, 1), role_t(h, 2)}};
     CF3 J = {{h->slot[EMOO_JX], h->slot[EMOO_JY], h->slot[EMOO_JZ]}};
     h->launches++;
-    k_yee_e<<<grd, blk, 0, h->stream>>>(g, dt, E, T, J);
+    launch_after(k_yee_e, grd, blk, 0, h->stream)(g, dt, E, T, J);
     // The B half reads E one plane past the high faces. The reference refreshes
     // those ghosts only after both halves, so at the periodic wrap B sees the
     // previous step's E: the leapfrog loses its time centring there and vacuum
@@ -681,7 +691,7 @@ int yee_f64(emoo_handle *h, double dt) {
     F3 B = {{role_b(h, 0), role_b(h, 1), role_b(h, 2)}};
     CF3 Ec = {{E.p[0], E.p[1], E.p[2]}};
     h->launches++;
-    k_yee_b<<<grd, blk, 0, h->stream>>>(g, dt, B, T, Ec);
+    launch_after(k_yee_b, grd, blk, 0, h->stream)(g, dt, B, T, Ec);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -695,11 +705,11 @@ int yee_half_f64(emoo_handle *h, double dt, int half) {
     if (half == 0) {
         F3 E = {{h->slot[EMOO_EX], h->slot[EMOO_EY], h->slot[EMOO_EZ]}};
         CF3 J = {{h->slot[EMOO_JX], h->slot[EMOO_JY], h->slot[EMOO_JZ]}};
-        k_yee_e<<<grd, blk, 0, h->stream>>>(g, dt, E, T, J);
+        launch_after(k_yee_e, grd, blk, 0, h->stream)(g, dt, E, T, J);
     } else {
         F3 B = {{role_b(h, 0), role_b(h, 1), role_b(h, 2)}};
         CF3 E = {{h->slot[EMOO_EX], h->slot[EMOO_EY], h->slot[EMOO_EZ]}};
-        k_yee_b<<<grd, blk, 0, h->stream>>>(g, dt, B, T, E);
+        launch_after(k_yee_b, grd, blk, 0, h->stream)(g, dt, B, T, E);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -711,7 +721,7 @@ int yee_es_f64(emoo_handle *h, double dt) {
     F3 E = {{h->slot[EMOO_EX], h->slot[EMOO_EY], h->slot[EMOO_EZ]}};
     CF3 J = {{h->slot[EMOO_JX], h->slot[EMOO_JY], h->slot[EMOO_JZ]}};
     h->launches++;
-    k_yee_es<<<phys_grid(g, blk), blk, 0, h->stream>>>(g, dt, E, J);
+    launch_after(k_yee_es, phys_grid(g, blk), blk, 0, h->stream)(g, dt, E, J);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -726,7 +736,7 @@ static int ghost_launch(emoo_handle *h, const int *ids, int nids, int dims_mask,
     dim3 blk(32, 8);
     dim3 grd((tb + 31) / 32, (ta + 7) / 8, nids * 6);
     h->launches++;
-    k_ghost<<<grd, blk, 0, h->stream>>>(g, fl, dims_mask, skip);
+    launch_after(k_ghost, grd, blk, 0, h->stream)(g, fl, dims_mask, skip);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -751,7 +761,7 @@ int fold_f64(emoo_handle *h, int d, int what) {
     }
     dim3 grd((g.n[o2] + 31) / 32, (g.n[o1] + 7) / 8, nz);
     h->launches++;
-    k_fold<<<grd, blk, 0, h->stream>>>(g, d, a, b, r);
+    launch_after(k_fold, grd, blk, 0, h->stream)(g, d, a, b, r);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -766,6 +776,7 @@ struct Slots9 {
 // f[n] += f[0], f[1] += f[n+1], f[2] += f[n+2] (the ghost planes' deposits to
 // their periodic images). One field per blockIdx.z.
 __global__ void k_periodic_full(Geom g, Slots9 fl, int d) {
+    after_previous();
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y * blockDim.y + threadIdx.y;
@@ -793,6 +804,7 @@ struct Wrap {
 // fields' loads in flight together. 49 x 37 x 29 cells, nine fields: 4.0 us
 // (9.6 us from the sources, a thread a point of the grid).
 __global__ void k_copy_images(Geom g, Slots9 fl, int nf, Wrap w, Slabs S) {
+    after_previous();
     int c[3], of[3];
     if (!ghost_point(S, g.n, w.w, blockIdx.x * blockDim.x + threadIdx.x, c, of)) return;
     const int64_t o = gidx(g, c[0], c[1], c[2]), from = gidx(g, of[0], of[1], of[2]);
@@ -814,6 +826,7 @@ __global__ void k_copy_images(Geom g, Slots9 fl, int nf, Wrap w, Slabs S) {
 // 1, transverse plane 0 -> 2; right wall (plane n+1): normal edge n+1 -> n,
 // transverse plane n+2 -> n. Whole transverse range; blockIdx.z = component.
 __global__ void k_mirror_fold(Geom g, Slots9 fl, int d, int right) {
+    after_previous();
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y * blockDim.y + threadIdx.y;
@@ -854,13 +867,13 @@ static int periodic_fold(emoo_handle *h, const int *ids, int nids) {
                 if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
                 dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
                 h->launches++;
-                k_mirror_fold<<<grd, blk, 0, h->stream>>>(g, fl, d, r);
+                launch_after(k_mirror_fold, grd, blk, 0, h->stream)(g, fl, d, r);
             }
             continue;
         }
         dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, nids);
         h->launches++;
-        k_periodic_full<<<grd, blk, 0, h->stream>>>(g, fl, d);
+        launch_after(k_periodic_full, grd, blk, 0, h->stream)(g, fl, d);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -910,7 +923,7 @@ int periodic_copies_f64(emoo_handle *h, const int *ids, int nids) {
     const int64_t ghosts = slab_size(S);
     if (!ghosts) return EMOO_OK;
     h->launches++;
-    k_copy_images<<<(unsigned)((ghosts + 127) / 128), 128, 0, h->stream>>>(h->g, fl, nids, w, S);
+    launch_after(k_copy_images, (unsigned)((ghosts + 127) / 128), 128, 0, h->stream)(h->g, fl, nids, w, S);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -932,7 +945,7 @@ static int plane_launch(emoo_handle *h, const PlaneSet *ps, int n, const int *sk
         dim3 blk(32, 8);
         dim3 grd((m + 31) / 32, (m + 7) / 8, pl.n);
         h->launches++;
-        k_plane_set<<<grd, blk, 0, h->stream>>>(g, pl, skip);
+        launch_after(k_plane_set, grd, blk, 0, h->stream)(g, pl, skip);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -966,7 +979,7 @@ int fill_f64(emoo_handle *h, double *p, int64_t n, double v, cudaStream_t s) {
     int64_t b = std::min<int64_t>((n + 255) / 256, 152 * 16);
     if (b < 1) b = 1;
     h->launches++;
-    k_fill<<<(int)b, 256, 0, s>>>(p, n, v);
+    launch_after(k_fill, (int)b, 256, 0, s)(p, n, v);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -1173,7 +1186,7 @@ int phi_to_e_f64(emoo_handle *h) {
     dim3 blk(32, 8);
     F3 E = {{h->slot[EMOO_EX], h->slot[EMOO_EY], h->slot[EMOO_EZ]}};
     h->launches++;
-    k_phi_to_e<<<phys_grid(g, blk), blk, 0, h->stream>>>(g, h->slot[EMOO_PHI1], E);
+    launch_after(k_phi_to_e, phys_grid(g, blk), blk, 0, h->stream)(g, h->slot[EMOO_PHI1], E);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -1184,7 +1197,7 @@ int a_to_b_f64(emoo_handle *h) {
     // AToB writes through the field pointer table: the fixed B slots.
     F3 B = {{h->slot[EMOO_BX], h->slot[EMOO_BY], h->slot[EMOO_BZ]}};
     h->launches++;
-    k_a_to_b<<<phys_grid(g, blk), blk, 0, h->stream>>>(g, h->slot[EMOO_AX1], h->slot[EMOO_AY1], h->slot[EMOO_AZ1], B);
+    launch_after(k_a_to_b, phys_grid(g, blk), blk, 0, h->stream)(g, h->slot[EMOO_AX1], h->slot[EMOO_AY1], h->slot[EMOO_AZ1], B);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -1197,7 +1210,7 @@ int field_energy_f64(emoo_handle *h, double out6[6]) {
     // the history reads the field pointer table: fixed B slots
     CF3 B = {{h->slot[EMOO_BX], h->slot[EMOO_BY], h->slot[EMOO_BZ]}};
     h->launches++;
-    k_field_energy<<<rb, 256, 0, h->stream>>>(g, E, B, h->red);
+    launch_after(k_field_energy, rb, 256, 0, h->stream)(g, E, B, h->red);
     EMOO_CUDA(cudaGetLastError());
     std::vector<double> part((size_t)rb * 6);
     EMOO_CUDA(cudaMemcpyAsync(part.data(), h->red, part.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));

@@ -113,6 +113,7 @@ __device__ __forceinline__ R nb_sum(const Lv &L, const C *c, const R *u, int i, 
 // taken over the FP32 values (the stop test needs no more): this kernel runs
 // on the FP64 pipe, so everything after the residual itself stays off it.
 __global__ void k_mg_residual64(Lv L, Fine F, double *dmax) {
+    after_previous();
     __shared__ float sh[8];
     const int k = L.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = L.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
@@ -223,6 +224,7 @@ __device__ __forceinline__ float prolong_value(const LV &Cl, const LV &F, int i,
 // One colour of a red-black Gauss-Seidel sweep: the points with
 // (i + j + k) & 1 == colour take u = (neighbour sum - f) / diag.
 __global__ void k_mg_smooth(Lv L, int colour) {
+    after_previous();
     const int j = L.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = L.lo[0] + blockIdx.z;
     if (j > L.hi[1] || i > L.hi[0]) return;
@@ -234,6 +236,7 @@ __global__ void k_mg_smooth(Lv L, int colour) {
 
 // One damped Jacobi half-step at the unknowns, src -> dst.
 __global__ void k_mg_jacobi(Lv L, const float *src, float *dst) {
+    after_previous();
     const int k = L.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = L.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = L.lo[0] + blockIdx.z;
@@ -245,6 +248,7 @@ __global__ void k_mg_jacobi(Lv L, const float *src, float *dst) {
 
 // w = f - Laplacian(u) at the unknowns (FP32 levels)
 __global__ void k_mg_residual(Lv L) {
+    after_previous();
     const int k = L.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = L.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = L.lo[0] + blockIdx.z;
@@ -254,6 +258,7 @@ __global__ void k_mg_residual(Lv L) {
 }
 
 __global__ void k_mg_restrict(Lv F, Lv Cl) {
+    after_previous();
     const int K = Cl.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int J = Cl.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int I = Cl.lo[0] + blockIdx.z;
@@ -262,6 +267,7 @@ __global__ void k_mg_restrict(Lv F, Lv Cl) {
 }
 
 __global__ void k_mg_prolong(Lv Cl, Lv F) {
+    after_previous();
     const int k = F.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = F.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = F.lo[0] + blockIdx.z;
@@ -271,6 +277,7 @@ __global__ void k_mg_prolong(Lv Cl, Lv F) {
 
 // u += e at the unknowns (e: level 0's correction)
 __global__ void k_mg_correct(Lv L, Fine F) {
+    after_previous();
     const int k = L.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = L.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = L.lo[0] + blockIdx.z;
@@ -365,6 +372,7 @@ __device__ __forceinline__ void column(const Lv &L, const float *from, const flo
 template <bool RBGS, int MODE>
 __global__ void __launch_bounds__(TILE_THREADS, 1) k_mg_tile(const __grid_constant__ Lv L, const __grid_constant__ Lv C,
                                                              const __grid_constant__ TileLeg G) {
+    after_previous();
     extern __shared__ float sm[];
     const int bt[3] = {(int)blockIdx.z, (int)blockIdx.y, (int)blockIdx.x};
     int b0[3], bs[3], first[3], last[3];  // tile with halo: origin and size; its own points
@@ -709,6 +717,7 @@ __device__ void tail_up(const Tail &T, int l, float *sm) {
 }
 
 __global__ void __launch_bounds__(TAIL_THREADS) k_mg_tail(const __grid_constant__ Tail T) {
+    after_previous();
     extern __shared__ float sm[];
     for (int t = threadIdx.x; t < T.smem; t += blockDim.x) sm[t] = 0.0f;
     __syncthreads();
@@ -741,6 +750,7 @@ __global__ void __launch_bounds__(TAIL_THREADS) k_mg_tail(const __grid_constant_
 // the FP64 problem from the grid slots: u takes the slot's values on the
 // unknowns and on external boundary planes (the PoissonBC values), f = mult R
 __global__ void k_mg_load(Geom g, Lv L, Fine F, const double *slot, const double *R, double mult) {
+    after_previous();
     const int k = 1 + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = 1 + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = 1 + blockIdx.z;
@@ -753,6 +763,7 @@ __global__ void k_mg_load(Geom g, Lv L, Fine F, const double *slot, const double
 
 // the unknowns of the solution (less `shift`) into the zeroed slot
 __global__ void k_mg_store(Geom g, Lv L, const double *u, double *slot, double shift) {
+    after_previous();
     const int k = L.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = L.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = L.lo[0] + blockIdx.z;
@@ -762,6 +773,7 @@ __global__ void k_mg_store(Geom g, Lv L, const double *u, double *slot, double s
 
 // per-block sums of a over the unknowns (fixed order within a block)
 __global__ void k_mg_sum(Lv L, const double *a, double *part) {
+    after_previous();
     __shared__ double sh[32];
     const int64_t m0 = L.hi[0] - L.lo[0] + 1, m1 = L.hi[1] - L.lo[1] + 1, m2 = L.hi[2] - L.lo[2] + 1;
     const int64_t n = m0 * m1 * m2;
@@ -785,6 +797,7 @@ __global__ void k_mg_sum(Lv L, const double *a, double *part) {
 }
 
 __global__ void k_mg_shift(Lv L, double *a, double m) {
+    after_previous();
     const int k = L.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = L.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = L.lo[0] + blockIdx.z;
@@ -870,7 +883,7 @@ void tile_leg(emoo_handle *h, int mode, const Lv &L, const Lv &C, TileLeg G, int
     G.T = tile_size(L, mode == SWEEP);
     const dim3 grd((L.P[2] + G.T - 1) / G.T, (L.P[1] + G.T - 1) / G.T, (L.P[0] + G.T - 1) / G.T);
     launches++;
-    tile_kernel(L, mode)<<<grd, G.T == 8 ? TILE_THREADS : TILE_THREADS / 2, tile_smem(L, G.T, mode), h->stream>>>(L, C, G);
+    launch_after(tile_kernel(L, mode), grd, G.T == 8 ? TILE_THREADS : TILE_THREADS / 2, tile_smem(L, G.T, mode), h->stream)(L, C, G);
 }
 
 int coarse_sweeps(const Lv &L) {
@@ -947,8 +960,8 @@ void smooth(emoo_handle *h, const Lv &L, int sweeps, int &launches) {
     if (!L.rb) {
         for (int s = 0; s < sweeps; s++) {
             launches += 2;
-            k_mg_jacobi<<<pts_grid(L, blk), blk, 0, h->stream>>>(L, L.u, L.w);
-            k_mg_jacobi<<<pts_grid(L, blk), blk, 0, h->stream>>>(L, L.w, L.u);
+            launch_after(k_mg_jacobi, pts_grid(L, blk), blk, 0, h->stream)(L, L.u, L.w);
+            launch_after(k_mg_jacobi, pts_grid(L, blk), blk, 0, h->stream)(L, L.w, L.u);
         }
         return;
     }
@@ -957,7 +970,7 @@ void smooth(emoo_handle *h, const Lv &L, int sweeps, int &launches) {
     for (int s = 0; s < sweeps; s++)
         for (int c = 0; c < 2; c++) {
             launches++;
-            k_mg_smooth<<<grd, blk, 0, h->stream>>>(L, c);
+            launch_after(k_mg_smooth, grd, blk, 0, h->stream)(L, c);
         }
 }
 
@@ -969,7 +982,7 @@ const float *vcycle(emoo_handle *h, MgState *s, size_t l, int &launches) {
     if (l == s->tail_from) {
         const Tail T = make_tail(s, l);
         launches++;
-        k_mg_tail<<<1, TAIL_THREADS, T.smem * sizeof(float), h->stream>>>(T);
+        launch_after(k_mg_tail, 1, TAIL_THREADS, T.smem * sizeof(float), h->stream)(T);
         return L.u;
     }
     dim3 blk(32, 8);
@@ -994,16 +1007,16 @@ const float *vcycle(emoo_handle *h, MgState *s, size_t l, int &launches) {
     if (!coarsest) {
         Lv C = s->lv[l + 1];
         launches += 2;
-        k_mg_residual<<<pts_grid(L, blk), blk, 0, h->stream>>>(L);
-        k_mg_restrict<<<pts_grid(C, blk), blk, 0, h->stream>>>(L, C);
+        launch_after(k_mg_residual, pts_grid(L, blk), blk, 0, h->stream)(L);
+        launch_after(k_mg_restrict, pts_grid(C, blk), blk, 0, h->stream)(L, C);
         C.u = const_cast<float *>(vcycle(h, s, l + 1, launches));
         launches++;
-        k_mg_prolong<<<pts_grid(L, blk), blk, 0, h->stream>>>(C, L);
+        launch_after(k_mg_prolong, pts_grid(L, blk), blk, 0, h->stream)(C, L);
         smooth(h, L, NU, launches);
     }
     if (l == 0) {
         launches++;
-        k_mg_correct<<<pts_grid(L, blk), blk, 0, h->stream>>>(L, s->fine);
+        launch_after(k_mg_correct, pts_grid(L, blk), blk, 0, h->stream)(L, s->fine);
     }
     return L.u;
 }
@@ -1014,7 +1027,7 @@ void residual64(emoo_handle *h, MgState *s, int &launches) {
     const Lv &L0 = s->lv[0];
     cudaMemsetAsync(s->dmax, 0, sizeof(double), h->stream);
     launches++;
-    k_mg_residual64<<<pts_grid(L0, blk), blk, 0, h->stream>>>(L0, s->fine, s->dmax);
+    launch_after(k_mg_residual64, pts_grid(L0, blk), blk, 0, h->stream)(L0, s->fine, s->dmax);
     cudaMemcpyAsync(s->hmax, s->dmax, sizeof(double), cudaMemcpyDeviceToHost, h->stream);
 }
 
@@ -1134,7 +1147,7 @@ int mg_setup(emoo_handle *h, MgState *s) {
 
 int sum_unknowns(emoo_handle *h, MgState *s, const double *a, double *out) {
     h->launches++;
-    k_mg_sum<<<RB, 256, 0, h->stream>>>(s->lv[0], a, s->part);
+    launch_after(k_mg_sum, RB, 256, 0, h->stream)(s->lv[0], a, s->part);
     EMOO_CUDA(cudaGetLastError());
     EMOO_CUDA(cudaMemcpyAsync(s->hpart, s->part, RB * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     EMOO_CUDA(cudaStreamSynchronize(h->stream));
@@ -1184,7 +1197,7 @@ int multigrid_f64(emoo_handle *h, int id1, int id2, int rid, double mult, int *c
         const int ei = L0.per[0] ? L0.P[0] : L0.P[0] + 1;
         dim3 grd((ek + blk.x - 1) / blk.x, (ej + blk.y - 1) / blk.y, ei);
         h->launches++;
-        k_mg_load<<<grd, blk, 0, h->stream>>>(g, L0, s->fine, h->slot[id1], h->slot[rid], mult);
+        launch_after(k_mg_load, grd, blk, 0, h->stream)(g, L0, s->fine, h->slot[id1], h->slot[rid], mult);
     }
     const bool allper = L0.per[0] && L0.per[1] && L0.per[2];
     const double nunk = (double)unknowns(L0);
@@ -1192,7 +1205,7 @@ int multigrid_f64(emoo_handle *h, int id1, int id2, int rid, double mult, int *c
         double sum;
         EMOO_TRY(sum_unknowns(h, s, s->fine.f, &sum));
         h->launches++;
-        k_mg_shift<<<pts_grid(L0, blk), blk, 0, h->stream>>>(L0, s->fine.f, sum / nunk);
+        launch_after(k_mg_shift, pts_grid(L0, blk), blk, 0, h->stream)(L0, s->fine.f, sum / nunk);
     }
     int launches = 0;
     residual64(h, s, launches);
@@ -1218,7 +1231,7 @@ int multigrid_f64(emoo_handle *h, int id1, int id2, int rid, double mult, int *c
         shift = sum / nunk;
     }
     h->launches++;
-    k_mg_store<<<pts_grid(L0, blk), blk, 0, h->stream>>>(g, L0, s->fine.u, h->slot[id1], shift);
+    launch_after(k_mg_store, pts_grid(L0, blk), blk, 0, h->stream)(g, L0, s->fine.u, h->slot[id1], shift);
     EMOO_CUDA(cudaGetLastError());
     EMOO_TRY(poisson_field_bc(h, id1));
     EMOO_CUDA(cudaMemcpyAsync(h->slot[id2], h->slot[id1], (size_t)g.npts * sizeof(double), cudaMemcpyDeviceToDevice,

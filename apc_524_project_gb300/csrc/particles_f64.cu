@@ -287,6 +287,7 @@ __global__ void k_particle_bc(BCTab bc, PState S, int64_t np, DevCounters *ctr) 
 // what: 0 J, 1 J and rho, 2 rho only
 __global__ void __launch_bounds__(PART_BLOCK) k_deposit(Geom g, SpeciesTab st, PState S, int64_t np, DepositPtrs D,
                                                         int what, DevCounters *ctr) {
+    after_previous<false>();
     __shared__ CommitTile tiles[PART_WARPS];
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     bool active = false;
@@ -420,6 +421,7 @@ template <bool REL, int MODE>
 __global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
                                                          int64_t np, DepositPtrs D, double dt,
                                                          DevCounters *ctr) {
+    after_previous<false>();
     constexpr bool UNIT = MODE != ANY;
     __shared__ CommitTile tiles[PART_WARPS];
     __shared__ double s_move[6][PART_BLOCK];  // start and end of the listed moves
@@ -529,6 +531,7 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, 
 template <bool REL, int MODE>
 __global__ void __launch_bounds__(PART_BLOCK) k_fused(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
                                                       int64_t np, DepositPtrs D, double dt, DevCounters *ctr) {
+    after_previous<false>();
     constexpr bool UNIT = MODE != ANY;
     __shared__ CommitTile tiles[PART_WARPS];
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -583,6 +586,7 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused(Geom g, SpeciesTab st, BCT
 // Per-block partial sums of the history's particle terms
 // (src/IO/output.cpp:76-87): {sum 1/2 m v^2, sum m vx, sum m vy, sum m vz}.
 __global__ void k_moments(SpeciesTab st, PState S, int64_t np, double *part) {
+    after_previous();
     double acc[4] = {0, 0, 0, 0};
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < np; p += (int64_t)gridDim.x * blockDim.x) {
         double vx = S.vx[p], vy = S.vy[p], vz = S.vz[p];
@@ -611,6 +615,7 @@ __global__ void k_moments(SpeciesTab st, PState S, int64_t np, double *part) {
 // Sort keys: species * ncell + reference cellID; removed particles get the
 // largest key so they end up behind every live one.
 __global__ void k_keys(Geom g, SpeciesTab st, PState S, int64_t np, uint32_t *key, uint32_t dead_key, DevCounters *ctr) {
+    after_previous();
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= np) return;
     double x = S.x[p];
@@ -742,7 +747,7 @@ int deposit_f64(emoo_handle *h, int with_rho) {
     SpeciesTab st;
     species_tab(h, h->dtp, st);
     h->launches++;
-    k_deposit<<<blocks_for(h->np), 256, 0, h->stream>>>(h->g, st, pstate(h), h->np, deposit_ptrs(h), with_rho, h->ctr);
+    launch_after(k_deposit, blocks_for(h->np), 256, 0, h->stream)(h->g, st, pstate(h), h->np, deposit_ptrs(h), with_rho, h->ctr);
     EMOO_CUDA(cudaGetLastError());
     return rho_background_f64(h, with_rho);
 }
@@ -755,7 +760,7 @@ int deposit_rho_f64(emoo_handle *h) {
         SpeciesTab st;
         species_tab(h, h->dtp, st);
         h->launches++;
-        k_deposit<<<blocks_for(h->np), 256, 0, h->stream>>>(h->g, st, pstate(h), h->np, deposit_ptrs(h), 2, h->ctr);
+        launch_after(k_deposit, blocks_for(h->np), 256, 0, h->stream)(h->g, st, pstate(h), h->np, deposit_ptrs(h), 2, h->ctr);
         EMOO_CUDA(cudaGetLastError());
     }
     return rho_background_f64(h, 1);
@@ -765,10 +770,10 @@ template <bool REL, int MODE>
 static void launch_fused(emoo_handle *h, const SpeciesTab &st, double dtp) {
     const int nb = blocks_for(h->np, PART_BLOCK);
     if (h->policy == EMOO_POLICY_CORRECTED)
-        k_fused_vb<REL, MODE><<<nb, PART_BLOCK, 0, h->stream>>>(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
+        launch_after(k_fused_vb<REL, MODE>, nb, PART_BLOCK, 0, h->stream)(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
                                                                 deposit_ptrs(h), dtp, h->ctr);
     else
-        k_fused<REL, MODE><<<nb, PART_BLOCK, 0, h->stream>>>(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
+        launch_after(k_fused<REL, MODE>, nb, PART_BLOCK, 0, h->stream)(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
                                                              deposit_ptrs(h), dtp, h->ctr);
 }
 
@@ -811,7 +816,7 @@ int particle_moments_f64(emoo_handle *h, double out4[4]) {
     SpeciesTab st;
     species_tab(h, h->dtp, st);
     h->launches++;
-    k_moments<<<nb, 256, 0, h->stream>>>(st, pstate(h), h->np, h->red);
+    launch_after(k_moments, nb, 256, 0, h->stream)(st, pstate(h), h->np, h->red);
     EMOO_CUDA(cudaGetLastError());
     std::vector<double> part((size_t)nb * 4);
     EMOO_CUDA(cudaMemcpyAsync(part.data(), h->red, part.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -858,7 +863,7 @@ int sort_keys_f64(emoo_handle *h) {
     species_tab(h, h->dtp, st);
     uint32_t dead = (uint32_t)((int64_t)h->nspec * h->g.ncell + 1);
     h->launches++;
-    k_keys<<<blocks_for(h->np), 256, 0, h->stream>>>(h->g, st, pstate(h), h->np, h->key[0], dead, h->ctr);
+    launch_after(k_keys, blocks_for(h->np), 256, 0, h->stream)(h->g, st, pstate(h), h->np, h->key[0], dead, h->ctr);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }

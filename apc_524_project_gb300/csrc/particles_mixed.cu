@@ -289,6 +289,7 @@ __device__ __forceinline__ float4 edge_coef_true(float f00, float f10, float f11
 // that follows accumulates into (a fill of its own costs a launch more).
 template <bool CORR>
 __global__ void __launch_bounds__(256) k_pack_m(MGeom g, MGather P, float4 *__restrict__ pack, uint4 *wj) {
+    after_previous();
     __shared__ float4 stage[8][32 * PACK_F4];
     const int lane = threadIdx.x, k0 = blockIdx.x * 32 + 1, k = k0 + lane;
     const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -889,6 +890,7 @@ template <bool REL, bool FIRST, bool CORR = false, bool HOST = false>
 __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
     k_fused_m(MGeom g, Div3 dv, MSpecies st, BCTab bc, const float4 *__restrict__ pack, MState S, int64_t np,
               MDeposit D, const float *g0, DevCounters *ctr, const MHost *__restrict__ Hp, int store_pre) {
+    after_previous<false>();
     __shared__ __align__(16) float s_w[FUSED_WARPS][DEP_JSLOTS * COL_STRIDE];
     __shared__ int s_key[FUSED_WARPS][32];
     constexpr bool VBL = CORR;  // the corrected policy's pieces go through a list
@@ -1116,6 +1118,7 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
 template <bool CORR>
 __global__ void __launch_bounds__(256) k_deposit_m(MGeom g, Div3 dv, MSpecies st, MState S, int64_t np, MDeposit D, int what,
                                                    int gam) {
+    after_previous<false>();
     __shared__ __align__(16) float s_w[8][20 * COL_STRIDE];
     __shared__ int s_key[8][32];
     const int64_t p = (int64_t)(blockIdx.x * blockDim.x + threadIdx.x);
@@ -1182,9 +1185,9 @@ struct MFold {
 // One component of J at point (i, j, k), unfolded: the sum of the four record
 // slots that feed it (slot q of cell p - off(q), the inverse of the deposit
 // table; corr: the corrected policy's Jx index, slot 4 from cell p - 1).
-__device__ __forceinline__ unsigned long long j_raw(const unsigned long long *__restrict__ wj, int64_t p, int sx, int sy,
+__device__ __forceinline__ unsigned long long j_raw(const unsigned long long *wj, int64_t p, int sx, int sy,
                                                     int a, bool corr) {
-    auto slot = [&](int64_t c, int k) -> unsigned long long { return c >= 0 ? __ldg(wj + c * DEP_JSLOTS + k) : 0ull; };
+    auto slot = [&](int64_t c, int k) -> unsigned long long { return c >= 0 ? wj[c * DEP_JSLOTS + k] : 0ull; };
     if (a == 0) return slot(p, 0) + slot(p - sy, 3) + slot(corr ? p - 1 : p - sy, 4) + slot(p - sy - 1, 7);
     if (a == 1) return slot(p, 1) + slot(p - 1, 6) + slot(p - sx - 1, 8) + slot(p - sx, 10);
     return slot(p, 2) + slot(p - sy, 5) + slot(p - sx - sy, 9) + slot(p - sx, 11);
@@ -1227,9 +1230,10 @@ __device__ __forceinline__ bool fold_reaches(const MGeom &g, const MFold &f, int
 // instead of 22. Integer sums: the same words as a gather, three folds and the
 // update one after the other, which took five launches and read J again.
 template <bool CORR>
-__global__ void __launch_bounds__(256) k_current_e_m(MGeom g, MFold f, const unsigned long long *__restrict__ wj, MFix4 J,
+__global__ void __launch_bounds__(256) k_current_e_m(MGeom g, MFold f, const unsigned long long *wj, MFix4 J,
                                                      MF3 E, MCF3 T, float dt, float q0, int es, int t1, int t2, Slabs S,
                                                      int planes) {
+    after_previous();
     int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
     const bool edge = CORR && (int)blockIdx.z >= planes;
     if (edge) {
@@ -1253,18 +1257,19 @@ __global__ void __launch_bounds__(256) k_current_e_m(MGeom g, MFold f, const uns
     unsigned long long c[3];
     if (edge) {
     } else if (o >= (int64_t)sx + sy + 1) {
-        // J record of cell c: wj + 12 c (96 bytes, 32-byte aligned)
+        // J record of cell c: wj + 12 c (96 bytes, 32-byte aligned). Plain loads: the
+        // read-only path may be taken ahead of after_previous().
         auto rec = [&](int64_t q) { return wj + q * DEP_JSLOTS; };
-        const ulonglong2 g0a = __ldg(reinterpret_cast<const ulonglong2 *>(rec(o)));  // slots 0, 1
-        const unsigned long long g0b = __ldg(rec(o) + 2);
-        const unsigned long long g2a = __ldg(rec(o - sy) + 3);
-        const ulonglong2 g2b = __ldg(reinterpret_cast<const ulonglong2 *>(rec(o - sy) + 4));  // 4, 5
-        const unsigned long long g1 = __ldg(rec(o - 1) + 6);
-        const unsigned long long g3 = __ldg(rec(o - sy - 1) + 7);
-        const unsigned long long g5 = __ldg(rec(o - sx - 1) + 8);
-        const unsigned long long g6 = __ldg(rec(o - sx - sy) + 9);
-        const ulonglong2 g4 = __ldg(reinterpret_cast<const ulonglong2 *>(rec(o - sx) + 10));  // 10, 11
-        const unsigned long long q3 = CORR ? __ldg(rec(o - 1) + 4) : g2b.x;
+        const ulonglong2 g0a = *reinterpret_cast<const ulonglong2 *>(rec(o));  // slots 0, 1
+        const unsigned long long g0b = rec(o)[2];
+        const unsigned long long g2a = rec(o - sy)[3];
+        const ulonglong2 g2b = *reinterpret_cast<const ulonglong2 *>(rec(o - sy) + 4);  // 4, 5
+        const unsigned long long g1 = rec(o - 1)[6];
+        const unsigned long long g3 = rec(o - sy - 1)[7];
+        const unsigned long long g5 = rec(o - sx - 1)[8];
+        const unsigned long long g6 = rec(o - sx - sy)[9];
+        const ulonglong2 g4 = *reinterpret_cast<const ulonglong2 *>(rec(o - sx) + 10);  // 10, 11
+        const unsigned long long q3 = CORR ? rec(o - 1)[4] : g2b.x;
         c[0] = g0a.x + g2a + q3 + g3;    // q 0, 1, 3, 2
         c[1] = g0a.y + g1 + g5 + g4.x;   // q 4, 5, 6, 7
         c[2] = g0b + g2b.y + g6 + g4.y;  // q 8, 11, 10, 9
@@ -1414,6 +1419,7 @@ template <bool UNIT>
 __global__ void k_from_f64(Geom g, MState S, int64_t at, int64_t n, const double *x, const double *y,
                            const double *z, const double *vx, const double *vy, const double *vz, const double *gam,
                            int rel, int vmode, float *g0, DevCounters *ctr) {
+    after_previous();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double pos[3] = {x[i], y[i], z[i]}, v[3] = {vx[i], vy[i], vz[i]};
         const double ga = gam ? gam[i] : 0.0;  // new_particle() leaves gamma at 0
@@ -1442,6 +1448,7 @@ __global__ void k_from_f64(Geom g, MState S, int64_t at, int64_t n, const double
 template <bool UNIT>
 __global__ void k_to_f64(Geom g, Div3 dv, MState S, int64_t at, int64_t n, double *x, double *y, double *z, double *vx,
                          double *vy, double *vz, double *gam, int rel, const float *g0) {
+    after_previous();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int64_t p = at + i;
         int32_t c = S.cell[p];
@@ -1471,14 +1478,17 @@ __global__ void k_to_f64(Geom g, Div3 dv, MState S, int64_t at, int64_t n, doubl
 }
 
 __global__ void k_d2f(const double *a, float *b, int64_t n) {
+    after_previous();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         b[i] = (float)a[i];
 }
 __global__ void k_f2d(const float *a, double *b, int64_t n) {
+    after_previous();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         b[i] = (double)a[i];
 }
 __global__ void k_fix2d(const long long *a, double *b, int64_t n, double q0) {
+    after_previous();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         b[i] = (double)a[i] * q0;
 }
@@ -1487,6 +1497,7 @@ __global__ void k_d2fix(const double *a, long long *b, int64_t n, double iq0) {
         b[i] = __double2ll_rn(a[i] * iq0);
 }
 __global__ void k_fillf(float *a, int64_t n, float v) {
+    after_previous();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         a[i] = v;
 }
@@ -1498,6 +1509,7 @@ struct MJ3 {
 };
 
 __global__ void k_yee_e_m(MGeom g, MF3 E, MCF3 T, MJ3 J, float dt, float q0) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int i = blockIdx.z + 1;
@@ -1511,6 +1523,7 @@ __global__ void k_yee_e_m(MGeom g, MF3 E, MCF3 T, MJ3 J, float dt, float q0) {
 }
 
 __global__ void k_yee_b_m(MGeom g, MF3 B, MCF3 T, MCF3 E, float dt) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int i = blockIdx.z + 1;
@@ -1523,6 +1536,7 @@ __global__ void k_yee_b_m(MGeom g, MF3 B, MCF3 T, MCF3 E, float dt) {
 }
 
 __global__ void k_yee_es_m(MGeom g, MF3 E, MJ3 J, float dt, float q0) {
+    after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
     int i = blockIdx.z + 1;
@@ -1539,6 +1553,7 @@ struct MList6 {
 // Periodic ghost fill over the physical transverse range (same scheme as the
 // FP64 k_ghost): all copies read physical points, any dims run at once.
 __global__ void k_ghost_m(MGeom g, MList6 fl, int dims_mask) {
+    after_previous();
     int z = blockIdx.z;
     int r = z & 1;
     int d = (z >> 1) % 3;
@@ -1562,6 +1577,7 @@ __global__ void k_ghost_m(MGeom g, MList6 fl, int dims_mask) {
 // Periodic fold of one dimension on the fixed-point accumulators (exact
 // integer adds); the folded ghost plane is left as the reference leaves it.
 __global__ void k_fold_m(MGeom g, int d, long long *f0, long long *f1, long long *f2) {
+    after_previous();
     int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
     int q = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int p = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -1584,6 +1600,7 @@ __global__ void k_fold_m(MGeom g, int d, long long *f0, long long *f1, long long
 // blockIdx.z.
 
 __global__ void k_fold_full_m(MGeom g, MFix4 fl, int d, int t1, int t2) {
+    after_previous();
     const int q = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y * blockDim.y + threadIdx.y;
     if (q >= t2 || r >= t1) return;
     const int o1 = (d == 0) ? 1 : 0, o2 = (d == 2) ? 1 : 2;
@@ -1621,6 +1638,7 @@ __device__ __forceinline__ float b_half(const MGeom &g, const MCF3 &T, const MF3
 // own threads).
 __global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, Slabs S, int planes, int update, int all,
                                                    MF3 E, MF3 B, MF3 T, float dt) {
+    after_previous();
     const MCF3 Tc = {{T.p[0], T.p[1], T.p[2]}};
     int c[3], of[3];
     if ((int)blockIdx.z < planes) {
@@ -1681,6 +1699,7 @@ struct MPlaneList {
 };
 
 __global__ void k_plane_m(MGeom g, MPlaneList pl, int tot0, int tot1, int tot2) {
+    after_previous();
     int e = blockIdx.z;
     if (e >= pl.n) return;
     const MPlane &ps = pl.s[e];
@@ -1710,6 +1729,7 @@ __global__ void k_plane_m(MGeom g, MPlaneList pl, int tot0, int tot1, int tot2) 
 constexpr int DIAG_CHUNK = 8;
 
 __global__ void k_moments_m(MSpecies st, MState S, int64_t np, int rel, const float *g0, double *part) {
+    after_previous();
     double acc[4] = {0, 0, 0, 0};
     float f[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     int k = 0;
@@ -1750,6 +1770,7 @@ __global__ void k_moments_m(MSpecies st, MState S, int64_t np, int rel, const fl
 }
 
 __global__ void k_energy_m(MGeom g, MCF3 E, MCF3 B, double hv, double *part) {
+    after_previous();
     double acc[6] = {0, 0, 0, 0, 0, 0};
     int64_t nphys = (int64_t)g.n[0] * g.n[1] * g.n[2];
     float f[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
@@ -2325,10 +2346,10 @@ static void from_f64(emoo_handle *h, int64_t at, int64_t n, const double *x, con
     const int rel = h->info.relativity != 0;
     h->launches++;
     if (h->g.unit)
-        k_from_f64<true><<<nblk(n), 256, 0, h->stream>>>(h->g, mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel, vmode,
+        launch_after(k_from_f64<true>, nblk(n), 256, 0, h->stream)(h->g, mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel, vmode,
                                                          h->g0, h->ctr);
     else
-        k_from_f64<false><<<nblk(n), 256, 0, h->stream>>>(h->g, mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel, vmode,
+        launch_after(k_from_f64<false>, nblk(n), 256, 0, h->stream)(h->g, mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel, vmode,
                                                           h->g0, h->ctr);
 }
 
@@ -2337,10 +2358,10 @@ static void to_f64(emoo_handle *h, int64_t at, int64_t n, double *x, double *y, 
     const int rel = h->info.relativity != 0;
     h->launches++;
     if (h->g.unit)
-        k_to_f64<true><<<nblk(n), 256, 0, h->stream>>>(h->g, div3(h), mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel,
+        launch_after(k_to_f64<true>, nblk(n), 256, 0, h->stream)(h->g, div3(h), mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel,
                                                        g0);
     else
-        k_to_f64<false><<<nblk(n), 256, 0, h->stream>>>(h->g, div3(h), mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel,
+        launch_after(k_to_f64<false>, nblk(n), 256, 0, h->stream)(h->g, div3(h), mstate(h), at, n, x, y, z, vx, vy, vz, gam, rel,
                                                         g0);
 }
 
@@ -2435,7 +2456,7 @@ int mixed_ghost_fill(emoo_handle *h) {
         if (!mask) return EMOO_OK;
         dim3 grd((tb + 31) / 32, (ta + 7) / 8, 36);
         h->launches++;
-        k_ghost_m<<<grd, blk, 0, h->stream>>>(mg, fl, mask);
+        launch_after(k_ghost_m, grd, blk, 0, h->stream)(mg, fl, mask);
         mask = 0;
         EMOO_CUDA(cudaGetLastError());
         return EMOO_OK;
@@ -2472,7 +2493,7 @@ int mixed_plane_sets(emoo_handle *h, const PlaneSet *ps, int n) {
     dim3 blk(32, 8);
     dim3 grd((m + 31) / 32, (m + 7) / 8, n);
     h->launches++;
-    k_plane_m<<<grd, blk, 0, h->stream>>>(mg, pl, g.tot[0], g.tot[1], g.tot[2]);
+    launch_after(k_plane_m, grd, blk, 0, h->stream)(mg, pl, g.tot[0], g.tot[1], g.tot[2]);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -2481,6 +2502,7 @@ int mixed_plane_sets(emoo_handle *h, const PlaneSet *ps, int n) {
 // the current a reflected particle deposited beyond its wall goes to the
 // mirrored points inside, normal component negated; ghost values cleared.
 __global__ void k_mirror_fold_m(MGeom g, MFix4 fl, int d, int right, int t1, int t2) {
+    after_previous();
     const int q = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y * blockDim.y + threadIdx.y;
     if (q >= t2 || r >= t1) return;
     const int a = blockIdx.z;
@@ -2522,13 +2544,13 @@ static int mixed_fold_full(emoo_handle *h, int what) {
                 if (h->bc.pbc[2 * d + r] != PBC_REFLECTING) continue;
                 dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, 3);
                 h->launches++;
-                k_mirror_fold_m<<<grd, blk, 0, h->stream>>>(mg, fl, d, r, g.tot[o1], g.tot[o2]);
+                launch_after(k_mirror_fold_m, grd, blk, 0, h->stream)(mg, fl, d, r, g.tot[o1], g.tot[o2]);
             }
             continue;
         }
         dim3 grd((g.tot[o2] + 31) / 32, (g.tot[o1] + 7) / 8, n);
         h->launches++;
-        k_fold_full_m<<<grd, blk, 0, h->stream>>>(mg, fl, d, g.tot[o1], g.tot[o2]);
+        launch_after(k_fold_full_m, grd, blk, 0, h->stream)(mg, fl, d, g.tot[o1], g.tot[o2]);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -2583,7 +2605,7 @@ static int mixed_b_ghost(emoo_handle *h, double dtp, bool all, bool update) {
     const dim3 grd((mg.n[2] + 31) / 32, (mg.n[1] + 7) / 8, 1);
     const int64_t ghosts = slab_size(S);
     launch_with_edges(h, grd, update ? mg.n[0] : 0, ghosts, [&](dim3 grid, int planes) {
-        k_b_ghost_m<<<grid, blk, 0, h->stream>>>(mg, S, planes, update, all, E, B, T, (float)dtp);
+        launch_after(k_b_ghost_m, grid, blk, 0, h->stream)(mg, S, planes, update, all, E, B, T, (float)dtp);
     });
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -2612,7 +2634,7 @@ static int mixed_fold(emoo_handle *h, int what) {
         dim3 blk(32, 8);
         dim3 grd((g.n[o2] + 31) / 32, (g.n[o1] + 7) / 8, nz);
         h->launches++;
-        k_fold_m<<<grd, blk, 0, h->stream>>>(mg, d, a, b, r);
+        launch_after(k_fold_m, grd, blk, 0, h->stream)(mg, d, a, b, r);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -2711,8 +2733,8 @@ static int mixed_fused(emoo_handle *h, double dtp, int mode, bool push = true, b
         const int what = mode == DEP_J ? 1 : mode == DEP_RHO ? 2 : 3, gam = rel && !first ? 1 : 0;
         const unsigned db = (unsigned)((h->np + 255) / 256);
         h->launches++;
-        if (corr) k_deposit_m<true><<<db, 256, 0, h->stream>>>(mg, dv, st, S, h->np, D, what, gam);
-        else k_deposit_m<false><<<db, 256, 0, h->stream>>>(mg, dv, st, S, h->np, D, what, gam);
+        if (corr) launch_after(k_deposit_m<true>, db, 256, 0, h->stream)(mg, dv, st, S, h->np, D, what, gam);
+        else launch_after(k_deposit_m<false>, db, 256, 0, h->stream)(mg, dv, st, S, h->np, D, what, gam);
         EMOO_CUDA(cudaGetLastError());
         return mixed_finish_deposit(h, mode);
     }
@@ -2722,16 +2744,16 @@ static int mixed_fused(emoo_handle *h, double dtp, int mode, bool push = true, b
         dim3 pg((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
         h->launches++;
         uint4 *zero = reinterpret_cast<uint4 *>(h->mf->wj);
-        if (corr) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, zero);
-        else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, zero);
+        if (corr) launch_after(k_pack_m<true>, pg, blk, 0, h->stream)(mg, P, h->mf->pack, zero);
+        else launch_after(k_pack_m<false>, pg, blk, 0, h->stream)(mg, P, h->mf->pack, zero);
         EMOO_CUDA(cudaGetLastError());
     }
     h->launches++;
     if (h->prof_on) EMOO_CUDA(cudaEventRecord(h->prof_ev[0], h->stream));
 #define EMOO_FUSED_M(R, F, C)                                                                                   \
-    k_fused_m<R, F, C><<<grd, FUSED_BLOCK, 0, h->stream>>>(mg, dv, st, h->bc, pk, S, h->np, D, g0, h->ctr, nullptr, 0)
+    launch_after(k_fused_m<R, F, C>, grd, FUSED_BLOCK, 0, h->stream)(mg, dv, st, h->bc, pk, S, h->np, D, g0, h->ctr, nullptr, 0)
 #define EMOO_FUSED_HOST(R, C)                                                                                      \
-    k_fused_m<R, false, C, true><<<grd, FUSED_BLOCK, 0, h->stream>>>(mg, dv, st, h->bc, pk, S, h->np, D, g0, h->ctr, \
+    launch_after(k_fused_m<R, false, C, true>, grd, FUSED_BLOCK, 0, h->stream)(mg, dv, st, h->bc, pk, S, h->np, D, g0, h->ctr, \
                                                                      h->mhost, store_pre)
     if (host) {  // the host-resident step: after the first push, J only
         if (corr) {
@@ -2786,12 +2808,12 @@ static int mixed_step_fields(emoo_handle *h, double dtp, int fold_what) {
             S.rest[d] = g.tot[d] - S.listed[d];
         }
         launch_with_edges(h, all, g.tot[0], slab_size(S), [&](dim3 grid, int planes) {
-            k_current_e_m<true><<<grid, blk, 0, h->stream>>>(mg, f, h->mf->wj, J, E, T, (float)dtp, (float)h->mf->q0, es,
+            launch_after(k_current_e_m<true>, grid, blk, 0, h->stream)(mg, f, h->mf->wj, J, E, T, (float)dtp, (float)h->mf->q0, es,
                                                              g.tot[1], g.tot[2], S, planes);
         });
     } else {
         h->launches++;
-        k_current_e_m<false><<<all, blk, 0, h->stream>>>(mg, f, h->mf->wj, J, E, T, (float)dtp, (float)h->mf->q0, es,
+        launch_after(k_current_e_m<false>, all, blk, 0, h->stream)(mg, f, h->mf->wj, J, E, T, (float)dtp, (float)h->mf->q0, es,
                                                          g.tot[1], g.tot[2], S, g.tot[0]);
     }
     EMOO_CUDA(cudaGetLastError());
@@ -2807,7 +2829,7 @@ static int mixed_step_fields(emoo_handle *h, double dtp, int fold_what) {
         MCF3 Ec = {{E.p[0], E.p[1], E.p[2]}};
         dim3 grd((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
         h->launches++;
-        k_yee_b_m<<<grd, blk, 0, h->stream>>>(mg, B, T, Ec, (float)dtp);
+        launch_after(k_yee_b_m, grd, blk, 0, h->stream)(mg, B, T, Ec, (float)dtp);
         EMOO_CUDA(cudaGetLastError());
     }
     return mixed_ghost_fill(h);
@@ -2823,12 +2845,12 @@ int mixed_yee_public(emoo_handle *h, double dtp, int es) {
     MJ3 J = {{h->mf->J[0], h->mf->J[1], h->mf->J[2]}};
     if (es) {
         h->launches++;
-        k_yee_es_m<<<grd, blk, 0, h->stream>>>(mg, E, J, (float)dtp, (float)h->mf->q0);
+        launch_after(k_yee_es_m, grd, blk, 0, h->stream)(mg, E, J, (float)dtp, (float)h->mf->q0);
     } else {
         h->bswap ^= 1;  // the member-pointer swap of evolveFields
         MCF3 T = {{mt_role(h, 0), mt_role(h, 1), mt_role(h, 2)}};
         h->launches++;
-        k_yee_e_m<<<grd, blk, 0, h->stream>>>(mg, E, T, J, (float)dtp, (float)h->mf->q0);
+        launch_after(k_yee_e_m, grd, blk, 0, h->stream)(mg, E, T, J, (float)dtp, (float)h->mf->q0);
         // the B half reads E at plane n+1: refreshed first under the corrected
         // policy (time-centred at the periodic wrap, as yee_f64)
         if (h->policy == EMOO_POLICY_CORRECTED) {
@@ -2838,7 +2860,7 @@ int mixed_yee_public(emoo_handle *h, double dtp, int es) {
         MF3 B = {{mb_role(h, 0), mb_role(h, 1), mb_role(h, 2)}};
         MCF3 Ec = {{E.p[0], E.p[1], E.p[2]}};
         h->launches++;
-        k_yee_b_m<<<grd, blk, 0, h->stream>>>(mg, B, T, Ec, (float)dtp);
+        launch_after(k_yee_b_m, grd, blk, 0, h->stream)(mg, B, T, Ec, (float)dtp);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -2889,20 +2911,20 @@ int mixed_key_bits(emoo_handle *h) {
 // Field readback: FP32 storage or fixed point converted to FP64 in the slot.
 int mixed_get_field(emoo_handle *h, int id, double *out_dev) {
     int64_t n = h->g.npts;
-    if (id <= EMOO_EZ) k_f2d<<<nblk(n), 256, 0, h->stream>>>(h->mf->E[id], out_dev, n);
-    else if (id <= EMOO_BZ) k_f2d<<<nblk(n), 256, 0, h->stream>>>(h->mf->Bslot[id - EMOO_BX], out_dev, n);
-    else if (id <= EMOO_RHO) k_fix2d<<<nblk(n), 256, 0, h->stream>>>(h->mf->J[id - EMOO_JX], out_dev, n, h->mf->q0);
-    else if (id <= EMOO_BZ_TM1) k_f2d<<<nblk(n), 256, 0, h->stream>>>(h->mf->Bslot[3 + id - EMOO_BX_TM1], out_dev, n);
+    if (id <= EMOO_EZ) launch_after(k_f2d, nblk(n), 256, 0, h->stream)(h->mf->E[id], out_dev, n);
+    else if (id <= EMOO_BZ) launch_after(k_f2d, nblk(n), 256, 0, h->stream)(h->mf->Bslot[id - EMOO_BX], out_dev, n);
+    else if (id <= EMOO_RHO) launch_after(k_fix2d, nblk(n), 256, 0, h->stream)(h->mf->J[id - EMOO_JX], out_dev, n, h->mf->q0);
+    else if (id <= EMOO_BZ_TM1) launch_after(k_f2d, nblk(n), 256, 0, h->stream)(h->mf->Bslot[3 + id - EMOO_BX_TM1], out_dev, n);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
 
 int mixed_set_field(emoo_handle *h, int id, const double *in_dev) {
     int64_t n = h->g.npts;
-    if (id <= EMOO_EZ) k_d2f<<<nblk(n), 256, 0, h->stream>>>(in_dev, h->mf->E[id], n);
-    else if (id <= EMOO_BZ) k_d2f<<<nblk(n), 256, 0, h->stream>>>(in_dev, h->mf->Bslot[id - EMOO_BX], n);
+    if (id <= EMOO_EZ) launch_after(k_d2f, nblk(n), 256, 0, h->stream)(in_dev, h->mf->E[id], n);
+    else if (id <= EMOO_BZ) launch_after(k_d2f, nblk(n), 256, 0, h->stream)(in_dev, h->mf->Bslot[id - EMOO_BX], n);
     else if (id <= EMOO_RHO) k_d2fix<<<nblk(n), 256, 0, h->stream>>>(in_dev, h->mf->J[id - EMOO_JX], n, 1.0 / h->mf->q0);
-    else if (id <= EMOO_BZ_TM1) k_d2f<<<nblk(n), 256, 0, h->stream>>>(in_dev, h->mf->Bslot[3 + id - EMOO_BX_TM1], n);
+    else if (id <= EMOO_BZ_TM1) launch_after(k_d2f, nblk(n), 256, 0, h->stream)(in_dev, h->mf->Bslot[3 + id - EMOO_BX_TM1], n);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -2913,7 +2935,7 @@ int mixed_set_field(emoo_handle *h, int id, const double *in_dev) {
 int mixed_deposit_to_f64(emoo_handle *h) {
     int64_t n = h->g.npts;
     for (int c = 0; c < 4; c++)
-        k_fix2d<<<nblk(n), 256, 0, h->stream>>>(h->mf->J[c], h->slot[EMOO_JX + c], n, h->mf->q0);
+        launch_after(k_fix2d, nblk(n), 256, 0, h->stream)(h->mf->J[c], h->slot[EMOO_JX + c], n, h->mf->q0);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -2923,11 +2945,11 @@ int mixed_fields_from_slots(emoo_handle *h) {
     int64_t n = h->g.npts;
     for (int c = 0; c < 3; c++) {
         h->launches++;
-        k_d2f<<<nblk(n), 256, 0, h->stream>>>(h->slot[EMOO_EX + c], h->mf->E[c], n);
+        launch_after(k_d2f, nblk(n), 256, 0, h->stream)(h->slot[EMOO_EX + c], h->mf->E[c], n);
         h->launches++;
-        k_d2f<<<nblk(n), 256, 0, h->stream>>>(h->slot[EMOO_BX + c], h->mf->Bslot[c], n);
+        launch_after(k_d2f, nblk(n), 256, 0, h->stream)(h->slot[EMOO_BX + c], h->mf->Bslot[c], n);
         h->launches++;
-        k_d2f<<<nblk(n), 256, 0, h->stream>>>(h->slot[EMOO_BX_TM1 + c], h->mf->Bslot[3 + c], n);
+        launch_after(k_d2f, nblk(n), 256, 0, h->stream)(h->slot[EMOO_BX_TM1 + c], h->mf->Bslot[3 + c], n);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -2937,11 +2959,11 @@ int mixed_const_fields(emoo_handle *h) {
     int64_t n = h->g.npts;
     for (int c = 0; c < 3; c++) {
         h->launches++;
-        k_fillf<<<nblk(n), 256, 0, h->stream>>>(h->mf->E[c], n, (float)h->info.E0[c]);
+        launch_after(k_fillf, nblk(n), 256, 0, h->stream)(h->mf->E[c], n, (float)h->info.E0[c]);
         h->launches++;
-        k_fillf<<<nblk(n), 256, 0, h->stream>>>(h->mf->Bslot[c], n, (float)h->info.B0[c]);
+        launch_after(k_fillf, nblk(n), 256, 0, h->stream)(h->mf->Bslot[c], n, (float)h->info.B0[c]);
         h->launches++;
-        k_fillf<<<nblk(n), 256, 0, h->stream>>>(h->mf->Bslot[3 + c], n, (float)h->info.B0[c]);
+        launch_after(k_fillf, nblk(n), 256, 0, h->stream)(h->mf->Bslot[3 + c], n, (float)h->info.B0[c]);
     }
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -2959,7 +2981,7 @@ int mixed_moments(emoo_handle *h, double out4[4]) {
     MSpecies st = mspecies(h, h->dtp);
     const float *g0 = (h->first_push && h->g0) ? h->g0 : nullptr;
     h->launches++;
-    k_moments_m<<<nb, 256, 0, h->stream>>>(st, mstate(h), h->np, h->info.relativity != 0, g0, h->red);
+    launch_after(k_moments_m, nb, 256, 0, h->stream)(st, mstate(h), h->np, h->info.relativity != 0, g0, h->red);
     EMOO_CUDA(cudaGetLastError());
     std::vector<double> part((size_t)nb * 4);
     EMOO_CUDA(cudaMemcpyAsync(part.data(), h->red, part.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -2981,7 +3003,7 @@ int mixed_field_energy(emoo_handle *h, double out6[6]) {
     MGeom mg = mgeom(h, h->dtp);
     MCF3 E = {{h->mf->E[0], h->mf->E[1], h->mf->E[2]}};
     MCF3 B = {{h->mf->Bslot[0], h->mf->Bslot[1], h->mf->Bslot[2]}};  // fixed slots, like the history
-    k_energy_m<<<nb, 256, 0, h->stream>>>(mg, E, B, 0.5 * g.vol, h->red);
+    launch_after(k_energy_m, nb, 256, 0, h->stream)(mg, E, B, 0.5 * g.vol, h->red);
     EMOO_CUDA(cudaGetLastError());
     std::vector<double> part((size_t)nb * 6);
     EMOO_CUDA(cudaMemcpyAsync(part.data(), h->red, part.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -3113,8 +3135,8 @@ int mixed_interpolate(emoo_handle *h) {
     dim3 blk(32, 8);
     dim3 pg((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
     h->launches += 2;
-    if (h->policy == EMOO_POLICY_CORRECTED) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, nullptr);
-    else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, nullptr);
+    if (h->policy == EMOO_POLICY_CORRECTED) launch_after(k_pack_m<true>, pg, blk, 0, h->stream)(mg, P, h->mf->pack, nullptr);
+    else launch_after(k_pack_m<false>, pg, blk, 0, h->stream)(mg, P, h->mf->pack, nullptr);
     if (h->np > 0)
         k_interpolate_m<<<nblk(h->np), 256, 0, h->stream>>>(h->mf->pack, mstate(h), h->np, h->cap, h->fcache);
     EMOO_CUDA(cudaGetLastError());
@@ -3191,8 +3213,8 @@ int mixed_ad_particles(emoo_handle *h, const MSnapView &S, const int32_t *cell_a
         dim3 blk(32, 8);
         dim3 pg((g.n[2] + 31) / 32, (g.n[1] + 7) / 8, g.n[0]);
         h->launches++;
-        if (h->policy == EMOO_POLICY_CORRECTED) k_pack_m<true><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, nullptr);
-        else k_pack_m<false><<<pg, blk, 0, h->stream>>>(mg, P, h->mf->pack, nullptr);
+        if (h->policy == EMOO_POLICY_CORRECTED) launch_after(k_pack_m<true>, pg, blk, 0, h->stream)(mg, P, h->mf->pack, nullptr);
+        else launch_after(k_pack_m<false>, pg, blk, 0, h->stream)(mg, P, h->mf->pack, nullptr);
         EMOO_CUDA(cudaGetLastError());
     }
     MSnapC SC{S.cell, {S.o[0], S.o[1], S.o[2]}, {S.u[0], S.u[1], S.u[2]}};

@@ -33,6 +33,7 @@ constexpr int RS_BINS9 = 512;  // 9-bit digits
 template <int BINS>
 __global__ void __launch_bounds__(RS_THREADS) k_hist(const uint32_t *keys, int64_t n, int shift, uint32_t mask,
                                                      uint32_t *hist, int nblocks) {
+    after_previous<false>();
     __shared__ uint32_t cnt[BINS];
     for (int d = threadIdx.x; d < BINS; d += RS_THREADS) cnt[d] = 0;
     __syncthreads();
@@ -58,6 +59,7 @@ template <int BINS>
 __global__ void __launch_bounds__(RS_THREADS, 5) k_scatter(const uint32_t *kin, const uint32_t *vin, uint32_t *kout,
                                                         uint32_t *vout, int64_t n, int shift, uint32_t mask,
                                                         const uint32_t *hist, int nblocks) {
+    after_previous<false>();
     static_assert(BINS % RS_THREADS == 0 && RS_TILE <= 65535, "digits per thread; 16-bit counts");
     constexpr int DPT = BINS / RS_THREADS;  // digits per thread
     __shared__ uint16_t wc[RS_THREADS / 32][BINS];
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(RS_THREADS, 5) k_scatter(const uint32_t *kin, 
 #pragma unroll
         for (int c = 0; c < RS_ITEMS; c++) {
             int64_t idx = base + c * 32 + lane;
-            key[c] = idx < n ? __ldg(kin + idx) : 0u;
+            key[c] = idx < n ? kin[idx] : 0u;
         }
 #pragma unroll
         for (int c = 0; c < RS_ITEMS; c++) {
@@ -136,11 +138,11 @@ __global__ void __launch_bounds__(RS_THREADS, 5) k_scatter(const uint32_t *kin, 
     for (int c = 0; c < RS_ITEMS; c++) {
         int64_t idx = base + c * 32 + lane;
         if (idx >= n) continue;
-        const uint32_t k = __ldg(kin + idx);  // read again (L2)
+        const uint32_t k = kin[idx];  // read again (L2)
         uint32_t dg = (k >> shift) & mask;
         uint32_t lp = s_start[dg] + wc[w][dg] + ((rank2[c >> 1] >> (16 * (c & 1))) & 0xffffu);
         s_key[lp] = k;
-        s_val[lp] = vin ? __ldg(vin + idx) : (uint32_t)idx;
+        s_val[lp] = vin ? vin[idx] : (uint32_t)idx;
     }
     __syncthreads();
     const int64_t tbase = (int64_t)blockIdx.x * RS_TILE;
@@ -156,6 +158,7 @@ __global__ void __launch_bounds__(RS_THREADS, 5) k_scatter(const uint32_t *kin, 
 
 // In-place exclusive scan of each RS_TILE-element tile; tile totals to sums.
 __global__ void __launch_bounds__(RS_THREADS) k_scan_tile(uint32_t *data, int64_t m, uint32_t *sums) {
+    after_previous();
     __shared__ uint32_t wsum[RS_THREADS / 32];
     int64_t base = (int64_t)blockIdx.x * RS_TILE + (int64_t)threadIdx.x * RS_ITEMS;
     uint32_t v[RS_ITEMS];
@@ -189,6 +192,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_scan_tile(uint32_t *data, int64_
 }
 
 __global__ void k_scan_add(uint32_t *data, int64_t m, const uint32_t *sums) {
+    after_previous();
     int64_t base = (int64_t)blockIdx.x * RS_TILE;
     uint32_t a = sums[blockIdx.x];
     for (int i = threadIdx.x; i < RS_TILE; i += blockDim.x) {
@@ -210,15 +214,15 @@ int scan_excl(emoo_handle *h, uint32_t *data, int64_t m, uint32_t *tmp) {
     int64_t t = tiles(m);
     if (t <= 1) {
         h->launches++;
-        k_scan_tile<<<1, RS_THREADS, 0, h->stream>>>(data, m, nullptr);
+        launch_after(k_scan_tile, 1, RS_THREADS, 0, h->stream)(data, m, nullptr);
         EMOO_CUDA(cudaGetLastError());
         return EMOO_OK;
     }
     h->launches++;
-    k_scan_tile<<<(unsigned)t, RS_THREADS, 0, h->stream>>>(data, m, tmp);
+    launch_after(k_scan_tile, (unsigned)t, RS_THREADS, 0, h->stream)(data, m, tmp);
     EMOO_TRY(scan_excl(h, tmp, t, tmp + t));
     h->launches++;
-    k_scan_add<<<(unsigned)t, RS_THREADS, 0, h->stream>>>(data, m, tmp);
+    launch_after(k_scan_add, (unsigned)t, RS_THREADS, 0, h->stream)(data, m, tmp);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -227,12 +231,13 @@ int scan_excl(emoo_handle *h, uint32_t *data, int64_t m, uint32_t *tmp) {
 // (one 16-byte permutation load, 4 independent loads in flight, vector
 // stores); the < 4 items of the tail go one by one.
 template <typename T>
-__global__ void k_gather(const T *__restrict__ src, T *__restrict__ dst, const uint32_t *__restrict__ perm, int64_t n) {
+__global__ void k_gather(const T *src, T *__restrict__ dst, const uint32_t *perm, int64_t n) {
+    after_previous<false>();
     static_assert(sizeof(T) == 4 || sizeof(T) == 8, "payload element size");
     const int64_t n4 = n >> 2;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n4; j += stride) {
-        const uint4 pp = __ldg(reinterpret_cast<const uint4 *>(perm) + j);
+        const uint4 pp = reinterpret_cast<const uint4 *>(perm)[j];
         const T a = src[pp.x], b = src[pp.y], c = src[pp.z], d = src[pp.w];
         T *o = dst + 4 * j;
         if constexpr (sizeof(T) == 4) {
@@ -268,7 +273,7 @@ int gather_one(emoo_handle *h, T *&arr, const uint32_t *perm, int64_t n) {
     // 20 steps: 26.9 ms at four blocks per SM, 32.9 ms at sixteen, 34.3 ms at one).
     int nb = (int)std::min<int64_t>((n / 4 + 255) / 256, 152 * 4);
     h->launches++;
-    k_gather<T><<<std::max(nb, 1), 256, 0, h->stream>>>(arr, tmp, perm, n);  // base pointers are cudaMalloc'd
+    launch_after(k_gather<T>, std::max(nb, 1), 256, 0, h->stream)(arr, tmp, perm, n);  // base pointers are cudaMalloc'd
     EMOO_CUDA(cudaGetLastError());
     scratch = (void *)arr;
     arr = tmp;
@@ -276,6 +281,7 @@ int gather_one(emoo_handle *h, T *&arr, const uint32_t *perm, int64_t n) {
 }
 
 __global__ void k_species_bounds(const uint32_t *keys, int64_t n, int nspec, int64_t ncell, int64_t *bounds) {
+    after_previous();
     int s = threadIdx.x;
     if (s > nspec) return;
     uint64_t target = (uint64_t)s * (uint64_t)ncell;
@@ -322,18 +328,18 @@ int radix_sort_perm(emoo_handle *h, int64_t n, int key_bits) {
         const uint32_t *vin = ps == 0 ? nullptr : h->perm[cur];
         h->launches++;
         if (bits > 8)
-            k_hist<RS_BINS9><<<nblocks, RS_THREADS, 0, h->stream>>>(h->key[cur], n, shift, mask, h->hist, nblocks);
+            launch_after(k_hist<RS_BINS9>, nblocks, RS_THREADS, 0, h->stream)(h->key[cur], n, shift, mask, h->hist, nblocks);
         else
-            k_hist<RS_BINS><<<nblocks, RS_THREADS, 0, h->stream>>>(h->key[cur], n, shift, mask, h->hist, nblocks);
+            launch_after(k_hist<RS_BINS>, nblocks, RS_THREADS, 0, h->stream)(h->key[cur], n, shift, mask, h->hist, nblocks);
         EMOO_CUDA(cudaGetLastError());
         EMOO_TRY(scan_excl(h, h->hist, nh, h->scan_tmp));
         h->launches++;
         if (bits > 8)
-            k_scatter<RS_BINS9><<<nblocks, RS_THREADS, 0, h->stream>>>(h->key[cur], vin, h->key[cur ^ 1],
+            launch_after(k_scatter<RS_BINS9>, nblocks, RS_THREADS, 0, h->stream)(h->key[cur], vin, h->key[cur ^ 1],
                                                                        h->perm[cur ^ 1], n, shift, mask, h->hist,
                                                                        nblocks);
         else
-            k_scatter<RS_BINS><<<nblocks, RS_THREADS, 0, h->stream>>>(h->key[cur], vin, h->key[cur ^ 1],
+            launch_after(k_scatter<RS_BINS>, nblocks, RS_THREADS, 0, h->stream)(h->key[cur], vin, h->key[cur ^ 1],
                                                                       h->perm[cur ^ 1], n, shift, mask, h->hist,
                                                                       nblocks);
         EMOO_CUDA(cudaGetLastError());
@@ -351,8 +357,9 @@ int radix_sort_perm(emoo_handle *h, int64_t n, int key_bits) {
 // The mixed form's sorted cells straight from the sorted keys (species *
 // npts + cell; removed particles carry keys from live_end on): a streaming
 // pass in place of a gather through the permutation.
-__global__ void k_cells_from_keys(const uint32_t *__restrict__ key, int64_t n, uint32_t npts, uint32_t live_end,
+__global__ void k_cells_from_keys(const uint32_t *key, int64_t n, uint32_t npts, uint32_t live_end,
                                   int32_t *__restrict__ cell) {
+    after_previous();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += stride) {
         const uint32_t k = key[j];
@@ -374,7 +381,7 @@ int gather_payload(emoo_handle *h, int64_t n, bool cells_from_keys) {
         // the sort keys of mixed_sort_keys: the cell is the key modulo npts
         int nb = (int)std::min<int64_t>((n + 255) / 256, 152 * 16);
         h->launches++;
-        k_cells_from_keys<<<std::max(nb, 1), 256, 0, h->stream>>>(
+        launch_after(k_cells_from_keys, std::max(nb, 1), 256, 0, h->stream)(
             h->key[0], n, (uint32_t)h->g.npts, (uint32_t)((int64_t)h->nspec * h->g.npts), h->cell);
         EMOO_CUDA(cudaGetLastError());
     } else {
@@ -398,7 +405,7 @@ int gather_payload(emoo_handle *h, int64_t n, bool cells_from_keys) {
 int count_species(emoo_handle *h, int64_t n, int64_t stride, int64_t *counts_host) {
     if (!h->d_spec_count) EMOO_CUDA(cudaMalloc(&h->d_spec_count, sizeof(int64_t) * (EMOO_NSPEC + 1)));
     h->launches++;
-    k_species_bounds<<<1, 64, 0, h->stream>>>(h->key[0], n, h->nspec, stride, h->d_spec_count);
+    launch_after(k_species_bounds, 1, 64, 0, h->stream)(h->key[0], n, h->nspec, stride, h->d_spec_count);
     EMOO_CUDA(cudaGetLastError());
     int64_t b[EMOO_NSPEC + 1];
     EMOO_CUDA(cudaMemcpyAsync(b, h->d_spec_count, sizeof(int64_t) * (h->nspec + 1), cudaMemcpyDeviceToHost, h->stream));
@@ -466,13 +473,13 @@ int noalloc_scratch(NoAllocScratch **out) {
 int noalloc_scan(cudaStream_t s, uint32_t *data, int64_t m, uint32_t *tmp) {
     int64_t t = tiles(m);
     if (t <= 1) {
-        k_scan_tile<<<1, RS_THREADS, 0, s>>>(data, m, nullptr);
+        launch_after(k_scan_tile, 1, RS_THREADS, 0, s)(data, m, nullptr);
         EMOO_CUDA(cudaGetLastError());
         return EMOO_OK;
     }
-    k_scan_tile<<<(unsigned)t, RS_THREADS, 0, s>>>(data, m, tmp);
+    launch_after(k_scan_tile, (unsigned)t, RS_THREADS, 0, s)(data, m, tmp);
     EMOO_TRY(noalloc_scan(s, tmp, t, tmp + t));
-    k_scan_add<<<(unsigned)t, RS_THREADS, 0, s>>>(data, m, tmp);
+    launch_after(k_scan_add, (unsigned)t, RS_THREADS, 0, s)(data, m, tmp);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -509,10 +516,10 @@ extern "C" int emoo_sort_permutation_noalloc(const uint32_t *keys, int64_t n, in
         uint32_t *kout = last ? nullptr : sc->key[ps & 1];
         // alternate so that the last pass lands in the caller's array
         uint32_t *vout = ((passes - 1 - ps) % 2 == 0) ? perm : scr_perm;
-        k_hist<RS_BINS><<<nblocks, RS_THREADS, 0, s>>>(kin, n, shift, mask, sc->hist, nblocks);
+        launch_after(k_hist<RS_BINS>, nblocks, RS_THREADS, 0, s)(kin, n, shift, mask, sc->hist, nblocks);
         EMOO_CUDA(cudaGetLastError());
         EMOO_TRY(noalloc_scan(s, sc->hist, nhist, sc->scan));
-        k_scatter<RS_BINS><<<nblocks, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, shift, mask, sc->hist, nblocks);
+        launch_after(k_scatter<RS_BINS>, nblocks, RS_THREADS, 0, s)(kin, vin, kout, vout, n, shift, mask, sc->hist, nblocks);
         EMOO_CUDA(cudaGetLastError());
         kin = kout;
         vin = vout;
