@@ -72,17 +72,19 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // launch). Data that those kernels write is not read through the read-only path
 // (__ldg, const __restrict__) at an address known beforehand: such loads may be
 // moved above the wait. About 2 us a launch where kernels are short: 20 steps
-// on 8^3 cells 921 -> 666 us, V-cycles on 128 x 64 x 64 5.26 -> 4.94 ms, the
+// on 8^3 cells 921 -> 647 us, V-cycles on 128 x 64 x 64 4.9 -> 4.7 ms, the
 // gradient of a 32^3 laser run 25.7 -> 24.0 ms.
 //
-// EARLY: the next launch's first blocks may also wait on the SMs that this
-// kernel's last blocks leave free. Not for the particle kernels and the sort:
-// their shared memory would leave the waiting kernel its small L1 (a laser
-// between walls, 20 steps: 3967 us, 3625 us without).
+// EARLY: once its own wait is over, the next launch's first blocks may wait on
+// the SMs that this kernel's last blocks leave free (allowed before the wait,
+// several kernels queue up there: a thousand half-sweeps on 49 x 31 x 27 points
+// took 61 ms instead of 43). Not for the particle kernels and the sort: their
+// shared memory would leave the waiting kernel its small L1 (a laser between
+// walls, 20 steps: 3967 us, 3625 us without).
 template <bool EARLY = true>
 __device__ __forceinline__ void after_previous() {
-    if (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 template <class... P>
