@@ -108,11 +108,24 @@ __device__ __forceinline__ R nb_sum(const Lv &L, const C *c, const R *u, int i, 
            c[2] * (u[lidx(L, i, j, wrap_dn(L, 2, k))] + u[lidx(L, i, j, wrap_up(L, 2, k))]);
 }
 
+// What a level's u takes with a new right side f, by who reads it next: nothing
+// (tiles that begin with f, the tail), zero, or the first half-sweep from zero,
+// which needs no neighbours (red points, or all of the Jacobi partner w).
+enum { START_NONE, START_ZERO, START_SWEPT };
+
+__device__ __forceinline__ void start_level(const Lv &L, int start, int64_t o, int parity, float f) {
+    if (start == START_ZERO) L.u[o] = 0.0f;
+    if (start != START_SWEPT) return;
+    const float v = (0.0f - f) * L.idiag;
+    if (L.rb) L.u[o] = parity ? 0.0f : v;
+    else L.w[o] = OMEGA * v;
+}
+
 // The FP64 residual of the fine problem: level 0's right side takes it (as
-// FP32), level 0's correction restarts at zero, and *dmax the maximum |r|,
+// FP32), level 0's correction restarts, and *dmax the maximum |r|,
 // taken over the FP32 values (the stop test needs no more): this kernel runs
 // on the FP64 pipe, so everything after the residual itself stays off it.
-__global__ void k_mg_residual64(Lv L, Fine F, double *dmax) {
+__global__ void k_mg_residual64(Lv L, Fine F, double *dmax, int start) {
     after_previous();
     __shared__ float sh[8];
     const int k = L.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
@@ -123,7 +136,7 @@ __global__ void k_mg_residual64(Lv L, Fine F, double *dmax) {
         const int64_t o = lidx(L, i, j, k);
         const float r = f64_to_f32(F.f[o] - (nb_sum(L, F.c, F.u, i, j, k) - F.diag * F.u[o]));
         L.f[o] = r;
-        L.u[o] = 0.0f;
+        start_level(L, start, o, (i + j + k) & 1, r);
         a = fabsf(r);
     }
     for (int off = 16; off > 0; off >>= 1) a = fmaxf(a, __shfl_down_sync(0xffffffffu, a, off));
@@ -166,19 +179,17 @@ __device__ __forceinline__ float restrict_sum(const int *crs, const float *r, co
     return s;
 }
 
-// the same on a whole level, where the neighbour below may be found by
-// wrapping; coarse f takes it and coarse u restarts at zero
+// the same on a whole level, at a coarse point, where the neighbour below may be
+// found by wrapping
 template <class LV>
-__device__ __forceinline__ void restrict_point(const LV &F, const float *r, const LV &Cl, int I, int J, int K) {
+__device__ __forceinline__ float restrict_value(const LV &F, const float *r, int I, int J, int K) {
     using S = decltype(F.sx + F.sy);
     const int at[3] = {F.crs[0] ? 2 * I - 1 : I, F.crs[1] ? 2 * J - 1 : J, F.crs[2] ? 2 * K - 1 : K};
     const S up[3] = {F.sx, F.sy, 1};
     S dn[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) dn[d] = F.per[d] && at[d] == 1 ? (F.P[d] - 1) * up[d] : -up[d];
-    const auto o = lidx(Cl, I, J, K);
-    Cl.f[o] = restrict_sum(F.crs, r + lidx(F, at[0], at[1], at[2]), dn, up);
-    Cl.u[o] = 0.0f;
+    return restrict_sum(F.crs, r + lidx(F, at[0], at[1], at[2]), dn, up);
 }
 
 // coarse index pair and weight of the second feeding fine index f of a
@@ -257,13 +268,16 @@ __global__ void k_mg_residual(Lv L) {
     L.w[o] = L.f[o] - (nb_sum(L, L.c, L.u, i, j, k) - L.diag * L.u[o]);
 }
 
-__global__ void k_mg_restrict(Lv F, Lv Cl) {
+__global__ void k_mg_restrict(Lv F, Lv Cl, int start) {
     after_previous();
     const int K = Cl.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int J = Cl.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int I = Cl.lo[0] + blockIdx.z;
     if (K > Cl.hi[2] || J > Cl.hi[1] || I > Cl.hi[0]) return;
-    restrict_point(F, F.w, Cl, I, J, K);
+    const int64_t o = lidx(Cl, I, J, K);
+    const float f = restrict_value(F, F.w, I, J, K);
+    Cl.f[o] = f;
+    start_level(Cl, start, o, (I + J + K) & 1, f);
 }
 
 __global__ void k_mg_prolong(Lv Cl, Lv F) {
@@ -275,15 +289,23 @@ __global__ void k_mg_prolong(Lv Cl, Lv F) {
     F.u[lidx(F, i, j, k)] += prolong_value(Cl, F, i, j, k);
 }
 
-// u += e at the unknowns (e: level 0's correction)
-__global__ void k_mg_correct(Lv L, Fine F) {
+// The last half-sweep of level 0 (black points, or the Jacobi step from w), its
+// finished correction added to the solution.
+__global__ void k_mg_finish(Lv L, Fine F) {
     after_previous();
     const int k = L.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = L.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
     const int i = L.lo[0] + blockIdx.z;
     if (k > L.hi[2] || j > L.hi[1] || i > L.hi[0]) return;
     const int64_t o = lidx(L, i, j, k);
-    F.u[o] += f64_of_f32(L.u[o]);
+    float e;
+    if (L.rb) {
+        e = (i + j + k) & 1 ? (nb_sum(L, L.c, L.u, i, j, k) - L.f[o]) * L.idiag : L.u[o];
+    } else {
+        const float x = L.w[o];
+        e = x + OMEGA * ((nb_sum(L, L.c, L.w, i, j, k) - L.f[o]) * L.idiag - x);
+    }
+    F.u[o] += f64_of_f32(e);
 }
 
 // ---- smaller levels above the tail, in tiles
@@ -318,7 +340,7 @@ struct TileLeg {
     const float *src;  // u in (UP, SWEEP)
     float *dst;        // u out
     double *sol;       // not null: the FP64 solution takes it instead (level 0's last leg)
-    int zero;          // DOWN: the next level starts from its u, set it to zero
+    int start;         // DOWN: of the next level
 };
 
 __host__ __device__ __forceinline__ int tile_sy(int e2) { return e2 | 1; }
@@ -556,8 +578,9 @@ __global__ void __launch_bounds__(TILE_THREADS, 1) k_mg_tile(const __grid_consta
         const float *r = f + ((L.crs[0] ? 2 * i - 1 : i) - b0[0]) * sx + ((L.crs[1] ? 2 * j - 1 : j) - b0[1]) * sy +
                          (L.crs[2] ? 2 * k - 1 : k) - b0[2];
         const int64_t o = lidx(C, i, j, k);
-        C.f[o] = restrict_sum(L.crs, r, dn, up);
-        if (G.zero) C.u[o] = 0.0f;
+        const float v = restrict_sum(L.crs, r, dn, up);
+        C.f[o] = v;
+        start_level(C, G.start, o, (i + j + k) & 1, v);
     }
 }
 
@@ -698,7 +721,8 @@ __device__ void tail_down(const Tail &T, int l, float *sm) {
     G::sync();
     for (int t = G::rank(); t < T.lv[l + 1].n; t += G::size()) {
         const uint4 q = __ldg(T.pts + T.lv[l + 1].pts + t);
-        restrict_point(L, L.r, C, q.y, q.z, q.w);
+        C.f[q.x & 0xffffu] = restrict_value(L, L.r, q.y, q.z, q.w);
+        C.u[q.x & 0xffffu] = 0.0f;
     }
     G::sync();
 }
@@ -955,23 +979,27 @@ Tail make_tail(const MgState *s, size_t l, std::vector<uint4> *pts = nullptr) {
     return T;
 }
 
-void smooth(emoo_handle *h, const Lv &L, int sweeps, int &launches) {
+// `sweeps` sweeps of a level a kernel a half-sweep, without the first `skip`
+// half-sweeps (done where the right side was formed) and, with `sol`, the last
+// adding the correction to it.
+void smooth(emoo_handle *h, const Lv &L, int sweeps, int skip, const Fine *sol, int &launches) {
     dim3 blk(32, 8);
-    if (!L.rb) {
-        for (int s = 0; s < sweeps; s++) {
-            launches += 2;
-            launch_after(k_mg_jacobi, pts_grid(L, blk), blk, 0, h->stream)(L, L.u, L.w);
-            launch_after(k_mg_jacobi, pts_grid(L, blk), blk, 0, h->stream)(L, L.w, L.u);
-        }
-        return;
-    }
     const int m2 = L.hi[2] - L.lo[2] + 1;
-    dim3 grd(((m2 + 1) / 2 + blk.x - 1) / blk.x, (L.hi[1] - L.lo[1] + 1 + blk.y - 1) / blk.y, L.hi[0] - L.lo[0] + 1);
-    for (int s = 0; s < sweeps; s++)
-        for (int c = 0; c < 2; c++) {
-            launches++;
-            launch_after(k_mg_smooth, grd, blk, 0, h->stream)(L, c);
-        }
+    const dim3 half(((m2 + 1) / 2 + blk.x - 1) / blk.x, (L.hi[1] - L.lo[1] + 1 + blk.y - 1) / blk.y, L.hi[0] - L.lo[0] + 1);
+    for (int s = skip; s < 2 * sweeps; s++) {
+        launches++;
+        if (sol && s + 1 == 2 * sweeps) launch_after(k_mg_finish, pts_grid(L, blk), blk, 0, h->stream)(L, *sol);
+        else if (L.rb) launch_after(k_mg_smooth, half, blk, 0, h->stream)(L, s & 1);
+        else launch_after(k_mg_jacobi, pts_grid(L, blk), blk, 0, h->stream)(L, s & 1 ? L.w : L.u, s & 1 ? L.u : L.w);
+    }
+}
+
+// How level l starts from a new right side.
+int level_start(const MgState *s, size_t l) {
+    if (l == s->tail_from) return START_NONE;
+    const bool coarsest = l + 1 == s->lv.size();
+    if (tile_size(s->lv[l], coarsest)) return coarsest ? START_ZERO : START_NONE;
+    return START_SWEPT;
 }
 
 // One V-cycle from level l; returns where the level's correction is (level 0's
@@ -997,27 +1025,25 @@ const float *vcycle(emoo_handle *h, MgState *s, size_t l, int &launches) {
     }
     if (tiles) {
         Lv C = s->lv[l + 1];
-        const int zero = l + 1 != s->tail_from && (l + 2 == s->lv.size() || !tile_size(C, false));
-        tile_leg(h, DOWN, L, C, {0, nullptr, L.u, nullptr, zero}, launches);
+        tile_leg(h, DOWN, L, C, {0, nullptr, L.u, nullptr, level_start(s, l + 1)}, launches);
         C.u = const_cast<float *>(vcycle(h, s, l + 1, launches));
         tile_leg(h, UP, L, C, {0, L.u, L.w, sol, 0}, launches);
         return L.w;
     }
-    smooth(h, L, coarsest ? coarse_sweeps(L) : NU, launches);
-    if (!coarsest) {
-        Lv C = s->lv[l + 1];
-        launches += 2;
-        launch_after(k_mg_residual, pts_grid(L, blk), blk, 0, h->stream)(L);
-        launch_after(k_mg_restrict, pts_grid(C, blk), blk, 0, h->stream)(L, C);
-        C.u = const_cast<float *>(vcycle(h, s, l + 1, launches));
-        launches++;
-        launch_after(k_mg_prolong, pts_grid(L, blk), blk, 0, h->stream)(C, L);
-        smooth(h, L, NU, launches);
+    const Fine *fine = l == 0 ? &s->fine : nullptr;
+    if (coarsest) {
+        smooth(h, L, coarse_sweeps(L), 1, fine, launches);
+        return L.u;
     }
-    if (l == 0) {
-        launches++;
-        launch_after(k_mg_correct, pts_grid(L, blk), blk, 0, h->stream)(L, s->fine);
-    }
+    Lv C = s->lv[l + 1];
+    smooth(h, L, NU, 1, nullptr, launches);
+    launches += 2;
+    launch_after(k_mg_residual, pts_grid(L, blk), blk, 0, h->stream)(L);
+    launch_after(k_mg_restrict, pts_grid(C, blk), blk, 0, h->stream)(L, C, level_start(s, l + 1));
+    C.u = const_cast<float *>(vcycle(h, s, l + 1, launches));
+    launches++;
+    launch_after(k_mg_prolong, pts_grid(L, blk), blk, 0, h->stream)(C, L);
+    smooth(h, L, NU, 0, fine, launches);
     return L.u;
 }
 
@@ -1027,7 +1053,7 @@ void residual64(emoo_handle *h, MgState *s, int &launches) {
     const Lv &L0 = s->lv[0];
     cudaMemsetAsync(s->dmax, 0, sizeof(double), h->stream);
     launches++;
-    launch_after(k_mg_residual64, pts_grid(L0, blk), blk, 0, h->stream)(L0, s->fine, s->dmax);
+    launch_after(k_mg_residual64, pts_grid(L0, blk), blk, 0, h->stream)(L0, s->fine, s->dmax, level_start(s, 0));
     cudaMemcpyAsync(s->hmax, s->dmax, sizeof(double), cudaMemcpyDeviceToHost, h->stream);
 }
 
