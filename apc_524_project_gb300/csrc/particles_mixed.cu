@@ -1238,19 +1238,19 @@ __device__ __forceinline__ bool fold_reaches(const MGeom &g, const MFold &f, int
 // reference policy plane 1 of a periodic dimension adds plane n + 1's two
 // transverse components over the physical transverse range; under the
 // corrected one (CORR) the points near a boundary sum their images over all
-// dimensions, in blocks of their own after the first `planes` planes of blocks:
-// among the others every warp holds some, and 128 x 48 x 48 cells took 34 us
-// instead of 22. Integer sums: the same words as a gather, three folds and the
+// dimensions, in blocks of their own, the first `edges` planes of blocks (they
+// take longest): among the others every warp holds some, and 128 x 48 x 48
+// cells took 34 us instead of 18.7. Integer sums: the same words as a gather, three folds and the
 // update one after the other, which took five launches and read J again.
 template <bool CORR>
 __global__ void __launch_bounds__(256) k_current_e_m(MGeom g, MFold f, const unsigned long long *wj, MFix4 J,
                                                      MF3 E, MCF3 T, float dt, float q0, int es, int t1, int t2, Slabs S,
-                                                     int planes) {
+                                                     int edges) {
     after_previous();
-    int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = blockIdx.z;
-    const bool edge = CORR && (int)blockIdx.z >= planes;
+    int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, i = (int)blockIdx.z - edges;
+    const bool edge = CORR && i < 0;
     if (edge) {
-        const uint32_t block = (blockIdx.z - planes) * gridDim.y * gridDim.x + blockIdx.y * gridDim.x + blockIdx.x;
+        const uint32_t block = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         int d, c[3];
         if (!slab_point(S, block * 256 + threadIdx.y * 32 + threadIdx.x, d, c)) return;
 #pragma unroll
@@ -1332,6 +1332,16 @@ __global__ void __launch_bounds__(256) k_current_e_m(MGeom g, MFold f, const uns
 #pragma unroll
         for (int a = 0; a < 3; a++) c[a] = sum[a];
     }
+    // E's and B_tm1's loads before the first store, which they might alias
+    float e[3] = {}, tx[3] = {}, ty[3] = {}, tz[3] = {};
+    if (phys && !es) {
+        const float *Tx = T.p[0], *Ty = T.p[1], *Tz = T.p[2];
+        tx[0] = Tx[o], tx[1] = Tx[o - sy], tx[2] = Tx[o - 1];
+        ty[0] = Ty[o], ty[1] = Ty[o - sx], ty[2] = Ty[o - 1];
+        tz[0] = Tz[o], tz[1] = Tz[o - sx], tz[2] = Tz[o - sy];
+#pragma unroll
+        for (int a = 0; a < 3; a++) e[a] = E.p[a][o];
+    }
 #pragma unroll
     for (int a = 0; a < 3; a++) J.p[a][o] = (long long)c[a];
     if (!phys) return;
@@ -1343,10 +1353,9 @@ __global__ void __launch_bounds__(256) k_current_e_m(MGeom g, MFold f, const uns
         E.p[2][o] = -dt * (FOURPI_F * jz);
         return;
     }
-    const float *Tx = T.p[0], *Ty = T.p[1], *Tz = T.p[2];
-    E.p[0][o] -= dt * ((Ty[o] - Ty[o - 1]) * g.idf[2] - (Tz[o] - Tz[o - sy]) * g.idf[1] + FOURPI_F * jx);
-    E.p[1][o] -= dt * ((Tz[o] - Tz[o - sx]) * g.idf[0] - (Tx[o] - Tx[o - 1]) * g.idf[2] + FOURPI_F * jy);
-    E.p[2][o] -= dt * ((Tx[o] - Tx[o - sy]) * g.idf[1] - (Ty[o] - Ty[o - sx]) * g.idf[0] + FOURPI_F * jz);
+    E.p[0][o] = e[0] - dt * ((ty[0] - ty[2]) * g.idf[2] - (tz[0] - tz[2]) * g.idf[1] + FOURPI_F * jx);
+    E.p[1][o] = e[1] - dt * ((tz[0] - tz[1]) * g.idf[0] - (tx[0] - tx[2]) * g.idf[2] + FOURPI_F * jy);
+    E.p[2][o] = e[2] - dt * ((tx[0] - tx[1]) * g.idf[1] - (ty[0] - ty[1]) * g.idf[0] + FOURPI_F * jz);
 }
 
 // J (what & 1) and rho (what & 2) at every grid point from the per-cell
@@ -1642,26 +1651,26 @@ __device__ __forceinline__ float b_half(const MGeom &g, const MCF3 &T, const MF3
 }
 
 // The corrected policy's B half and ghost copies in one pass. Blocks of planes
-// z < planes: B (with `update`) at the physical points, E's forward
+// z >= edges: B (with `update`) at the physical points, E's forward
 // neighbours across a periodic boundary taken from the physical points they
 // are images of, so that E's ghost values need not be filled between the two
-// halves. The blocks after them: the ghost points of E, and with `all` of B
+// halves. The blocks before them: the ghost points of E, and with `all` of B
 // and B_tm1, from the points they are images of; a ghost of an updated point
 // forms the new B itself, so nothing in the pass waits for another part of it.
 // 128 x 48 x 48 cells: 7.4 us (21.8 us with the images written by the points'
 // own threads).
-__global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, Slabs S, int planes, int update, int all,
+__global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, Slabs S, int edges, int update, int all,
                                                    MF3 E, MF3 B, MF3 T, float dt) {
     after_previous();
     const MCF3 Tc = {{T.p[0], T.p[1], T.p[2]}};
     int c[3], of[3];
-    if ((int)blockIdx.z < planes) {
-        of[0] = (int)blockIdx.z + 1;
+    if ((int)blockIdx.z >= edges) {
+        of[0] = (int)blockIdx.z - edges + 1;
         of[1] = (int)(blockIdx.y * blockDim.y + threadIdx.y) + 1;
         of[2] = (int)(blockIdx.x * blockDim.x + threadIdx.x) + 1;
         if (of[1] > g.n[1] || of[2] > g.n[2]) return;
     } else {
-        const uint32_t block = (blockIdx.z - planes) * gridDim.y * gridDim.x + blockIdx.y * gridDim.x + blockIdx.x;
+        const uint32_t block = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         if (!ghost_point(S, g.n, g.wrap, block * (blockDim.x * blockDim.y) + threadIdx.y * blockDim.x + threadIdx.x, c,
                          of))
             return;
@@ -1680,7 +1689,7 @@ __global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, Slabs S, int planes,
 #pragma unroll
     for (int a = 0; a < 3; a++)
         if (half) b[a] = b_half(g, Tc, E, a, o, up, dt);
-    if ((int)blockIdx.z < planes) {
+    if ((int)blockIdx.z >= edges) {
 #pragma unroll
         for (int a = 0; a < 3; a++) B.p[a][o] = b[a];
         return;
@@ -2586,21 +2595,22 @@ static int mixed_light_planes(emoo_handle *h) {
     return n ? mixed_plane_sets(h, ps, n) : EMOO_OK;
 }
 
-// A launch of `planes` planes of blocks (grd.x x grd.y of 256 threads) and, behind
-// them, as many blocks as `edges` points of their own take: together, or where
-// the planes leave no room in the grid, one after the other.
+// A launch of `planes` planes of blocks (grd.x x grd.y of 256 threads) and, before
+// them, the planes of blocks that `edges` points of their own take, launched
+// with their number: together, or where that leaves no room in the grid, one
+// after the other.
 template <class F>
 static void launch_with_edges(emoo_handle *h, dim3 grd, int planes, int64_t edges, F launch) {
     const int64_t per = (int64_t)grd.x * grd.y * 256, more = (edges + per - 1) / per;
     const bool together = planes + more <= 65535;
+    if (!together) {
+        h->launches++;
+        launch(dim3((unsigned)((edges + 255) / 256)), 1);
+    }
     grd.z = (unsigned)(planes + (together ? more : 0));
     if (grd.z) {
         h->launches++;
-        launch(grd, planes);
-    }
-    if (!together) {
-        h->launches++;
-        launch(dim3((unsigned)((edges + 255) / 256)), 0);
+        launch(grd, together ? (int)more : 0);
     }
 }
 
@@ -2618,8 +2628,8 @@ static int mixed_b_ghost(emoo_handle *h, double dtp, bool all, bool update) {
     const dim3 blk(32, 8);
     const dim3 grd((mg.n[2] + 31) / 32, (mg.n[1] + 7) / 8, 1);
     const int64_t ghosts = slab_size(S);
-    launch_with_edges(h, grd, update ? mg.n[0] : 0, ghosts, [&](dim3 grid, int planes) {
-        launch_after(k_b_ghost_m, grid, blk, 0, h->stream)(mg, S, planes, update, all, E, B, T, (float)dtp);
+    launch_with_edges(h, grd, update ? mg.n[0] : 0, ghosts, [&](dim3 grid, int first) {
+        launch_after(k_b_ghost_m, grid, blk, 0, h->stream)(mg, S, first, update, all, E, B, T, (float)dtp);
     });
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
@@ -2821,14 +2831,14 @@ static int mixed_step_fields(emoo_handle *h, double dtp, int fold_what) {
             S.listed[d] = f.per[d] || f.mirror[2 * d] || f.mirror[2 * d + 1] ? std::min(6, g.tot[d]) : 0;
             S.rest[d] = g.tot[d] - S.listed[d];
         }
-        launch_with_edges(h, all, g.tot[0], slab_size(S), [&](dim3 grid, int planes) {
+        launch_with_edges(h, all, g.tot[0], slab_size(S), [&](dim3 grid, int first) {
             launch_after(k_current_e_m<true>, grid, blk, 0, h->stream)(mg, f, h->mf->wj, J, E, T, (float)dtp, (float)h->mf->q0, es,
-                                                             g.tot[1], g.tot[2], S, planes);
+                                                             g.tot[1], g.tot[2], S, first);
         });
     } else {
         h->launches++;
         launch_after(k_current_e_m<false>, all, blk, 0, h->stream)(mg, f, h->mf->wj, J, E, T, (float)dtp, (float)h->mf->q0, es,
-                                                         g.tot[1], g.tot[2], S, g.tot[0]);
+                                                         g.tot[1], g.tot[2], S, 0);
     }
     EMOO_CUDA(cudaGetLastError());
     if (fold_what & FOLD_RHO) EMOO_TRY(mixed_fold(h, FOLD_RHO));
