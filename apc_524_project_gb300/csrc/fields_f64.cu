@@ -66,12 +66,15 @@ __global__ void k_yee_b(Geom g, double dt, F3 B, CF3 T, CF3 E) {
     int64_t o = gidx(g, i, j, k);
     const double *Ex = E.p[0], *Ey = E.p[1], *Ez = E.p[2];
     double dx = g.d[0], dy = g.d[1], dz = g.d[2];
-    B.p[0][o] = T.p[0][o] + dt * (ddiv(Ey[o + 1] - Ey[o], dz, g.id[2], g.p2[2]) -
+    const double bx = T.p[0][o] + dt * (ddiv(Ey[o + 1] - Ey[o], dz, g.id[2], g.p2[2]) -
                                   ddiv(Ez[o + g.sy] - Ez[o], dy, g.id[1], g.p2[1]));
-    B.p[1][o] = T.p[1][o] + dt * (ddiv(Ez[o + g.sx] - Ez[o], dx, g.id[0], g.p2[0]) -
+    const double by = T.p[1][o] + dt * (ddiv(Ez[o + g.sx] - Ez[o], dx, g.id[0], g.p2[0]) -
                                   ddiv(Ex[o + 1] - Ex[o], dz, g.id[2], g.p2[2]));
-    B.p[2][o] = T.p[2][o] + dt * (ddiv(Ex[o + g.sy] - Ex[o], dy, g.id[1], g.p2[1]) -
+    const double bz = T.p[2][o] + dt * (ddiv(Ex[o + g.sy] - Ex[o], dy, g.id[1], g.p2[1]) -
                                   ddiv(Ey[o + g.sx] - Ey[o], dx, g.id[0], g.p2[0]));
+    B.p[0][o] = bx;  // stores last: the loads may not pass them
+    B.p[1][o] = by;
+    B.p[2][o] = bz;
 }
 
 // Grid::evolveFieldsES, src/grid/oGrid.cpp:67-81

@@ -1553,9 +1553,12 @@ __global__ void k_yee_b_m(MGeom g, MF3 B, MCF3 T, MCF3 E, float dt) {
     if (k > g.n[2] || j > g.n[1]) return;
     int64_t o = (int64_t)i * g.sx + (int64_t)j * g.sy + k;
     const float *Ex = E.p[0], *Ey = E.p[1], *Ez = E.p[2];
-    B.p[0][o] = T.p[0][o] + dt * ((Ey[o + 1] - Ey[o]) * g.idf[2] - (Ez[o + g.sy] - Ez[o]) * g.idf[1]);
-    B.p[1][o] = T.p[1][o] + dt * ((Ez[o + g.sx] - Ez[o]) * g.idf[0] - (Ex[o + 1] - Ex[o]) * g.idf[2]);
-    B.p[2][o] = T.p[2][o] + dt * ((Ex[o + g.sy] - Ex[o]) * g.idf[1] - (Ey[o + g.sx] - Ey[o]) * g.idf[0]);
+    const float bx = T.p[0][o] + dt * ((Ey[o + 1] - Ey[o]) * g.idf[2] - (Ez[o + g.sy] - Ez[o]) * g.idf[1]);
+    const float by = T.p[1][o] + dt * ((Ez[o + g.sx] - Ez[o]) * g.idf[0] - (Ex[o + 1] - Ex[o]) * g.idf[2]);
+    const float bz = T.p[2][o] + dt * ((Ex[o + g.sy] - Ex[o]) * g.idf[1] - (Ey[o + g.sx] - Ey[o]) * g.idf[0]);
+    B.p[0][o] = bx;  // stores last: the loads may not pass them
+    B.p[1][o] = by;
+    B.p[2][o] = bz;
 }
 
 __global__ void k_yee_es_m(MGeom g, MF3 E, MJ3 J, float dt, float q0) {
