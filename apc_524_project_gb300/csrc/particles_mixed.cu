@@ -865,6 +865,59 @@ __device__ __forceinline__ void commit_runs(float *col, int *keys, bool active, 
     __syncwarp();
 }
 
+// v += x unless `bits` holds `bit`: a test and a predicated add
+__device__ __forceinline__ void add_unless(float &v, float x, unsigned bits, unsigned bit) {
+    asm("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tand.b32 t, %2, %3;\n\tsetp.eq.u32 p, t, 0;\n\t@p add.rn.f32 %0, %0, %1;\n\t}"
+        : "+f"(v)
+        : "f"(x), "r"(bits), "r"(bit));
+}
+
+// commit_runs<12, true> for the corrected policy's kernel: the same sums, the
+// totals left in each run's last column and committed two at a time, a lane a
+// slot, without a branch a column. There it takes 3 % off the launch (10.0 M
+// particles: 360 -> 350 us); in the reference policy's kernel, with more warps
+// and more ends a warp, the interleaved walk is as much faster.
+template <bool GUARD>
+__device__ __forceinline__ void commit_listed(float *col, int2 *ends, bool active, int cell, unsigned long long *rec) {
+    const int lane = threadIdx.x & 31;
+    const unsigned act = __ballot_sync(0xffffffffu, active);
+    if (act == 0u) return;
+    const int key = active ? cell : -1 - lane;
+    const int prev = __shfl_up_sync(0xffffffffu, key, 1);
+    const unsigned heads = __ballot_sync(0xffffffffu, (lane & 15) == 0 || prev != key);
+    const unsigned last = ((heads >> 1) | 0x80000000u) & act;
+    if ((last >> lane) & 1u) ends[__popc(last & lanemask_lt())] = make_int2(cell, lane);
+    __syncwarp();
+    const int half = lane & 16;
+    const unsigned hd = heads >> half;
+    if ((lane & 15) < DEP_JSLOTS && heads != 0xffffffffu) {
+        float4 *row = reinterpret_cast<float4 *>(col + (lane & 15) * COL_STRIDE + half);
+        float acc = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float4 v = row[i];
+            add_unless(v.x, acc, hd, 1u << (4 * i));
+            add_unless(v.y, v.x, hd, 2u << (4 * i));
+            add_unless(v.z, v.y, hd, 4u << (4 * i));
+            add_unless(v.w, v.z, hd, 8u << (4 * i));
+            acc = v.w;
+            row[i] = v;
+        }
+    }
+    __syncwarp();
+    const int part = lane / DEP_JSLOTS, pos = lane - part * DEP_JSLOTS, n = __popc(last);
+    if (part < 2) {
+        unsigned long long *dst = rec + pos;
+        const float *v = col + dep_row(true, pos) * COL_STRIDE;
+#pragma unroll 2
+        for (int u = part; u < n; u += 2) {
+            const int2 e = ends[u];
+            atomicAdd(dst + (size_t)e.x * DEP_JSLOTS, (unsigned long long)f2ll_rn<GUARD>(v[e.y]));
+        }
+    }
+    __syncwarp();
+}
+
 // Fused gather + push + boundaries + deposit, one thread per particle.
 //
 // Deposit: each lane writes its particle's 12 J contributions as a column of a
@@ -905,7 +958,8 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
               MDeposit D, const float *g0, DevCounters *ctr, const MHost *__restrict__ Hp, int store_pre) {
     after_previous<false>();
     __shared__ __align__(16) float s_w[FUSED_WARPS][DEP_JSLOTS * COL_STRIDE];
-    __shared__ int s_key[FUSED_WARPS][32];
+    __shared__ int2 s_end[CORR ? FUSED_WARPS : 1][32];
+    __shared__ int s_key[CORR ? 1 : FUSED_WARPS][32];
     constexpr bool VBL = CORR;  // the corrected policy's pieces go through a list
     __shared__ float s_pl[VBL ? FUSED_WARPS : 1][DEP_JSLOTS][DEP_LIST + 1];
     __shared__ int s_plk[VBL ? FUSED_WARPS : 1][DEP_LIST];
@@ -923,7 +977,6 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
     const int64_t p = (int64_t)(blockIdx.x * blockDim.x + threadIdx.x);
     const int lane = threadIdx.x & 31;
     float *col = s_w[threadIdx.x >> 5];
-    int *keys = s_key[threadIdx.x >> 5];
     bool active = false;
     int mask = 0;
     int onew = 0;
@@ -1123,7 +1176,8 @@ __global__ void __launch_bounds__(FUSED_BLOCK, fused_min_blocks<CORR, HOST>())
         __syncthreads();
     }
     if (__any_sync(0xffffffffu, mask & 63)) count_cross(ctr, mask & 63);
-    commit_runs<12, true, !REL>(col, keys, active, onew, D.wj);
+    if (CORR) commit_listed<!REL>(col, s_end[threadIdx.x >> 5], active, onew, D.wj);
+    else commit_runs<12, true, !REL>(col, s_key[threadIdx.x >> 5], active, onew, D.wj);
 }
 
 // Particle_Handler::depositRhoJ at the current state: J (what & 1) and rho
