@@ -1465,12 +1465,15 @@ int emoo_step(emoo_handle *h, int nsteps, int64_t counts6[6]) {
         }
         if (h->precision == EMOO_FP64) {
             EMOO_TRY(fused_step_f64(h, h->dtp));
+            // the reference policy's folds of J go with the E half
+            const bool with_e = h->policy != EMOO_POLICY_CORRECTED && h->info.electrostatic != 1;
+            const int fold_now = with_e ? fold_what & ~FOLD_J : fold_what;
             if (h->policy == EMOO_POLICY_CORRECTED) EMOO_TRY(fold_full_f64(h, fold_what));
             else
-                for (int d = 0; d < 3; d++)
-                    if (h->bc.fbc[2 * d] == FBC_PERIODIC) EMOO_TRY(fold_f64(h, d, fold_what));
+                for (int d = 0; d < 3 && fold_now; d++)
+                    if (h->bc.fbc[2 * d] == FBC_PERIODIC) EMOO_TRY(fold_f64(h, d, fold_now));
             if (h->info.electrostatic == 1) EMOO_TRY(yee_es_f64(h, h->dtp));
-            else EMOO_TRY(yee_f64(h, h->dtp));
+            else EMOO_TRY(yee_f64(h, h->dtp, with_e));
             EMOO_TRY(execute_bc(h, EMOO_SEND_EB));
         } else {
             EMOO_TRY(mixed_step(h, h->dtp, fold_what));

@@ -230,7 +230,7 @@ void make_geom(const emoo_input_info &in, Geom &g);
 bool is_pow2(double v);
 
 // ---- FP64 field kernels (fields_f64.cu) ----
-int yee_f64(emoo_handle *h, double dt);
+int yee_f64(emoo_handle *h, double dt, bool fold_j = false);  // fold_j: after the reference policy's folds of J
 int yee_es_f64(emoo_handle *h, double dt);
 int ghost_fill_f64(emoo_handle *h, const int *ids, int nids, int dims_mask);
 constexpr int FOLD_J = 1, FOLD_RHO = 2, FOLD_ALL = 3;

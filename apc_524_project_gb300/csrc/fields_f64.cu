@@ -35,7 +35,16 @@ dim3 phys_grid(const Geom &g, dim3 blk) {
 
 // Grid::evolveFields, E half (src/grid/oGrid.cpp:23-40): E -= dt (curl-ish of
 // B_tm1 + 4 pi J) over physical points, B_tm1 being the freshly swapped role.
-__global__ void k_yee_e(Geom g, double dt, F3 E, CF3 T, CF3 J) {
+// FOLD: first the reference policy's periodic folds of J (k_fold, dimension by
+// dimension): plane 1 adds plane n + 1's two transverse components over the
+// physical transverse range. Those sources are no fold's target, so each point
+// forms its own sums in the folds' order.
+struct FoldDims {
+    int per[3];
+};
+
+template <bool FOLD>
+__global__ void k_yee_e(Geom g, double dt, F3 E, CF3 T, F3 J, FoldDims f) {
     after_previous();
     int k = blockIdx.x * blockDim.x + threadIdx.x + 1;
     int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
@@ -44,15 +53,30 @@ __global__ void k_yee_e(Geom g, double dt, F3 E, CF3 T, CF3 J) {
     int64_t o = gidx(g, i, j, k);
     const double *Tx = T.p[0], *Ty = T.p[1], *Tz = T.p[2];
     double dx = g.d[0], dy = g.d[1], dz = g.d[2];
+    double jx = J.p[0][o], jy = J.p[1][o], jz = J.p[2][o];
+    bool folded = false;
+    if (FOLD) {
+        const int64_t s0 = o + (int64_t)g.n[0] * g.sx, s1 = o + (int64_t)g.n[1] * g.sy, s2 = o + g.n[2];
+        const bool f0 = f.per[0] && i == 1, f1 = f.per[1] && j == 1, f2 = f.per[2] && k == 1;
+        if (f0) jy += J.p[1][s0], jz += J.p[2][s0];
+        if (f1) jx += J.p[0][s1], jz += J.p[2][s1];
+        if (f2) jx += J.p[0][s2], jy += J.p[1][s2];
+        folded = f0 || f1 || f2;
+    }
     double ex = E.p[0][o] - dt * (ddiv(Ty[o] - Ty[o - 1], dz, g.id[2], g.p2[2]) -
-                                  ddiv(Tz[o] - Tz[o - g.sy], dy, g.id[1], g.p2[1]) + FOURPI * J.p[0][o]);
+                                  ddiv(Tz[o] - Tz[o - g.sy], dy, g.id[1], g.p2[1]) + FOURPI * jx);
     double ey = E.p[1][o] - dt * (ddiv(Tz[o] - Tz[o - g.sx], dx, g.id[0], g.p2[0]) -
-                                  ddiv(Tx[o] - Tx[o - 1], dz, g.id[2], g.p2[2]) + FOURPI * J.p[1][o]);
+                                  ddiv(Tx[o] - Tx[o - 1], dz, g.id[2], g.p2[2]) + FOURPI * jy);
     double ez = E.p[2][o] - dt * (ddiv(Tx[o] - Tx[o - g.sy], dy, g.id[1], g.p2[1]) -
-                                  ddiv(Ty[o] - Ty[o - g.sx], dx, g.id[0], g.p2[0]) + FOURPI * J.p[2][o]);
+                                  ddiv(Ty[o] - Ty[o - g.sx], dx, g.id[0], g.p2[0]) + FOURPI * jz);
     E.p[0][o] = ex;
     E.p[1][o] = ey;
     E.p[2][o] = ez;
+    if (FOLD && folded) {
+        J.p[0][o] = jx;
+        J.p[1][o] = jy;
+        J.p[2][o] = jz;
+    }
 }
 
 // Grid::evolveFields, B half (src/grid/oGrid.cpp:43-57): B = B_tm1 + dt curl E.
@@ -675,7 +699,7 @@ int reduce_blocks(const Geom &g) {
 double *role_b(emoo_handle *h, int c) { return h->bswap ? h->slot[EMOO_BX_TM1 + c] : h->slot[EMOO_BX + c]; }
 double *role_t(emoo_handle *h, int c) { return h->bswap ? h->slot[EMOO_BX + c] : h->slot[EMOO_BX_TM1 + c]; }
 
-int yee_f64(emoo_handle *h, double dt) {
+int yee_f64(emoo_handle *h, double dt, bool fold_j) {
     // std::swap of the member pointers only (src/grid/oGrid.cpp:18-20)
     h->bswap ^= 1;
     const Geom &g = h->g;
@@ -683,9 +707,12 @@ int yee_f64(emoo_handle *h, double dt) {
     dim3 grd = phys_grid(g, blk);
     F3 E = {{h->slot[EMOO_EX], h->slot[EMOO_EY], h->slot[EMOO_EZ]}};
     CF3 T = {{role_t(h, 0), role_t(h, 1), role_t(h, 2)}};
-    CF3 J = {{h->slot[EMOO_JX], h->slot[EMOO_JY], h->slot[EMOO_JZ]}};
+    F3 J = {{h->slot[EMOO_JX], h->slot[EMOO_JY], h->slot[EMOO_JZ]}};
     h->launches++;
-    launch_after(k_yee_e, grd, blk, 0, h->stream)(g, dt, E, T, J);
+    FoldDims f;
+    for (int d = 0; d < 3; d++) f.per[d] = h->bc.fbc[2 * d] == FBC_PERIODIC;
+    if (fold_j) launch_after(k_yee_e<true>, grd, blk, 0, h->stream)(g, dt, E, T, J, f);
+    else launch_after(k_yee_e<false>, grd, blk, 0, h->stream)(g, dt, E, T, J, f);
     // The B half reads E one plane past the high faces. The reference refreshes
     // those ghosts only after both halves, so at the periodic wrap B sees the
     // previous step's E: the leapfrog loses its time centring there and vacuum
@@ -707,8 +734,8 @@ int yee_half_f64(emoo_handle *h, double dt, int half) {
     h->launches++;
     if (half == 0) {
         F3 E = {{h->slot[EMOO_EX], h->slot[EMOO_EY], h->slot[EMOO_EZ]}};
-        CF3 J = {{h->slot[EMOO_JX], h->slot[EMOO_JY], h->slot[EMOO_JZ]}};
-        launch_after(k_yee_e, grd, blk, 0, h->stream)(g, dt, E, T, J);
+        F3 J = {{h->slot[EMOO_JX], h->slot[EMOO_JY], h->slot[EMOO_JZ]}};
+        launch_after(k_yee_e<false>, grd, blk, 0, h->stream)(g, dt, E, T, J, FoldDims{});
     } else {
         F3 B = {{role_b(h, 0), role_b(h, 1), role_b(h, 2)}};
         CF3 E = {{h->slot[EMOO_EX], h->slot[EMOO_EY], h->slot[EMOO_EZ]}};
