@@ -473,13 +473,13 @@ int noalloc_scratch(NoAllocScratch **out) {
 int noalloc_scan(cudaStream_t s, uint32_t *data, int64_t m, uint32_t *tmp) {
     int64_t t = tiles(m);
     if (t <= 1) {
-        launch_after(k_scan_tile, 1, RS_THREADS, 0, s)(data, m, nullptr);
+        k_scan_tile<<<1, RS_THREADS, 0, s>>>(data, m, nullptr);
         EMOO_CUDA(cudaGetLastError());
         return EMOO_OK;
     }
-    launch_after(k_scan_tile, (unsigned)t, RS_THREADS, 0, s)(data, m, tmp);
+    k_scan_tile<<<(unsigned)t, RS_THREADS, 0, s>>>(data, m, tmp);
     EMOO_TRY(noalloc_scan(s, tmp, t, tmp + t));
-    launch_after(k_scan_add, (unsigned)t, RS_THREADS, 0, s)(data, m, tmp);
+    k_scan_add<<<(unsigned)t, RS_THREADS, 0, s>>>(data, m, tmp);
     EMOO_CUDA(cudaGetLastError());
     return EMOO_OK;
 }
@@ -516,10 +516,11 @@ extern "C" int emoo_sort_permutation_noalloc(const uint32_t *keys, int64_t n, in
         uint32_t *kout = last ? nullptr : sc->key[ps & 1];
         // alternate so that the last pass lands in the caller's array
         uint32_t *vout = ((passes - 1 - ps) % 2 == 0) ? perm : scr_perm;
-        launch_after(k_hist<RS_BINS>, nblocks, RS_THREADS, 0, s)(kin, n, shift, mask, sc->hist, nblocks);
+        // ordinary launches: `s` is the caller's stream, which may be capturing
+        k_hist<RS_BINS><<<nblocks, RS_THREADS, 0, s>>>(kin, n, shift, mask, sc->hist, nblocks);
         EMOO_CUDA(cudaGetLastError());
         EMOO_TRY(noalloc_scan(s, sc->hist, nhist, sc->scan));
-        launch_after(k_scatter<RS_BINS>, nblocks, RS_THREADS, 0, s)(kin, vin, kout, vout, n, shift, mask, sc->hist, nblocks);
+        k_scatter<RS_BINS><<<nblocks, RS_THREADS, 0, s>>>(kin, vin, kout, vout, n, shift, mask, sc->hist, nblocks);
         EMOO_CUDA(cudaGetLastError());
         kin = kout;
         vin = vout;
