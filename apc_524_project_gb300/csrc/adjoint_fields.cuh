@@ -195,7 +195,7 @@ struct WrapDims {
 
 // Adjoint of the whole-range ghost copies of the fields: each point with images
 // takes in their adjoints and clears them; blockIdx.y = field. 32^3 cells, nine
-// fields: 3.5 us (26 us with a thread a point of the grid for all fields).
+// fields: 4.0 us (26 us with a thread a point of the grid for all fields).
 template <class R>
 __global__ void k_copy_images_adj(Geom g, Slots9T<R> fl, WrapDims w, Slabs S) {
     after_previous();

@@ -1714,7 +1714,7 @@ __device__ __forceinline__ float b_half(const MGeom &g, const MCF3 &T, const MF3
 // halves. The blocks before them: the ghost points of E, and with `all` of B
 // and B_tm1, from the points they are images of; a ghost of an updated point
 // forms the new B itself, so nothing in the pass waits for another part of it.
-// 128 x 48 x 48 cells: 7.4 us (21.8 us with the images written by the points'
+// 128 x 48 x 48 cells: 8.3 us (21.8 us with the images written by the points'
 // own threads).
 __global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, Slabs S, int edges, int update, int all,
                                                    MF3 E, MF3 B, MF3 T, float dt) {
