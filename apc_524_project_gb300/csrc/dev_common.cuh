@@ -184,6 +184,34 @@ __device__ __forceinline__ bool ghost_point(const Slabs &S, const int n[3], cons
     return true;
 }
 
+// A warp's sums of N values a lane (4 or 8): lane l returns that of value
+// total_index<N>(l). Each step over lane bit 16, 8, 4, .. also halves the values
+// a lane still holds, which takes 9 FP64 additions for 8 values instead of 40
+// (6 instead of 20 for 4); the additions of a sum are paired as in a tree of its
+// own, so its bits are that tree's.
+template <int N>
+__device__ __forceinline__ double warp_totals(double (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+    int off = 16;
+#pragma unroll
+    for (int half = N / 2; half >= 1; half >>= 1, off >>= 1) {
+        const bool up = lane & off;
+#pragma unroll
+        for (int q = 0; q < half; q++) {
+            const double give = up ? v[q] : v[q + half];
+            v[q] = (up ? v[q + half] : v[q]) + __shfl_xor_sync(0xffffffffu, give, off);
+        }
+    }
+    for (; off > 0; off >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+    return v[0];
+}
+
+template <int N>
+__device__ __forceinline__ int total_index(int lane) {
+    return N == 8 ? ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)
+                  : ((lane >> 4) & 1) * 2 + ((lane >> 3) & 1);
+}
+
 __device__ __forceinline__ void atomic_max_nonneg(double *addr, double v) {
     // non-negative doubles order like their bit patterns
     atomicMax((unsigned long long *)addr, (unsigned long long)__double_as_longlong(v));

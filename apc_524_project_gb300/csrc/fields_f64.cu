@@ -610,7 +610,7 @@ __global__ void k_a_to_b(Geom g, const double *Ax, const double *Ay, const doubl
 // (src/IO/output.cpp:98-114; SQR(x) expands to x*x unparenthesised).
 __global__ void k_field_energy(Geom g, CF3 E, CF3 B, double *part) {
     after_previous();
-    double acc[6] = {0, 0, 0, 0, 0, 0};
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // 6 used
     int64_t nphys = (int64_t)g.n[0] * g.n[1] * g.n[2];
     double hv = 0.5 * g.vol;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nphys; t += (int64_t)gridDim.x * blockDim.x) {
@@ -627,11 +627,9 @@ __global__ void k_field_energy(Geom g, CF3 E, CF3 B, double *part) {
     }
     __shared__ double sh[32][6];
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int q = 0; q < 6; q++) {
-        double v = acc[q];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) sh[w][q] = v;
-    }
+    const double total = warp_totals<8>(acc);
+    const int at = total_index<8>(lane);
+    if ((lane & 3) == 0 && at < 6) sh[w][at] = total;
     __syncthreads();
     if (threadIdx.x < 6) {
         double v = 0.0;

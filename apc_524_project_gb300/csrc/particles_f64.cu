@@ -599,11 +599,9 @@ __global__ void k_moments(SpeciesTab st, PState S, int64_t np, double *part) {
     }
     __shared__ double sh[32][4];
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int q = 0; q < 4; q++) {
-        double v = acc[q];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) sh[w][q] = v;
-    }
+    const double total = warp_totals<4>(acc);
+    const int at = total_index<4>(lane);
+    if ((lane & 7) == 0) sh[w][at] = total;
     __syncthreads();
     if (threadIdx.x < 4) {
         double v = 0.0;

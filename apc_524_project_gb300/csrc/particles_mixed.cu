@@ -1805,7 +1805,9 @@ __global__ void k_plane_m(MGeom g, MPlaneList pl, int tot0, int tot1, int tot2) 
 // those partial sums in FP64: FP64 arithmetic per item would run on the
 // narrow FP64 pipe (2 lanes per clock per SM on this GPU), which made these
 // reductions cost more than a whole step. The partition is fixed by the launch
-// shape, so the sums are reproducible.
+// shape, so the sums are reproducible. On small boxes the sums over a warp were
+// most of what was left there (the field energies of 128 x 48 x 48 cells: 36 us, 14
+// with warp_totals).
 constexpr int DIAG_CHUNK = 8;
 
 __global__ void k_moments_m(MSpecies st, MState S, int64_t np, int rel, const float *g0, double *part) {
@@ -1827,20 +1829,18 @@ __global__ void k_moments_m(MSpecies st, MState S, int64_t np, int rel, const fl
         }
         if (++k == DIAG_CHUNK) {
             for (int q = 0; q < 4; q++) {
-                acc[q] += (double)f[q];
+                acc[q] += f64_of_f32(f[q]);
                 f[q] = 0.0f;
             }
             k = 0;
         }
     }
-    for (int q = 0; q < 4; q++) acc[q] += (double)f[q];
+    for (int q = 0; q < 4; q++) acc[q] += f64_of_f32(f[q]);
     __shared__ double sh[32][4];
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int q = 0; q < 4; q++) {
-        double v = acc[q];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) sh[w][q] = v;
-    }
+    const double total = warp_totals<4>(acc);
+    const int at = total_index<4>(lane);
+    if ((lane & 7) == 0) sh[w][at] = total;
     __syncthreads();
     if (threadIdx.x < 4) {
         double v = 0.0;
@@ -1851,7 +1851,7 @@ __global__ void k_moments_m(MSpecies st, MState S, int64_t np, int rel, const fl
 
 __global__ void k_energy_m(MGeom g, MCF3 E, MCF3 B, double hv, double *part) {
     after_previous();
-    double acc[6] = {0, 0, 0, 0, 0, 0};
+    double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // 6 used
     int64_t nphys = (int64_t)g.n[0] * g.n[1] * g.n[2];
     float f[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
     int cnt = 0;
@@ -1868,20 +1868,18 @@ __global__ void k_energy_m(MGeom g, MCF3 E, MCF3 B, double hv, double *part) {
         }
         if (++cnt == DIAG_CHUNK) {
             for (int q = 0; q < 6; q++) {
-                acc[q] += hv * (double)f[q];
+                acc[q] += hv * f64_of_f32(f[q]);
                 f[q] = 0.0f;
             }
             cnt = 0;
         }
     }
-    for (int q = 0; q < 6; q++) acc[q] += hv * (double)f[q];
+    for (int q = 0; q < 6; q++) acc[q] += hv * f64_of_f32(f[q]);
     __shared__ double sh[32][6];
     int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int q = 0; q < 6; q++) {
-        double v = acc[q];
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) sh[w][q] = v;
-    }
+    const double total = warp_totals<8>(acc);
+    const int at = total_index<8>(lane);
+    if ((lane & 3) == 0 && at < 6) sh[w][at] = total;
     __syncthreads();
     if (threadIdx.x < 6) {
         double v = 0.0;
