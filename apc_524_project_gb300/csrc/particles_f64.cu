@@ -146,7 +146,8 @@ __device__ __forceinline__ int64_t deposit_point(const Geom &g, int64_t o, int q
 // cells to the grid with one atomic. A warp of particles all in cells of
 // their own commits from registers. Summing by rows takes 16 FP64 additions a
 // warp for J (a shuffle tree per contribution took 60).
-constexpr int PART_BLOCK = 256;
+constexpr int PART_BLOCK = 256;  // at most; k_fused's launch takes half of it below a size
+constexpr int VB_BLOCK = 128;
 constexpr int PART_WARPS = PART_BLOCK / 32;
 constexpr int ROW = 34;  // doubles: rows on 16-byte boundaries, 16-byte reads of 8 rows without bank conflicts
 
@@ -418,14 +419,14 @@ __device__ void absorbed_exit(const Geom &g, const BCTab &bc, const DepositPtrs 
 // against 1877 us with every particle's pieces committed one by one (12
 // atomics a piece) and the FP64 tests, conversions and divisions in place.
 template <bool REL, int MODE>
-__global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
+__global__ void __launch_bounds__(VB_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
                                                          int64_t np, DepositPtrs D, double dt,
                                                          DevCounters *ctr) {
     after_previous<false>();
     constexpr bool UNIT = MODE != ANY;
-    __shared__ CommitTile tiles[PART_WARPS];
-    __shared__ double s_move[6][PART_BLOCK];  // start and end of the listed moves
-    __shared__ double s_coef[PART_BLOCK];
+    __shared__ CommitTile tiles[VB_BLOCK / 32];
+    __shared__ double s_move[6][VB_BLOCK];  // start and end of the listed moves
+    __shared__ double s_coef[VB_BLOCK];
     __shared__ int s_n;
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
@@ -513,7 +514,7 @@ __global__ void __launch_bounds__(PART_BLOCK) k_fused_vb(Geom g, SpeciesTab st, 
     }
     commit_deposit<12, 0>(g, D, tiles[threadIdx.x >> 5], active, o, c);
     __syncthreads();
-    for (int i = threadIdx.x; i < s_n; i += PART_BLOCK) {
+    for (int i = threadIdx.x; i < s_n; i += VB_BLOCK) {
         const double a[3] = {s_move[0][i], s_move[1][i], s_move[2][i]};
         const double b[3] = {s_move[3][i], s_move[4][i], s_move[5][i]};
         vb_deposit(g, D, a, b, s_coef[i]);
@@ -745,7 +746,7 @@ int deposit_f64(emoo_handle *h, int with_rho) {
     SpeciesTab st;
     species_tab(h, h->dtp, st);
     h->launches++;
-    launch_after(k_deposit, blocks_for(h->np), 256, 0, h->stream)(h->g, st, pstate(h), h->np, deposit_ptrs(h), with_rho, h->ctr);
+    launch_after(k_deposit, blocks_for(h->np, PART_BLOCK), PART_BLOCK, 0, h->stream)(h->g, st, pstate(h), h->np, deposit_ptrs(h), with_rho, h->ctr);
     EMOO_CUDA(cudaGetLastError());
     return rho_background_f64(h, with_rho);
 }
@@ -758,7 +759,7 @@ int deposit_rho_f64(emoo_handle *h) {
         SpeciesTab st;
         species_tab(h, h->dtp, st);
         h->launches++;
-        launch_after(k_deposit, blocks_for(h->np), 256, 0, h->stream)(h->g, st, pstate(h), h->np, deposit_ptrs(h), 2, h->ctr);
+        launch_after(k_deposit, blocks_for(h->np, PART_BLOCK), PART_BLOCK, 0, h->stream)(h->g, st, pstate(h), h->np, deposit_ptrs(h), 2, h->ctr);
         EMOO_CUDA(cudaGetLastError());
     }
     return rho_background_f64(h, 1);
@@ -766,13 +767,18 @@ int deposit_rho_f64(emoo_handle *h) {
 
 template <bool REL, int MODE>
 static void launch_fused(emoo_handle *h, const SpeciesTab &st, double dtp) {
-    const int nb = blocks_for(h->np, PART_BLOCK);
+    // Blocks of 128 leave a shorter last wave: 524,288 particles, 20 Langmuir
+    // steps, 4164 -> 4087 us, a gradient of as many 23.9 -> 23.5 ms. At 3.5 M,
+    // k_fused is 0.4 % faster with 256; k_fused_vb is not (blocks of 64, whose
+    // lists of moves fill few warps, took 17 % longer at 1.7 M).
+    const int blk = h->policy == EMOO_POLICY_CORRECTED ? VB_BLOCK : h->np < (1 << 20) ? PART_BLOCK / 2 : PART_BLOCK;
+    const int nb = blocks_for(h->np, blk);
     if (h->policy == EMOO_POLICY_CORRECTED)
-        launch_after(k_fused_vb<REL, MODE>, nb, PART_BLOCK, 0, h->stream)(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
-                                                                deposit_ptrs(h), dtp, h->ctr);
+        launch_after(k_fused_vb<REL, MODE>, nb, blk, 0, h->stream)(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
+                                                                   deposit_ptrs(h), dtp, h->ctr);
     else
-        launch_after(k_fused<REL, MODE>, nb, PART_BLOCK, 0, h->stream)(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
-                                                             deposit_ptrs(h), dtp, h->ctr);
+        launch_after(k_fused<REL, MODE>, nb, blk, 0, h->stream)(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
+                                                                deposit_ptrs(h), dtp, h->ctr);
 }
 
 int fused_step_f64(emoo_handle *h, double dtp) {
