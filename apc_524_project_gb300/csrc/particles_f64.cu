@@ -17,6 +17,7 @@
 // reciprocal, and grids of unit cells at the origin (UNIT) skip the divisions
 // and products by 1.
 #include <cuda_runtime.h>
+#include <stddef.h>
 
 #include <algorithm>
 #include <vector>
@@ -151,10 +152,14 @@ constexpr int VB_BLOCK = 128;
 constexpr int PART_WARPS = PART_BLOCK / 32;
 constexpr int ROW = 34;  // doubles: rows on 16-byte boundaries, 16-byte reads of 8 rows without bank conflicts
 
-struct CommitTile {
+struct alignas(16) CommitTile {
     double w[12 * ROW];
     int key[32];
 };
+// a row's parts are read as double2, in every tile of an array of them
+static_assert(alignof(CommitTile) % sizeof(double2) == 0 && offsetof(CommitTile, w) % sizeof(double2) == 0 &&
+                  sizeof(CommitTile) % sizeof(double2) == 0 && ROW * sizeof(double) % sizeof(double2) == 0,
+              "16-byte reads of a tile's rows");
 
 template <int NQ, int Q0>
 __device__ __forceinline__ void commit_deposit(const Geom &g, const DepositPtrs &D, CommitTile &tile, bool active,
