@@ -285,9 +285,11 @@ __global__ void k_jacobi_check(Geom g, const double *u1, const double *u2, doubl
 // a tile's two buffers (ping-pong, one ghost layer) and right side stay in
 // shared memory. After each sweep a block hands its face values to its six
 // neighbours and takes theirs; no block waits for any other. A value travels
-// as one 16-byte word of two (32 bits, sequence number) pairs, each 8-byte
-// pair written and read whole, so the reader polls the value itself and no
-// fence or flag is needed; two slots a face suffice, because a block writes
+// as two 64-bit words of (sequence number, 32 bits), each the element of a
+// vector access and so written and read whole (a vector access is no more than
+// its elements' accesses): the reader polls the value itself and no fence or
+// flag is needed. This is the exchange that collective libraries use for small
+// messages. Two slots a face suffice, because a block writes
 // sequence q + 2 only after it has read its neighbours' q + 1, which they made
 // from its q. A sweep of 32^3 takes 1.8 us, of which the FP64 pipe needs 0.6
 // (10 instructions a point, 8 warps an SM) and the exchange's latency the
@@ -305,13 +307,30 @@ constexpr int JT_THREADS = 1024;
 constexpr int JT_SPIN = 1 << 22;
 
 struct JacobiTiles {
-    int b[3];        // tiles per dimension
-    int t[3];        // points of the largest tile per dimension
-    int face;        // points of the largest face
-    uint4 *faces;    // [block][side][slot][face]
+    int b[3];           // tiles per dimension
+    int t[3];           // points of the largest tile per dimension
+    int face;           // points of the largest face
+    ulonglong2 *faces;  // [block][side][slot][face]
     unsigned long long *moved;  // [batch] OR over the blocks
     unsigned int *arrived;      // grid barrier
 };
+
+__device__ __forceinline__ void jt_send(ulonglong2 *to, double v, unsigned int seq) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v), tag = (unsigned long long)seq << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(to), "l"(tag | (b & 0xffffffffull)), "l"(tag | b >> 32)
+                 : "memory");
+}
+
+// the value that carries number seq; false when the wait ran out
+__device__ __forceinline__ bool jt_take(const ulonglong2 *from, unsigned int seq, double &v) {
+    unsigned long long x, y;
+    int spin = 0;
+    do {
+        asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "l"(from) : "memory");
+    } while (((unsigned int)(x >> 32) != seq || (unsigned int)(y >> 32) != seq) && ++spin < JT_SPIN);
+    v = __hiloint2double((int)(unsigned int)y, (int)(unsigned int)x);
+    return spin < JT_SPIN;
+}
 
 // blocks that passed barrier number `round` (1, 2, ..); false when it ran out
 __device__ __forceinline__ bool jt_barrier(unsigned int *arrived, unsigned int round) {
@@ -419,17 +438,8 @@ __global__ void __launch_bounds__(JT_THREADS) k_jacobi_tiles(Geom g, double *u1,
                 int d = hd, side = hside, q = hq, at = hat;
                 if (p != threadIdx.x) at = halo_at(p, d, side, q);
                 // my ghost plane on this side is the neighbour's face on the other
-                const uint4 *src = slot(nb[2 * d + side], 2 * d + 1 - side, seq) + q;
-                unsigned int x, f0, y, f1;
-                int spin = 0;
-                do {
-                    asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                 : "=r"(x), "=r"(f0), "=r"(y), "=r"(f1)
-                                 : "l"(src)
-                                 : "memory");
-                } while ((f0 != seq || f1 != seq) && ++spin < JT_SPIN);
-                got = got && spin < JT_SPIN;
-                cur[at] = __hiloint2double((int)y, (int)x);
+                const ulonglong2 *src = slot(nb[2 * d + side], 2 * d + 1 - side, seq) + q;
+                got = jt_take(src, seq, cur[at]) && got;
             }
             ok = __syncthreads_and(got);
             if (!ok) return true;
@@ -443,17 +453,13 @@ __global__ void __launch_bounds__(JT_THREADS) k_jacobi_tiles(Geom g, double *u1,
             const double v = ax * (cur[o - px] + cur[o + px]) + ay * (cur[o - py] + cur[o + py]) +
                              az * (cur[o - 1] + cur[o + 1]) - rhs[p];
             next[o] = v;
-            const unsigned int x = (unsigned int)__double2loint(v), y = (unsigned int)__double2hiint(v);
 #pragma unroll
             for (int d = 0; d < 3; d++) {
                 const int o1 = d == 0 ? 1 : 0, o2 = d == 2 ? 1 : 2;
 #pragma unroll
                 for (int side = 0; side < 2; side++) {
                     if (c[d] != (side ? sz[d] - 1 : 0)) continue;
-                    asm volatile("st.volatile.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(
-                                     slot(blockIdx.x, 2 * d + side, seq) + c[o1] * sz[o2] + c[o2]),
-                                 "r"(x), "r"(seq), "r"(y)
-                                 : "memory");
+                    jt_send(slot(blockIdx.x, 2 * d + side, seq) + c[o1] * sz[o2] + c[o2], v, seq);
                 }
             }
             // |v - u| >= tol on the words (false for NaN, as the comparison is)
@@ -1091,11 +1097,11 @@ static int jacobi_tiling(emoo_handle *h, JacobiTiles *jt, size_t *smem) {
     if (!jt->b[0]) return EMOO_OK;
     EMOO_CUDA(cudaFuncSetAttribute(k_jacobi_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
     const int blocks = jt->b[0] * jt->b[1] * jt->b[2], batches = ITER_MAX / JT_BATCH + 2;
-    const size_t faces = (size_t)blocks * 12 * jt->face * sizeof(uint4);
+    const size_t faces = (size_t)blocks * 12 * jt->face * sizeof(ulonglong2);
     const size_t bytes = faces + batches * sizeof(unsigned long long) + sizeof(unsigned long long);
     if (!h->jacobi_tiles) EMOO_CUDA(cudaMalloc(&h->jacobi_tiles, bytes));  // one grid, one size a handle
     char *p = (char *)h->jacobi_tiles;
-    jt->faces = (uint4 *)p;
+    jt->faces = (ulonglong2 *)p;
     jt->moved = (unsigned long long *)(p + faces);
     jt->arrived = (unsigned int *)(jt->moved + batches);
     EMOO_CUDA(cudaMemsetAsync(p, 0, bytes, h->stream));
