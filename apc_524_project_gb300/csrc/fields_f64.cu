@@ -1095,7 +1095,8 @@ static int jacobi_tiling(emoo_handle *h, JacobiTiles *jt, size_t *smem) {
             jt->face = (int)std::max(t[0] * t[1], std::max(t[0] * t[2], t[1] * t[2]));
         }
     if (!jt->b[0]) return EMOO_OK;
-    EMOO_CUDA(cudaFuncSetAttribute(k_jacobi_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+    // the limit is the function's, for every handle: always the device's largest
+    EMOO_CUDA(cudaFuncSetAttribute(k_jacobi_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
     const int blocks = jt->b[0] * jt->b[1] * jt->b[2], batches = ITER_MAX / JT_BATCH + 2;
     const size_t faces = (size_t)blocks * 12 * jt->face * sizeof(ulonglong2);
     const size_t bytes = faces + batches * sizeof(unsigned long long) + sizeof(unsigned long long);
