@@ -1132,9 +1132,10 @@ int mg_setup(emoo_handle *h, MgState *s) {
         if (unknowns(s->lv[q]) <= TAIL_MAX && make_tail(s, q).nl > 0) {
             s->tail_from = q;
             std::vector<uint4> pts;
-            const Tail T = make_tail(s, q, &pts);
-            cudaError_t e = cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)(T.smem * sizeof(float)));
+            make_tail(s, q, &pts);
+            // the limit is the function's, for every handle: always the largest tail's
+            cudaError_t e =
+                cudaFuncSetAttribute(k_mg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, TAIL_SMEM_MAX);
             if (e == cudaSuccess) e = cudaMalloc(&s->tail_pts, pts.size() * sizeof(uint4));
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(s->tail_pts, pts.data(), pts.size() * sizeof(uint4), cudaMemcpyHostToDevice,
