@@ -6,8 +6,8 @@
 // 64 of any other kind. The helpers below give the same results from integer
 // instructions on the halves of the word (truncation, conversions, halving,
 // tests), or with fewer FP64 instructions (several quotients over one
-// divisor). They are complete over all words: a rare case left to the FP64
-// instruction would be predicated in by the compiler and issued always.
+// divisor). The integer ones are complete over all words: a rare case left to
+// the FP64 instruction would be predicated in by the compiler and issued always.
 #ifndef EMOO_F64_OPS_CUH
 #define EMOO_F64_OPS_CUH
 
@@ -23,6 +23,12 @@ __device__ __forceinline__ bool f64_not_nan(double x) {
 }
 
 __device__ __forceinline__ bool f64_sign(double x) { return __double2hiint(x) < 0; }
+
+// x == 0, from the halves: the word's low 63 bits compared with 0 are made an
+// FP64 comparison by the compiler (seven of them took 2.7 % of a thermal run)
+__device__ __forceinline__ bool f64_zero(double x) {
+    return (((unsigned)__double2hiint(x) & 0x7fffffffu) | (unsigned)__double2loint(x)) == 0u;
+}
 
 // __double2int_rz(t): truncated, saturated, NaN to the smallest.
 __device__ __forceinline__ int f64_trunc(double t) {
@@ -101,26 +107,34 @@ __device__ __forceinline__ long long f64_key(double x) {
 // the exact remainder r = a - b q, fma(r, y, q) is a / b correctly rounded
 // (P. Markstein, "Computation of elementary functions on the IBM RISC System
 // /6000 processor", IBM J. Res. Dev. 34 (1990) 111): three instructions a
-// quotient instead of a division's ten. Used where b is of ordinary size;
-// for the others (a run that is blowing up) every quotient is divided out.
+// quotient instead of a division's ten. For a (f64_fit) and b in [2^-500, 2^500),
+// where neither the remainder nor the quotient leaves the normal range, and for
+// a zero a, whose sign the last addition loses and the integer instruction sets.
+// The caller divides for others (fields that vanish, a run that is blowing up).
+__device__ __forceinline__ bool f64_ordinary(double x) {
+    return (((unsigned)__double2hiint(x) >> 20) & 0x7ffu) - 523u < 1000u;
+}
+
 struct F64Quot {
     double b, y;
-    bool plain;
+    bool ordinary;
 };
 
 __device__ __forceinline__ F64Quot f64_divisor(double b) {
     F64Quot d;
     d.b = b;
-    const unsigned e = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
-    d.plain = e - 523u > 1000u;  // outside [2^-500, 2^500]
+    d.ordinary = f64_ordinary(b);
     d.y = __drcp_rn(b);
     return d;
 }
 
+// whether f64_quot takes a
+__device__ __forceinline__ bool f64_fit(double a) { return f64_ordinary(a) || f64_zero(a); }
+
 __device__ __forceinline__ double f64_quot(double a, const F64Quot &d) {
-    if (d.plain) return __ddiv_rn(a, d.b);
-    const double q = __dmul_rn(a, d.y);
-    return __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
+    const double q = __dmul_rn(a, d.y), v = __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
+    const unsigned sign = (unsigned)(__double2hiint(a) ^ __double2hiint(d.b)) & 0x80000000u;
+    return __hiloint2double((int)(((unsigned)__double2hiint(v) & 0x7fffffffu) | sign), __double2loint(v));
 }
 
 // 1 / sqrt(b) for b in [1, inf) as y0 (1 + c): y0 the approximation instruction
