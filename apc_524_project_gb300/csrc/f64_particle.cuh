@@ -26,6 +26,10 @@ __device__ __forceinline__ Rn operator*(Rn a, Rn b) { return __dmul_rn(a.v, b.v)
 // a * b + c rounded once, where a * b is exact (a power of two times b): the
 // value of the separate operations
 __device__ __forceinline__ Rn exact_fma(double a, Rn b, Rn c) { return __fma_rn(a, b.v, c.v); }
+// a sum as it comes out when it starts with 0: a zero is +0
+__device__ __forceinline__ Rn sum_from_zero(Rn a) {
+    return __hiloint2double(f64_zero(a.v) ? 0 : __double2hiint(a.v), __double2loint(a.v));
+}
 // x / d (ddiv): the exact reciprocal where d is a power of two
 __device__ __forceinline__ Rn div_by(Rn a, double d, double id, int p2) { return p2 ? __dmul_rn(a.v, id) : __ddiv_rn(a.v, d); }
 
@@ -84,8 +88,8 @@ __device__ __forceinline__ void gather_cell(const Geom &g, const GatherPtrs &P, 
         v[0] = E[0], v[1] = E[st[j]], v[2] = E[st[j] + st[k]], v[3] = E[st[k]];
         S[0] = (Rn(T[0]) + B[0]).v;
         S[1] = (Rn(T[st[i]]) + B[st[i]]).v;
-        const Rn s = w[j] * w[k] * v[0] + r[j] * w[k] * v[1] + r[j] * r[k] * v[2] + w[j] * r[k] * v[3];
-        const Rn b = w[i] * S[0] + r[i] * S[1];
+        const Rn s = sum_from_zero(w[j] * w[k] * v[0] + r[j] * w[k] * v[1] + r[j] * r[k] * v[2] + w[j] * r[k] * v[3]);
+        const Rn b = sum_from_zero(w[i] * S[0] + r[i] * S[1]);
         e[i] = UNIT ? s.v : div_by(s, g.area[i], g.iarea[i], g.area_p2[i]).v;
         b2[i] = UNIT ? b.v : div_by(b, g.d[i], g.id[i], g.p2[i]).v;
     }

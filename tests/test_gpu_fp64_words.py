@@ -58,10 +58,14 @@ def oracle_step(o):
 @pytest.mark.parametrize("seed", range(4))
 @pytest.mark.parametrize("scale", [0.0, 2.0 ** -920, 1e-290, 1e-304])
 @pytest.mark.parametrize("dt", [0.5, 0.45])
-def test_push_gives_the_oracles_words(dt, scale, seed):
+@pytest.mark.parametrize("policy", [abi.POLICY_REFERENCE, abi.POLICY_CORRECTED])
+def test_push_gives_the_oracles_words(policy, dt, scale, seed):
     cfg, p, fields = case(scale, seed)
     info = configs.input_info(cfg)
-    want = run(OracleBackend(info, dt), p, fields, oracle_step)
-    got = run(GpuBackend(info, dt), p, fields, lambda g: g.step(1))
+    o = OracleBackend(info, dt)
+    if policy == abi.POLICY_CORRECTED:
+        o.set_policy(policy)
+    want = run(o, p, fields, oracle_step)
+    got = run(GpuBackend(info, dt, policy=policy), p, fields, lambda g: g.step(1))
     for k in KEYS:
         np.testing.assert_array_equal(got[k].view(np.int64), want[k].view(np.int64), err_msg=k)
