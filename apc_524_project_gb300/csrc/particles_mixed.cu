@@ -539,14 +539,16 @@ __device__ __forceinline__ void m_to_f64(const Geom &g, const Div3 &dv, int32_t 
     }
     if (rel) {
         // v = u / sqrt(1 + u^2): u y0 is exact (24 and 21 bits), so v is rounded
-        // once (a quotient by the rounded gamma, twice)
+        // once (a quotient by the rounded gamma, twice); its sign is u's (a
+        // zero's is lost in the sum where c is negative)
         const double g2 = 1.0 + u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
         const F64Rsqrt r = f64_rsqrt(g2);
         const double y = __fma_rn(r.y0, r.c, r.y0), ga = g2 * y;
         out[6] = __fma_rn(__fma_rn(-ga, ga, g2), f64_half(y), ga);
         for (int a = 0; a < 3; a++) {
-            const double w = u[a] * r.y0;
-            out[3 + a] = __fma_rn(w, r.c, w);
+            const double w = u[a] * r.y0, v = __fma_rn(w, r.c, w);
+            const unsigned sign = __float_as_uint(uf[a]) & 0x80000000u;
+            out[3 + a] = __hiloint2double((int)(((unsigned)__double2hiint(v) & 0x7fffffffu) | sign), __double2loint(v));
         }
         if (__double2hiint(g2) >= 0x7ff00000) {  // u not finite
             out[6] = g2;
