@@ -152,9 +152,8 @@ __device__ __forceinline__ int64_t deposit_point(const Geom &g, int64_t o, int q
 // 1.08 of it with 16 particles a cell, 0.96 with 61; rho 1.03, 0.97). Summed one
 // after the other, with an atomic for each half, J's was 1.20 and 1.16 of it; the
 // step then took 0.6 % less.
-constexpr int PART_BLOCK = 256;  // at most; k_fused's launch takes half of it below a size
-constexpr int VB_BLOCK = 128;
-constexpr int PART_WARPS = PART_BLOCK / 32;
+constexpr int PART_BLOCK = 256;
+constexpr int FUSED_BLOCK = 128;  // k_fused, k_fused_vb (see launch_fused)
 constexpr int ROW = 34;  // doubles: rows on 16-byte boundaries, 16-byte reads of 8 rows without bank conflicts
 
 struct alignas(16) CommitTile {
@@ -308,7 +307,7 @@ __global__ void k_particle_bc(BCTab bc, PState S, int64_t np, DevCounters *ctr) 
 __global__ void __launch_bounds__(PART_BLOCK) k_deposit(Geom g, SpeciesTab st, PState S, int64_t np, DepositPtrs D,
                                                         int what, DevCounters *ctr) {
     after_previous<false>();
-    __shared__ CommitTile tiles[PART_WARPS];
+    __shared__ CommitTile tiles[PART_BLOCK / 32];
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     bool active = false;
     int64_t o = 0;
@@ -438,14 +437,14 @@ __device__ void absorbed_exit(const Geom &g, const BCTab &bc, const DepositPtrs 
 // against 1877 us with every particle's pieces committed one by one (12
 // atomics a piece) and the FP64 tests, conversions and divisions in place.
 template <bool REL, int MODE>
-__global__ void __launch_bounds__(VB_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
+__global__ void __launch_bounds__(FUSED_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
                                                          int64_t np, DepositPtrs D, double dt,
                                                          DevCounters *ctr) {
     after_previous<false>();
     constexpr bool UNIT = MODE != ANY;
-    __shared__ CommitTile tiles[VB_BLOCK / 32];
-    __shared__ double s_move[6][VB_BLOCK];  // start and end of the listed moves
-    __shared__ double s_coef[VB_BLOCK];
+    __shared__ CommitTile tiles[FUSED_BLOCK / 32];
+    __shared__ double s_move[6][FUSED_BLOCK];  // start and end of the listed moves
+    __shared__ double s_coef[FUSED_BLOCK];
     __shared__ int s_n;
     if (threadIdx.x == 0) s_n = 0;
     __syncthreads();
@@ -533,7 +532,7 @@ __global__ void __launch_bounds__(VB_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BC
     }
     commit_deposit<12, 0>(g, D, tiles[threadIdx.x >> 5], active, o, c);
     __syncthreads();
-    for (int i = threadIdx.x; i < s_n; i += VB_BLOCK) {
+    for (int i = threadIdx.x; i < s_n; i += FUSED_BLOCK) {
         const double a[3] = {s_move[0][i], s_move[1][i], s_move[2][i]};
         const double b[3] = {s_move[3][i], s_move[4][i], s_move[5][i]};
         vb_deposit(g, D, a, b, s_coef[i]);
@@ -549,11 +548,11 @@ __global__ void __launch_bounds__(VB_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BC
 // Relativistic, 3,538,944 particles in 48^3 unit cells, sorted: 1507 us a
 // launch against 2550 us.
 template <bool REL, int MODE>
-__global__ void __launch_bounds__(PART_BLOCK) k_fused(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
+__global__ void __launch_bounds__(FUSED_BLOCK) k_fused(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
                                                       int64_t np, DepositPtrs D, double dt, DevCounters *ctr) {
     after_previous<false>();
     constexpr bool UNIT = MODE != ANY;
-    __shared__ CommitTile tiles[PART_WARPS];
+    __shared__ CommitTile tiles[FUSED_BLOCK / 32];
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     bool active = false;
     int64_t o = 0;
@@ -786,12 +785,12 @@ int deposit_rho_f64(emoo_handle *h) {
 
 template <bool REL, int MODE>
 static void launch_fused(emoo_handle *h, const SpeciesTab &st, double dtp) {
-    // Blocks of 128 leave a shorter last wave: 524,288 particles, 20 Langmuir
-    // steps, 4164 -> 4087 us, a gradient of as many 23.9 -> 23.5 ms. At 3.5 M,
-    // k_fused is 0.4 % faster with 256; k_fused_vb is not (blocks of 64, whose
-    // lists of moves fill few warps, took 17 % longer at 1.7 M).
-    const int blk = h->policy == EMOO_POLICY_CORRECTED ? VB_BLOCK : h->np < (1 << 20) ? PART_BLOCK / 2 : PART_BLOCK;
-    const int nb = blocks_for(h->np, blk);
+    // Blocks of 128 leave a shorter last wave than blocks of 256: 131,072
+    // relativistic particles, 10 steps, 1320 -> 1240 us, 442,368 2855 -> 2775,
+    // 1.3 million 7260 -> 7180, 2.5 million 12770 -> 12700; at 1.0 and 3.5
+    // million the same. Blocks of 64, whose lists of moves fill few warps, took
+    // k_fused_vb 17 % longer at 1.7 million.
+    const int blk = FUSED_BLOCK, nb = blocks_for(h->np, blk);
     if (h->policy == EMOO_POLICY_CORRECTED)
         launch_after(k_fused_vb<REL, MODE>, nb, blk, 0, h->stream)(h->g, st, h->bc, gather_ptrs(h), pstate(h), h->np,
                                                                    deposit_ptrs(h), dtp, h->ctr);
