@@ -307,7 +307,8 @@ struct VayTape {
 };
 
 // vay_eval<double> keeping its intermediates: the same operations in the
-// same order (bit-identical x, v, gamma).
+// same order (bit-identical x, v, gamma). With vay_rev, for the host's checks of
+// the reverse; the adjoint kernel takes its tape from the step's own vay_push.
 AD_HD void vay_fwd(double qp, const double f[6], double dt, double x[3], double v[3], double &gamma, VayTape &T) {
     const double e[3] = {f[0], f[1], f[2]}, b[3] = {f[3], f[4], f[5]};
     double vXb[3];

@@ -433,9 +433,11 @@ __device__ void absorbed_exit(const Geom &g, const BCTab &bc, const DepositPtrs 
 // together by full warps: splitting their paths in place would make every
 // warp issue the whole piece arithmetic on the FP64 pipe for them, and their
 // pieces end in scattered atomics either way. Relativistic beams, 1,682,464
-// particles in 49x37x29 unit cells: 1063 us a launch, FP64 pipe 84 % active,
+// particles in 49x37x29 unit cells: 1056 us a launch, FP64 pipe 84 % active,
 // against 1877 us with every particle's pieces committed one by one (12
 // atomics a piece) and the FP64 tests, conversions and divisions in place.
+// A whole move's terms use fused adds and a product by 1 / 12: there is no
+// reference to match bit for bit, and vb_deposit's are within rounding of them.
 template <bool REL, int MODE>
 __global__ void __launch_bounds__(FUSED_BLOCK) k_fused_vb(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,
                                                          int64_t np, DepositPtrs D, double dt,
@@ -543,9 +545,9 @@ __global__ void __launch_bounds__(FUSED_BLOCK) k_fused_vb(Geom g, SpeciesTab st,
 // The fused time-loop kernel: gather at the current position (what
 // InterpolateEB cached at the end of the previous step), push, the six
 // boundaries, then the current deposit at the new position. Bound by the FP64
-// pipe: 228 FP64 instructions a particle (405 with tests, conversions and
+// pipe: some 230 FP64 instructions a particle (405 with tests, conversions and
 // divisions on that pipe and the deposit summed in shuffle trees), 85 % active.
-// Relativistic, 3,538,944 particles in 48^3 unit cells, sorted: 1507 us a
+// Relativistic, 3,538,944 particles in 48^3 unit cells, sorted: 1513 us a
 // launch against 2550 us.
 template <bool REL, int MODE>
 __global__ void __launch_bounds__(FUSED_BLOCK) k_fused(Geom g, SpeciesTab st, BCTab bc, GatherPtrs P, PState S,

@@ -803,10 +803,9 @@ __device__ __forceinline__ void j_terms(float jx, float jy, float jz, const floa
 // lane's particle by itself, 12 instructions of 32 scattered words, took 237
 // instead of 183 us a launch (8.4 M particles 19 steps after the sort), L2
 // processing four times the requests.
-//  - Runs of one or two particles (particles that have drifted apart, unsorted
-//    input): pairs are summed in their first column, then all 32 lanes commit
-//    (column, slot) pairs, NQ rounds, skipping the columns that head no run.
-//  - Longer runs: lane q (and q + 16 with SPLIT) walks row q in particle order
+//  - Every particle in a cell of its own (drifted apart, unsorted input): all 32
+//    lanes commit (column, slot) pairs, NQ rounds, skipping inactive columns.
+//  - Else: lane q (and q + 16 with SPLIT) walks row q in particle order
 //    and commits at each run's end.
 template <int NQ, bool SPLIT, bool GUARD>
 __device__ __forceinline__ void commit_runs(float *col, int *keys, bool active, int cell, unsigned long long *rec) {
@@ -1304,7 +1303,7 @@ __device__ __forceinline__ bool fold_reaches(const MGeom &g, const MFold &f, int
 // corrected one (CORR) the points near a boundary sum their images over all
 // dimensions, in blocks of their own, the first `edges` planes of blocks (they
 // take longest): among the others every warp holds some, and 128 x 48 x 48
-// cells took 34 us instead of 18.7. Integer sums: the same words as a gather, three folds and the
+// cells took 34 us instead of 17.2. Integer sums: the same words as a gather, three folds and the
 // update one after the other, which took five launches and read J again.
 template <bool CORR>
 __global__ void __launch_bounds__(256) k_current_e_m(MGeom g, MFold f, const unsigned long long *wj, MFix4 J,
@@ -1724,7 +1723,7 @@ __device__ __forceinline__ float b_half(const MGeom &g, const MCF3 &T, const MF3
 // halves. The blocks before them: the ghost points of E, and with `all` of B
 // and B_tm1, from the points they are images of; a ghost of an updated point
 // forms the new B itself, so nothing in the pass waits for another part of it.
-// 128 x 48 x 48 cells: 8.3 us (21.8 us with the images written by the points'
+// 128 x 48 x 48 cells: 6.7 us (21.8 us with the images written by the points'
 // own threads).
 __global__ void __launch_bounds__(256) k_b_ghost_m(MGeom g, Slabs S, int edges, int update, int all,
                                                    MF3 E, MF3 B, MF3 T, float dt) {
